@@ -445,16 +445,78 @@ __device__ __forceinline__ void load_amplitude(FrameDev& fr) {
     }
 }
 
+// mp_sinf for |x| < 2^22 pi, one value and a packed pair, bit for bit: k is
+// rounded by adding and taking away 1.5 * 2^23 (round to nearest even, as
+// rintf, with no conversion instruction), its parity is the sum's lowest bit,
+// and k * -P equals -k * P.  x * (1 / pi) stays a scalar product: a packed
+// one feeding the packed sum could be fused with it.
+constexpr float kRintMagic = 12582912.0f;
+__device__ __forceinline__ float sin_small(float x) {
+    const float km = fadd(fmul(x, 0x1.45f306p-2f), kRintMagic);
+    const float k = fsub(km, kRintMagic);
+    float r = ffma(k, -0x1.921fb6p+1f, x);
+    r = ffma(k, 0x1.777a5cp-24f, r);
+    r = ffma(k, 0x1.ee59dap-49f, r);
+    const float r2 = fmul(r, r);
+    float p = ffma(r2, 0x1.612462p-33f, -0x1.ae6456p-26f);
+    p = ffma(r2, p, 0x1.71de3ap-19f);
+    p = ffma(r2, p, -0x1.a01a02p-13f);
+    p = ffma(r2, p, 0x1.111112p-7f);
+    p = ffma(r2, p, -0x1.555556p-3f);
+    const float sn = ffma(fmul(r, r2), p, r);
+    return __uint_as_float(__float_as_uint(sn) ^ (__float_as_uint(km) << 31));
+}
+__device__ __forceinline__ float2 sin2_small(float x, float y) {
+    const float2 km = fadd2(make_float2(fmul(x, 0x1.45f306p-2f), fmul(y, 0x1.45f306p-2f)), dup2(kRintMagic));
+    const float2 k = fadd2(km, dup2(-kRintMagic));
+    float2 r = ffma2(k, dup2(-0x1.921fb6p+1f), make_float2(x, y));
+    r = ffma2(k, dup2(0x1.777a5cp-24f), r);
+    r = ffma2(k, dup2(0x1.ee59dap-49f), r);
+    const float2 r2 = fmul2(r, r);
+    float2 p = ffma2(r2, dup2(0x1.612462p-33f), dup2(-0x1.ae6456p-26f));
+    p = ffma2(r2, p, dup2(0x1.71de3ap-19f));
+    p = ffma2(r2, p, dup2(-0x1.a01a02p-13f));
+    p = ffma2(r2, p, dup2(0x1.111112p-7f));
+    p = ffma2(r2, p, dup2(-0x1.555556p-3f));
+    const float2 sn = ffma2(fmul2(r, r2), p, r);
+    return make_float2(__uint_as_float(__float_as_uint(sn.x) ^ (__float_as_uint(km.x) << 31)),
+                       __uint_as_float(__float_as_uint(sn.y) ^ (__float_as_uint(km.y) << 31)));
+}
+
 // kernels/dice.cl:51-67 -- eye-space displacement, updated coordinates used
-// immediately; fd are the three amplitudes.
+// immediately; fd are the three amplitudes.  The twelve sines form seven
+// dependent steps: sin(k x), sin(6 x) need the same x, and sin(k y) of one
+// step and sin(k' y) of the next the same y, so five of the steps evaluate a
+// packed pair.  Positions whose arguments could leave sin2_small's range
+// (more than 2^18 from the eye's axes, or not finite) take the general sine.
 __device__ __forceinline__ float4 displace(float4 pos, const float* fd) {
+    const float reach = fadd(fadd(fabsf(pos.x), fabsf(pos.y)), fadd(fadd(fabsf(fd[0]), fabsf(fd[1])), fabsf(fd[2])));
+    if (!(reach < 262144.0f)) {
+#pragma unroll 1
+        for (int i = 0; i < 3; ++i) {
+            const float k = i == 0 ? 5.0f : i == 1 ? 7.0f : 11.0f, f = i == 0 ? fd[0] : i == 1 ? fd[1] : fd[2];
+            pos.x = ffma(mp_sinf(fmul(fmul(pos.y, k), 2.0f)), f, pos.x);
+            pos.y = ffma(mp_sinf(fmul(fmul(pos.x, k), 2.0f)), f, pos.y);
+            pos.z = ffma(fmul(mp_sinf(fmul(fmul(pos.y, k), 2.0f)), mp_sinf(fmul(fmul(pos.x, 3.0f), 2.0f))), f, pos.z);
+        }
+        return pos;
+    }
     const float k[3] = {5.0f, 7.0f, 11.0f};
+    float sy = sin_small(fmul(fmul(pos.y, k[0]), 2.0f));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        pos.x = ffma(mp_sinf(fmul(fmul(pos.y, k[i]), 2.0f)), fd[i], pos.x);
-        pos.y = ffma(mp_sinf(fmul(fmul(pos.x, k[i]), 2.0f)), fd[i], pos.y);
-        pos.z = ffma(fmul(mp_sinf(fmul(fmul(pos.y, k[i]), 2.0f)), mp_sinf(fmul(fmul(pos.x, 3.0f), 2.0f))), fd[i],
-                     pos.z);
+        pos.x = ffma(sy, fd[i], pos.x);
+        const float2 sx = sin2_small(fmul(fmul(pos.x, k[i]), 2.0f), fmul(fmul(pos.x, 3.0f), 2.0f));
+        pos.y = ffma(sx.x, fd[i], pos.y);
+        float sz;
+        if (i < 2) {
+            const float2 s = sin2_small(fmul(fmul(pos.y, k[i]), 2.0f), fmul(fmul(pos.y, k[i < 2 ? i + 1 : 2]), 2.0f));
+            sz = s.x;
+            sy = s.y;
+        } else {
+            sz = sin_small(fmul(fmul(pos.y, k[i]), 2.0f));
+        }
+        pos.z = ffma(fmul(sz, sx.y), fd[i], pos.z);
     }
     return pos;
 }
@@ -467,11 +529,13 @@ __device__ __forceinline__ float dice_param(float rmin, float rmax, int n, const
     return ffma(fsub(rmax, rmin), fmul((float)n, inv), rmin);
 }
 // Eye position from precomputed parameters and weights of one vertex.
+// DISP: 0 no displacement, 1 displaced, -1 as fr.displacement says.
+template <int DISP = -1>
 __device__ __forceinline__ float4 dice_eye_w(int type, const float* mv, const FrameDev& fr, const float4* P, float tx,
                                              float ty, float4 vw, float4 cw) {
     float4 o = (type == 0) ? eval_bezier_dice_w(P, vw, cw) : eval_gregory_dice_w(P, tx, ty, vw, cw);
     float4 pos = mul_m44v4(mv, o);
-    if (fr.displacement) pos = displace(pos, fr.fdisp);
+    if (DISP > 0 || (DISP < 0 && fr.displacement)) pos = displace(pos, fr.fdisp);
     return pos;
 }
 __device__ __forceinline__ float4 dice_eye_m(int type, const float* mv, const FrameDev& fr, const float4* P,

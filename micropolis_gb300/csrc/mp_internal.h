@@ -130,7 +130,7 @@ void launch_clear(const Framebuffer& fb, const FrameDev& fr, int with_color, cud
 void launch_raster_fused(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
                          float* mshade, BigQuad* big, long long big_cap, unsigned long long* ctrl, int grid, int group,
                          cudaStream_t s);
-int raster_fused_grid(int PS, int group);
+int raster_fused_grid(int PS, int group, int displacement);
 // bound-and-split and rasterization overlapped in one launch: the first
 // n_bns_ctas blocks run bound-and-split, then every block consumes emitted
 // sub-patches as they become ready

@@ -283,7 +283,9 @@ __device__ __forceinline__ void stage_group(FusedSmem<PS, NS>& sm, long long bas
 // next_base in buffer b ^ 1.  Three phases (dice; block bounds and the list
 // of quads that can touch a pixel; raster), each ending with a barrier after
 // which both groups' buffers are complete.
-template <int PS, int NS>
+// DISP is the frame's displacement option, compiled in: frames without it
+// carry neither its code nor its registers.
+template <int PS, int NS, bool DISP>
 __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long long base, int n,
                                              long long next_base, int n_next, const DrawDev* __restrict__ draws,
                                              const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
@@ -309,7 +311,7 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
     int k = tid / NV, nv = (tid % NV) / G, nu = (tid % NV) % G;
     for (int i = tid; i < n * NV; i += TH) {
         const float* mvp = cur.mvp[k];
-        float4 pos = dice_eye_w(cur.tv[k][0], mvp, fr, cur.cp[k], sm.tx[k][nu], sm.ty[k][nv], sm.vw[k][nu],
+        float4 pos = dice_eye_w<DISP ? 1 : 0>(cur.tv[k][0], mvp, fr, cur.cp[k], sm.tx[k][nu], sm.ty[k][nv], sm.vw[k][nu],
                                 sm.cw[k][nv]);
         int px, py;
         float dep;
@@ -434,7 +436,7 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
     __syncthreads();
 }
 
-template <int PS, int NS>
+template <int PS, int NS, bool DISP>
 __global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>())
     raster_fused_kernel(const DrawDev* __restrict__ draws, FrameDev frp, SubPatches sub, Framebuffer fb,
                         float* __restrict__ mshade, BigQuad* big, long long big_cap, unsigned long long* ctrl) {
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>()
     if (base < S) stage_group(sm, base, (int)min((long long)NS, S - base), sub, draws, fr);
     for (int b = 0; base < S; base += stride, b ^= 1) {
         const long long next = base + stride;
-        raster_group<PS, NS>(sm, b, base, (int)min((long long)NS, S - base), next,
+        raster_group<PS, NS, DISP>(sm, b, base, (int)min((long long)NS, S - base), next,
                              next < S ? (int)min((long long)NS, S - next) : 0, draws, fr, sub, fb, mshade, big,
                              big_cap, ctrl, light, frags);
     }
@@ -547,7 +549,12 @@ __global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>()
         const int n = __syncthreads_count(ready);
         if (n == 0 || __syncthreads_or(gave_up)) break;
         stage_group(sm, base, n, sub, gdraws, fr);
-        raster_group<PS, NS>(sm, 0, base, n, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl, light, frags);
+        if (fr.displacement)
+            raster_group<PS, NS, true>(sm, 0, base, n, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl, light,
+                                       frags);
+        else
+            raster_group<PS, NS, false>(sm, 0, base, n, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl, light,
+                                        frags);
     }
     frags = __reduce_add_sync(0xffffffffu, (unsigned)frags);
     if ((threadIdx.x & 31) == 0 && frags) atomicAdd(cw(ctrl, kFragments), (unsigned long long)frags);
@@ -921,12 +928,17 @@ void launch_clear(const Framebuffer& fb, const FrameDev& fr, int with_color, cud
                                                                                              reset_ctrl, roots);
 }
 
-int raster_fused_grid(int PS, int group) {
+int raster_fused_grid(int PS, int group, int displacement) {
     int g = 0;
     dispatch_group(PS, group, [&](auto t) {
         using T = decltype(t);
-        g = resident_grid(raster_fused_kernel<T::ps, T::ns>, sizeof(FusedSmem<T::ps, T::ns>),
-                          fused_threads<T::ns>());
+        auto fit = [&](auto kernel) {
+            g = resident_grid(kernel, sizeof(FusedSmem<T::ps, T::ns>), fused_threads<T::ns>());
+        };
+        if (displacement)
+            fit(raster_fused_kernel<T::ps, T::ns, true>);
+        else
+            fit(raster_fused_kernel<T::ps, T::ns, false>);
     });
     return g;
 }
@@ -936,8 +948,14 @@ void launch_raster_fused(const DrawDev* draws, const FrameDev& fr, const SubPatc
                          cudaStream_t s) {
     dispatch_group(fr.PS, group, [&](auto t) {
         using T = decltype(t);
-        raster_fused_kernel<T::ps, T::ns><<<grid, fused_threads<T::ns>(), sizeof(FusedSmem<T::ps, T::ns>), s>>>(
-            draws, fr, sub, fb, mshade, big, big_cap, ctrl);
+        auto launch = [&](auto kernel) {
+            kernel<<<grid, fused_threads<T::ns>(), sizeof(FusedSmem<T::ps, T::ns>), s>>>(draws, fr, sub, fb, mshade, big,
+                                                                                        big_cap, ctrl);
+        };
+        if (fr.displacement)
+            launch(raster_fused_kernel<T::ps, T::ns, true>);
+        else
+            launch(raster_fused_kernel<T::ps, T::ns, false>);
     });
 }
 
