@@ -1,13 +1,12 @@
 // Bound-and-split kernels.
 //
 // Batched path: one persistent launch per frame over every draw's patches.
-// Warps hold queue tickets; a ticket below the root count is a root range
-// (0,0)-(1,1) of one patch, any other ticket is a slot that another warp
-// fills with a split child.  Emitted sub-patches and children are compacted
-// with warp ballots (one atomic per warp and role).  Termination: an
-// outstanding-work counter updated with one net atomic per warp step; the warp
-// that brings it to zero raises the done flag.  Every wait is bounded and
-// reports kErrTimeout instead of hanging.
+// Warps work depth first on stacks of their own in shared memory and hand
+// bundles of split pairs to warps without work (mp_bns_loop.cuh).  Emitted
+// sub-patches and children are compacted with warp ballots.  Termination: a
+// counter of unfinished units of work (roots, bundles); the warp that brings
+// it to zero raises the done flag.  Every wait is bounded and reports
+// kErrTimeout instead of hanging.
 //
 // Plain path: the reference's BOUNDED structure
 // (src/Reyes/BoundNSplitCLBounded.cpp:170-214, kernels/bound_n_split_multipass.cl):
@@ -26,7 +25,8 @@ namespace {
 
 
 constexpr int kBnsBlock = 128;
-constexpr int kBnsSmemDraws = 64;
+constexpr int kBnsSmemDraws = 8;
+constexpr size_t kBnsSmem = bns_smem<kBnsBlock, kStackPairs>();
 
 template <int CRIT>
 __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev* __restrict__ gdraws,
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev
                                                                    long long spin_limit) {
     // draw constants staged in shared memory when they fit
     __shared__ DrawDev s_draws[kBnsSmemDraws];
-    __shared__ float s_pts[27 * kBnsBlock];   // nine bound samples per thread
+    extern __shared__ __align__(16) float s_bns[];
     const bool staged = n_draws <= kBnsSmemDraws;
     if (staged) {
         const int words = n_draws * (int)(sizeof(DrawDev) / 4);
@@ -44,14 +44,16 @@ __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev
             reinterpret_cast<int*>(s_draws)[i] = __ldg(reinterpret_cast<const int*>(gdraws) + i);
         __syncthreads();
     }
-    bns_warp_loop<CRIT, CRIT == 0 ? kBnsBlock : 0>(staged ? s_draws : gdraws, root_prefix, n_draws, fr, q, out, nullptr,
-                                                   ctrl, spin_limit, s_pts);
+    // consecutive warp numbers on different SMs: the first roots spread over the chip
+    const int warp = (int)(blockIdx.x + gridDim.x * (threadIdx.x >> 5));
+    bns_warp_loop<CRIT, kStackPairs>(staged ? s_draws : gdraws, root_prefix, n_draws, fr, q, out, nullptr, ctrl,
+                                     spin_limit, s_bns, warp, (int)(gridDim.x * (kBnsBlock / 32)));
 }
 
 // ---------------------------------------------------------------------------
 // Plain path
 
-__global__ void bns_init_stack_kernel(Queue stack, int draw, int n) {
+__global__ void bns_init_stack_kernel(RangeStack stack, int draw, int n) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     // src/Reyes/BoundNSplitCLCPU.cpp:41-44: one root range per patch
@@ -69,7 +71,7 @@ constexpr unsigned long long kValMask = (1ull << 62) - 1;
 // bound kernel of one pass: decision, copy of the range to the pads, packed
 // scan key (draw + split << 31); also clears the scan state of this pass.
 template <int CRIT>
-__global__ void bns_pass_bound_kernel(const DrawDev* __restrict__ draws, FrameDev fr, Queue stack,
+__global__ void bns_pass_bound_kernel(const DrawDev* __restrict__ draws, FrameDev fr, RangeStack stack,
                                       long long offset, int batch, float4* pad_range, uint2* pad_meta,
                                       unsigned char* dec_out, unsigned long long* keys,
                                       unsigned long long* scan_state, long long n_tiles,
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(kScanBlock) scan_kernel(const unsigned long lo
 // to the output list, the two halves of each split back onto the stack.
 __global__ void bns_pass_move_kernel(const float4* __restrict__ pad_range, const uint2* __restrict__ pad_meta,
                                      const unsigned char* __restrict__ dec_in,
-                                     const unsigned long long* __restrict__ prefix, int batch, Queue stack,
+                                     const unsigned long long* __restrict__ prefix, int batch, RangeStack stack,
                                      long long offset, SubPatches out, long long out_base,
                                      unsigned long long* ctrl) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -242,10 +244,14 @@ int bns_persistent_grid(int criterion) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto fit = [&](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBnsSmem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBnsBlock, kBnsSmem);
+    };
     if (criterion == 1)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bns_persistent_kernel<1>, kBnsBlock, 0);
+        fit(bns_persistent_kernel<1>);
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bns_persistent_kernel<0>, kBnsBlock, 0);
+        fit(bns_persistent_kernel<0>);
     if (per_sm < 1) per_sm = 1;
     return sms * per_sm;
 }
@@ -254,19 +260,21 @@ void launch_bns_persistent(const DrawDev* draws, const int* root_prefix, int n_d
                            const Queue& q, const SubPatches& out, unsigned long long* ctrl, int grid,
                            long long spin_limit, cudaStream_t s) {
     if (fr.criterion == 1)
-        bns_persistent_kernel<1><<<grid, kBnsBlock, 0, s>>>(draws, root_prefix, n_draws, fr, q, out, ctrl, spin_limit);
+        bns_persistent_kernel<1><<<grid, kBnsBlock, kBnsSmem, s>>>(draws, root_prefix, n_draws, fr, q, out, ctrl,
+                                                                    spin_limit);
     else
-        bns_persistent_kernel<0><<<grid, kBnsBlock, 0, s>>>(draws, root_prefix, n_draws, fr, q, out, ctrl, spin_limit);
+        bns_persistent_kernel<0><<<grid, kBnsBlock, kBnsSmem, s>>>(draws, root_prefix, n_draws, fr, q, out, ctrl,
+                                                                    spin_limit);
 }
 
-void launch_bns_init_stack(const Queue& stack, int draw, int n_patches, cudaStream_t s) {
+void launch_bns_init_stack(const RangeStack& stack, int draw, int n_patches, cudaStream_t s) {
     if (n_patches <= 0) return;
     bns_init_stack_kernel<<<(n_patches + 255) / 256, 256, 0, s>>>(stack, draw, n_patches);
 }
 
 long long scan_state_words(long long n) { return (n + kScanTileItems - 1) / kScanTileItems + 1; }
 
-void launch_bns_pass(const DrawDev* draws, const FrameDev& fr, const Queue& stack, long long offset, int batch,
+void launch_bns_pass(const DrawDev* draws, const FrameDev& fr, const RangeStack& stack, long long offset, int batch,
                      float4* pad_range, uint2* pad_meta, unsigned char* dec, unsigned long long* keys,
                      unsigned long long* scan_state, const SubPatches& out, long long out_base,
                      unsigned long long* ctrl, long long spin_limit, cudaStream_t s) {

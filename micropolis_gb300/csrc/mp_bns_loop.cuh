@@ -37,12 +37,13 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
-// The per-frame reset of the bound-and-split control words: roots tickets
-// filled and outstanding, counters cleared, the frame epoch advanced.
+// The per-frame reset of the bound-and-split control words: every root
+// outstanding, counters cleared, the frame epoch advanced.
 __device__ __forceinline__ void bns_reset(unsigned long long* ctrl, long long roots) {
-    *cw(ctrl, kQTail) = ((unsigned long long)roots << 32) | (unsigned long long)roots;
+    *cw(ctrl, kQTail) = 0;
     *cw(ctrl, kQHead) = 0;
-    *cw(ctrl, kOutstanding) = 0;
+    *cw(ctrl, kRootHead) = 0;
+    *cw(ctrl, kOutstanding) = (unsigned long long)roots;
     *cw(ctrl, kOutCount) = 0;
     *cw(ctrl, kDone) = roots == 0 ? 1 : 0;
     *cw(ctrl, kStatus) = 0;
@@ -60,130 +61,282 @@ __device__ __forceinline__ void set_status(unsigned long long* ctrl, int code) {
     atomicCAS(cw(ctrl, kStatus), 0ull, (unsigned long long)code);
 }
 
-// kQTail packs two counters updated by one atomic: the high 32 bits count
-// queue tickets ever filled (roots included), the low 32 bits the items pushed
-// but not yet finished.  A warp step adds (2*splits << 32) + (2*splits -
-// processed); the borrow of a negative low part is cancelled by the carry.
+// kOutstanding packs two counters updated by one atomic: the low 32 bits
+// count units of work (root ranges, published bundles) whose split trees are
+// not finished, the high 32 bits the ranges split so far.
 constexpr unsigned long long kLow32 = 0xffffffffull;
 
-constexpr unsigned long long kNoTicket = ~0ull;
+// A warp's stack of pairs (the two children of a split) in shared memory: a
+// ring of C pairs and, beside it, a column of scratch for each lane's range;
+// word w of ring slot i at s[w * stack_stride<C>() + i], of lane l's scratch
+// at s[w * stack_stride<C>() + C + l].
+//   words 0-26   the parent's nine bound samples (spi() order), CPU criterion
+//   words 27-30  the parent's range
+//   word 31      patch id | split direction << 31 (1: x halved), GPU criterion
+//   word 32      draw | parent's depth << 24
+//   word 33      the parent's split path
+// Bundles of the global queue hold kBundlePairs pairs with the same words,
+// word w of pair p at kBundlePairs * w + p, then the number of pairs.
+constexpr int kPairWords = 34;
+constexpr int kStackPairs = 64;        // ring size of the standalone kernel
+constexpr int kStackPairsFrame = 32;   // and of the overlapped kernel, whose blocks also hold the raster's buffers
+// an odd stride: lanes on neighbouring words of one column use different banks
+template <int C>
+constexpr int stack_stride() {
+    return C + 33;
+}
+
+// Shared memory of the warp loop in a block of `threads`.
+template <int THREADS, int C>
+constexpr size_t bns_smem() {
+    return (THREADS / 32) * kPairWords * stack_stride<C>() * sizeof(float);
+}
 
 // Runs one warp's share of a frame's bound-and-split until the done flag is
 // raised.  Emitted sub-patches go to `out`; when out_seq is given, each
 // emitted slot is also marked with the frame's epoch (release) for consumers
 // that run concurrently.  CRIT selects the bound criterion (bns_decide).
-// With the CPU criterion and ST > 0 (the block's thread count), children take
-// six of their nine bound samples from the parent through the queue's pts
-// records (which must exist); `pts` is shared memory of 27 floats per thread
-// (point layout of spi()).
-template <int CRIT, int ST>
+// `warp` is the warp's number among the n_warps that run the loop.
+//
+// A warp works depth first on a stack of its own: a step takes up to 16
+// pairs (32 ranges, one per lane) and, while few pairs are left and roots
+// remain, roots on the lanes left over; every range that splits pushes one
+// pair.  Nothing is exchanged with other warps meanwhile but the output
+// count (one atomic per step).  Warps without work take a ticket of the
+// bundle queue and wait for its slot.  A warp with pairs to spare gives the
+// oldest (shallowest) ones away, up to kBundlePairs at a time, while tickets
+// outnumber bundles, and whenever its ring could overflow.  With the CPU criterion a step has three parts:
+//   the two lanes of a pair find its split direction, one the three lengths
+//   along x, the other those along y (only ranges that split pay for them);
+//   the new samples of all the step's ranges (three of a child, the other six
+//   are its parent's, nine of a root) are dealt to the lanes one by one, so
+//   a step of ten ranges takes a third of the time of a full one and lanes
+//   do not diverge by split direction;
+//   each lane bounds its range's nine points.
+template <int CRIT, int C>
 __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* __restrict__ root_prefix, int n_draws,
                                               const FrameDev& fr, const Queue& q, const SubPatches& out,
                                               unsigned* out_seq, unsigned long long* ctrl, long long spin_limit,
-                                              float* pts) {
-    constexpr bool inherit = CRIT == 0 && ST > 0;
-    constexpr int st = ST;
-    float* sp = inherit ? pts + threadIdx.x : nullptr;
+                                              float* smem, int warp, int n_warps) {
+    static_assert(C >= 32, "a step adds up to 16 pairs, or 32 to an empty ring");
+    // Pairs are given to waiting warps when more than kGiveAbove are left, and
+    // kKeep stay (a step of 16 ranges: on 1,024 Gregory patches bound-and-split
+    // takes 0.145 ms, 0.174 ms when 16 stay); the ring is relieved when the
+    // next step's pairs might not fit.
+    constexpr int kGiveAbove = 11, kKeep = 8, kFull = C - 16;
+    auto wrap = [](int i) { return i >= C ? i - C : i; };
+    constexpr bool samples = CRIT == 0;
+    constexpr int S = stack_stride<C>();
     const int lane = threadIdx.x & 31;
+    float* ring = smem + (threadIdx.x >> 5) * (kPairWords * S);
     const unsigned epoch = (unsigned)*(volatile unsigned long long*)cw(ctrl, kEpoch);
-    const unsigned long long R = *(volatile unsigned long long*)cw(ctrl, kRoots);
-    unsigned long long ticket = kNoTicket;
-    long long idle = 0;
-    unsigned sleep_ns = 32;
-    unsigned max_depth = 0;   // deepest emitted sub-patch of this warp so far (lane 0)
+    const long long R = (long long)*(volatile unsigned long long*)cw(ctrl, kRoots);
+    // the first roots and tickets are dealt by warp number, without atomics:
+    // the lowest `busy` warps start with `share` roots each
+    const int share = (int)min(32ll, (R + n_warps - 1) / n_warps);
+    const long long busy = share > 0 ? min((long long)n_warps, (R + share - 1) / share) : 0;
+    const bool more_roots = (long long)n_warps * share < R;   // the rest is taken with atomics
+    long long root = (long long)warp * share;                 // this warp's next roots: [root, root_end)
+    long long root_end = max(root, min(root + share, R));
+    bool roots_left = more_roots;
+    unsigned units = (unsigned)(root_end - root);             // units taken since the last report
+    unsigned splits = 0;                                      // ranges split since the last report
+    bool first_ticket = warp >= busy;
+    int bottom = 0, n = 0;    // ring: pairs bottom .. bottom + n - 1 (mod C)
+    unsigned max_depth = 0;   // deepest emitted sub-patch of this warp so far
     while (true) {
-        // hand new tickets to the lanes that have none
-        unsigned need = __ballot_sync(0xffffffffu, ticket == kNoTicket);
-        if (need) {
-            int leader = __ffs(need) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(cw(ctrl, kQHead), (unsigned long long)__popc(need));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (ticket == kNoTicket) ticket = base + __popc(need & lanemask_lt());
+        if (roots_left && root >= root_end && n < 8) {
+            unsigned long long t = 0;
+            if (lane == 0) t = atomicAdd(cw(ctrl, kRootHead), (unsigned long long)share);
+            root = (long long)n_warps * share + (long long)__shfl_sync(0xffffffffu, t, 0);
+            root_end = max(root, min(root + share, R));
+            units += (unsigned)(root_end - root);
+            roots_left = root < root_end;
         }
-        bool ready = false;
-        if (ticket < R) {
-            ready = true;
-        } else {
-            unsigned long long slot = ticket - R;
-            if ((long long)slot < q.capacity) ready = ld_acquire_u32(q.seq + slot) == epoch;
-        }
-        unsigned rmask = __ballot_sync(0xffffffffu, ready);
-        if (rmask == 0) {
-            unsigned long long done = 0;
-            if (lane == 0) done = *(volatile unsigned long long*)cw(ctrl, kDone);
-            done = __shfl_sync(0xffffffffu, done, 0);
-            if (done) break;
-            if (++idle > spin_limit) {
-                if (lane == 0) {
-                    set_status(ctrl, kErrTimeout);
-                    st_release_u64(cw(ctrl, kDone), 1ull);
+        if (n == 0 && root >= root_end) {
+            // out of work: report, then wait (bounded) for a bundle
+            long long slot = warp - busy;
+            int got = 0;
+            if (lane == 0) {
+                if (units) {
+                    const unsigned long long delta = ((unsigned long long)splits << 32) - units;
+                    if (((atomicAdd(cw(ctrl, kOutstanding), delta) + delta) & kLow32) == 0)
+                        st_release_u64(cw(ctrl, kDone), 1ull);
                 }
-                break;
+                if (!first_ticket) slot = n_warps - busy + (long long)atomicAdd(cw(ctrl, kQHead), 1ull);
+                long long idle = 0;
+                unsigned sleep_ns = 32;
+                while (true) {
+                    if (slot < q.capacity && ld_acquire_u32(q.seq + slot) == epoch) {
+                        got = 1;
+                        break;
+                    }
+                    if (*(volatile unsigned long long*)cw(ctrl, kDone)) break;
+                    if (++idle > spin_limit) {
+                        set_status(ctrl, kErrTimeout);
+                        st_release_u64(cw(ctrl, kDone), 1ull);
+                        break;
+                    }
+                    __nanosleep(sleep_ns);
+                    if (sleep_ns < 512) sleep_ns <<= 1;
+                }
             }
-            __nanosleep(sleep_ns);
-            if (sleep_ns < 512) sleep_ns <<= 1;
-            continue;
+            got = __shfl_sync(0xffffffffu, got, 0);
+            if (!got) break;
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            first_ticket = false;
+            units = 1;
+            splits = 0;
+            const unsigned* rec = q.words + slot * kBundleWords;
+            n = (int)__ldcg(rec + kPairWords * kBundlePairs);
+            bottom = 0;
+            for (int i = lane; i < kPairWords * kBundlePairs; i += 32)
+                ring[(i / kBundlePairs) * S + (i % kBundlePairs)] = __uint_as_float(__ldcg(rec + i));
+            __syncwarp();
         }
-        idle = 0;
-        sleep_ns = 32;
+        // this step's ranges: pairs from the top of the ring, then roots
+        const int pop = min(n, 16);
+        const int n_root = (int)min((long long)(32 - 2 * pop), root_end - root);
+        // tickets taken and bundles published so far, for the hand-over below
+        // (loaded here so that the bounds cover the latency)
+        const bool may_give = n + pop + n_root > kGiveAbove;
+        unsigned long long taken = 0, filled = 0;
+        if (may_give && lane == 0) {
+            taken = *(volatile unsigned long long*)cw(ctrl, kQHead);
+            filled = *(volatile unsigned long long*)cw(ctrl, kQTail);
+        }
+        const int src = wrap(bottom + max(n - 1 - (lane >> 1), 0));
+        const bool child = lane < 2 * pop, active = lane < 2 * pop + n_root;
+        const int half = lane & 1;
         float4 r = make_float4(0.f, 0.f, 1.f, 1.f);
         int pid = 0, draw = 0, depth = 0;
         unsigned path = 0;
+        bool split_x = false;   // of the pair's parent
         int dec = -1;
-        if (ready) {
-            int flag = kInheritNone;
-            if (ticket < R) {
-                // root: find the draw whose patch range holds this ticket
-                int lo = 0, hi = n_draws - 1;
-                while (lo < hi) {
-                    int mid = (lo + hi + 1) >> 1;
-                    if ((unsigned long long)__ldg(root_prefix + mid) <= ticket) lo = mid; else hi = mid - 1;
-                }
-                draw = lo;
-                pid = (int)(ticket - (unsigned long long)__ldg(root_prefix + lo));
-            } else {
-                unsigned long long slot = ticket - R;
-                r = __ldcg(q.range + slot);
-                uint2 m = __ldcg(q.meta + slot);
-                pid = (int)m.x;
-                draw = (int)(m.y & 0xffffffu);
-                depth = (int)(m.y >> 24);
-                if (q.path) path = __ldcg(q.path + slot);
-                if (inherit) flag = load_inherited(q.pts + slot * kPtsPerSlot, sp, st);
-            }
-            if (inherit)
-                dec = bns_decide_inherit(draws[draw], fr, pid, r, depth, flag, sp, st);
-            else
-                dec = bns_decide<CRIT>(draws[draw], fr, pid, r, depth);
+        float length = 0.0f;
+        if (samples && child) length = split_length(ring + src, S, half);
+        if (samples) {
+            const float other = __shfl_xor_sync(0xffffffffu, length, 1);
+            split_x = !(half ? other < length : length < other);   // vlen < hlen halves y
         }
-        // One lane issues the step's three independent atomics back to back,
-        // so their round trips overlap: output slots for emitted sub-patches,
-        // the packed ticket / outstanding-work update for split children (see
-        // kQTail above), and the next tickets of the lanes finished here.
+        if (child) {
+            const float* it = ring + src;
+            const float4 pr = make_float4(it[27 * S], it[28 * S], it[29 * S], it[30 * S]);
+            const unsigned w31 = __float_as_uint(it[31 * S]), w32 = __float_as_uint(it[32 * S]);
+            if (!samples) split_x = w31 >> 31;
+            pid = (int)(w31 & 0x7fffffffu);
+            draw = (int)(w32 & 0xffffffu);
+            depth = (int)(w32 >> 24) + 1;
+            path = __float_as_uint(it[33 * S]);
+            float4 c0, c1;
+            split_children(pr, split_x ? kSplitX : kSplitY, c0, c1);
+            r = half ? c1 : c0;
+            // the high half sets bit 31 - parent's depth (paths deeper than 32 keep their first 32 bits)
+            if (half && depth <= 32) path |= 0x80000000u >> (depth - 1);
+        } else if (active) {
+            // root: find the draw whose patch range holds it
+            const long long rt = root + (lane - 2 * pop);
+            int lo = 0, hi = n_draws - 1;
+            while (lo < hi) {
+                int mid = (lo + hi + 1) >> 1;
+                if (__ldg(root_prefix + mid) <= rt) lo = mid; else hi = mid - 1;
+            }
+            draw = lo;
+            pid = (int)(rt - __ldg(root_prefix + lo));
+        }
+        F3 pts[9];   // the range's samples, (iu, iv) at 3 * iv + iu (CPU criterion)
+        if (samples) {
+            // past the depth where sample parameters stay exact nothing is shared
+            const bool share_pts = !__any_sync(0xffffffffu, child && depth > kInheritMaxDepth);
+            const int flag = !child || !share_pts ? kInheritNone : split_x ? kInheritX : kInheritY;
+            const int n_ct = 2 * pop * (share_pts ? 3 : 9), n_t = n_ct + 9 * n_root;
+#pragma unroll 1
+            for (int t0 = 0; t0 < n_t; t0 += 32) {
+                const int t = t0 + lane;
+                int q, k;   // sample k of lane q's range
+                if (share_pts && t < n_ct) {
+                    q = t / 3;
+                    k = t - 3 * q;
+                } else {
+                    const int u = share_pts ? t - n_ct : t;
+                    q = u / 9;
+                    k = u - 9 * q;
+                    if (share_pts) q += 2 * pop;
+                }
+                q &= 31;
+                const float4 rq = make_float4(__shfl_sync(0xffffffffu, r.x, q), __shfl_sync(0xffffffffu, r.y, q),
+                                              __shfl_sync(0xffffffffu, r.z, q), __shfl_sync(0xffffffffu, r.w, q));
+                const int pq = __shfl_sync(0xffffffffu, pid, q);
+                const int dq = __shfl_sync(0xffffffffu, draw | (flag << 24), q);
+                if (t < n_t) {
+                    const int fq = dq >> 24;
+                    const int iu = fq == kInheritX ? 1 : fq == kInheritY ? k : k % 3;
+                    const int iv = fq == kInheritX ? k : fq == kInheritY ? 1 : k / 3;
+                    const float sv = fadd(rq.x, fmul(fmul(fsub(rq.z, rq.x), (float)iu), 0.5f));
+                    const float su = fadd(rq.y, fmul(fmul(fsub(rq.w, rq.y), (float)iv), 0.5f));
+                    const F3 p = bound_sample(draws[dq & 0xffffff], pq, sv, su);
+                    float* to = ring + C + q + spi(iu, iv, 0, S);
+                    to[0] = p.x;
+                    to[S] = p.y;
+                    to[2 * S] = p.z;
+                }
+            }
+            __syncwarp();
+            if (active) {
+#pragma unroll
+                for (int iv = 0; iv < 3; ++iv)
+#pragma unroll
+                    for (int iu = 0; iu < 3; ++iu) {
+                        // the child's line 0 / 2 is the parent's line half / half + 1
+                        int at = C + lane + spi(iu, iv, 0, S);
+                        if (flag == kInheritX && iu != 1) at = src + spi(half + (iu >> 1), iv, 0, S);
+                        if (flag == kInheritY && iv != 1) at = src + spi(iu, half + (iv >> 1), 0, S);
+                        pts[3 * iv + iu] = F3{ring[at], ring[at + S], ring[at + 2 * S]};
+                    }
+                dec = bns_decide_points(draws[draw], fr, pts, depth);
+            }
+        } else if (active) {
+            dec = bns_decide<CRIT>(draws[draw], fr, pid, r, depth);
+        }
+        root += n_root;
+        // emitted sub-patches: slots from one atomic, whose round trip the pushes below overlap
         const unsigned emask = __ballot_sync(0xffffffffu, dec == kDraw);
         const bool split = dec == kSplitX || dec == kSplitY;
         const unsigned smask = __ballot_sync(0xffffffffu, split);
-        const long long n_child = 2ll * __popc(smask);
-        const long long net = n_child - (long long)__popc(rmask);
         const unsigned emit_depth = __reduce_max_sync(0xffffffffu, dec == kDraw ? (unsigned)depth : 0u);
-        unsigned long long obase = 0, old = 0, tbase = 0;
-        if (lane == 0) {
-            if (emask) obase = atomicAdd(cw(ctrl, kOutCount), (unsigned long long)__popc(emask));
-            if (emit_depth > max_depth) {
-                // the sort packs the frame's keys into root bits above this many path bits
-                max_depth = emit_depth;
-                atomicMax(cw(ctrl, kMaxDepth), (unsigned long long)emit_depth);
-            }
-            old = atomicAdd(cw(ctrl, kQTail), ((unsigned long long)n_child << 32) + (unsigned long long)net);
-            tbase = atomicAdd(cw(ctrl, kQHead), (unsigned long long)__popc(rmask));
+        unsigned long long obase = 0;
+        if (lane == 0 && emask) obase = atomicAdd(cw(ctrl, kOutCount), (unsigned long long)__popc(emask));
+        if (emit_depth > max_depth) {
+            // the sort packs the frame's keys into root bits above this many path bits
+            max_depth = emit_depth;
+            if (lane == 0) atomicMax(cw(ctrl, kMaxDepth), (unsigned long long)emit_depth);
         }
+        // split ranges: one pair each, once every lane has read the popped pairs
+        __syncwarp();
+        n -= pop;
+        if (split) {
+            float* it = ring + wrap(bottom + n + __popc(smask & lanemask_lt()));
+            if (samples) {
+#pragma unroll
+                for (int j = 0; j < 9; ++j) {
+                    it[3 * j * S] = pts[j].x;
+                    it[(3 * j + 1) * S] = pts[j].y;
+                    it[(3 * j + 2) * S] = pts[j].z;
+                }
+            }
+            it[27 * S] = r.x;
+            it[28 * S] = r.y;
+            it[29 * S] = r.z;
+            it[30 * S] = r.w;
+            it[31 * S] = __uint_as_float((unsigned)pid | (!samples && dec == kSplitX ? 0x80000000u : 0u));
+            it[32 * S] = __uint_as_float((unsigned)draw | ((unsigned)depth << 24));
+            it[33 * S] = __uint_as_float(path);
+        }
+        n += __popc(smask);
+        splits += (unsigned)__popc(smask);
         obase = __shfl_sync(0xffffffffu, obase, 0);
-        old = __shfl_sync(0xffffffffu, old, 0);
-        tbase = __shfl_sync(0xffffffffu, tbase, 0);
-        // emitted sub-patches
         if (dec == kDraw) {
-            unsigned long long o = obase + __popc(emask & lanemask_lt());
+            const unsigned long long o = obase + __popc(emask & lanemask_lt());
             if ((long long)o < out.capacity) {
                 out.range[o] = r;
                 out.meta[o] = make_int2(pid, draw);
@@ -194,48 +347,44 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
                 set_status(ctrl, kErrOverflow);
             }
         }
-        bool fits = true;
-        if (split) {
-            const unsigned long long t0 = (old >> 32) + 2ull * __popc(smask & lanemask_lt());
-            const unsigned long long s0 = t0 - R;
-            fits = (long long)(s0 + 1) < q.capacity;
-            if (fits) {
-                float4 c0, c1;
-                split_children(r, dec, c0, c1);
-                const unsigned meta_y = (unsigned)draw | ((unsigned)(depth + 1) << 24);
-                q.range[s0] = c0;
-                q.range[s0 + 1] = c1;
-                q.meta[s0] = make_uint2((unsigned)pid, meta_y);
-                q.meta[s0 + 1] = make_uint2((unsigned)pid, meta_y);
-                if (q.path) {
-                    // the high half sets bit 31 - depth (paths deeper than 32 keep their first 32 bits)
-                    q.path[s0] = path;
-                    q.path[s0 + 1] = depth < 32 ? path | (0x80000000u >> depth) : path;
+        __syncwarp();
+        // hand the oldest pairs over: to waiting warps, and what crowds the ring
+        long long wanting = 0;
+        if (may_give && n > kGiveAbove) {
+            if ((long long)filled < q.capacity) wanting = (long long)taken + (n_warps - busy) - (long long)filled;
+            wanting = __shfl_sync(0xffffffffu, wanting, 0);
+        }
+        while (n > kFull || (wanting > 0 && n > kGiveAbove)) {
+            const int give = min(kBundlePairs, n - kKeep);
+            unsigned long long slot = 0;
+            if (lane == 0) {
+                slot = atomicAdd(cw(ctrl, kQTail), 1ull);
+                if ((long long)slot < q.capacity) atomicAdd(cw(ctrl, kOutstanding), 1ull);
+            }
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            if ((long long)slot < q.capacity) {
+                unsigned* rec = q.words + slot * kBundleWords;
+                for (int i = lane; i < kPairWords * kBundlePairs; i += 32)
+                    if (i % kBundlePairs < give)
+                        rec[i] = __float_as_uint(
+                            ring[(i / kBundlePairs) * S + wrap(bottom + i % kBundlePairs)]);
+                if (lane == 0) rec[kPairWords * kBundlePairs] = (unsigned)give;
+                __syncwarp();
+                if (lane == 0) {
+                    // release: the pairs and the outstanding count are visible before the slot's epoch
+                    fence_acq_rel_gpu();
+                    st_relaxed_u32(q.seq + slot, epoch);
                 }
-                if (inherit) {
-                    store_inherited(q.pts + s0 * kPtsPerSlot, dec, 0, depth + 1, sp, st);
-                    store_inherited(q.pts + (s0 + 1) * kPtsPerSlot, dec, 1, depth + 1, sp, st);
-                }
-                // release: the item stores above are visible before the slots' epochs
-                fence_acq_rel_gpu();
-                st_relaxed_u32(q.seq + s0, epoch);
-                st_relaxed_u32(q.seq + s0 + 1, epoch);
+            } else if (n > kFull) {
+                set_status(ctrl, kErrOverflow);   // no room: the pairs are lost, the host grows the queue
             } else {
-                set_status(ctrl, kErrOverflow);
+                break;                            // no room, but they can stay here
             }
+            bottom = wrap(bottom + give);
+            n -= give;
+            --wanting;
         }
-        const unsigned lost = __ballot_sync(0xffffffffu, !fits);
-        if (lane == 0) {
-            long long remaining = (long long)(old & kLow32) + net;
-            if (lost) {
-                // children that found no slot are never processed: take them back
-                const long long back = -2ll * __popc(lost);
-                unsigned long long o2 = atomicAdd(cw(ctrl, kQTail), (unsigned long long)back);
-                remaining = (long long)(o2 & kLow32) + back;
-            }
-            if (remaining == 0) st_release_u64(cw(ctrl, kDone), 1ull);
-        }
-        if (ready) ticket = tbase + __popc(rmask & lanemask_lt());
+        __syncwarp();
     }
 }
 

@@ -73,7 +73,7 @@ struct mp_ctx {
     Framebuffer fb{};
 
     // plain path
-    Queue stack{};
+    RangeStack stack{};
     float4* pad_range = nullptr;
     uint2* pad_meta = nullptr;
     unsigned char* dec = nullptr;
@@ -169,7 +169,8 @@ void perspective(float fovy_rad, float aspect, float zn, float zf, float* m) {
 }
 
 // first-frame guesses; both grow (and the frame is rendered again) on overflow
-long long auto_queue_cap(long long roots) { return std::min(std::max(1LL << 22, roots * 32), 1LL << 28); }
+// (the queue holds bundles of up to 2 * kBundlePairs ranges, only those that change warps)
+long long auto_queue_cap(long long roots) { return std::min(std::max(1LL << 15, roots / 2), 1LL << 20); }
 long long auto_sub_cap(long long roots) { return std::min(std::max(1LL << 21, roots * 64), 1LL << 26); }
 
 void free_sorted(mp_ctx* c) {
@@ -190,17 +191,11 @@ mp_status grow_queue(mp_ctx* c, long long need) {
     if (need <= c->q.capacity) return MP_OK;
     c->graph_stale = true;
     long long cap = std::max(need, c->q.capacity * 2);
-    cudaFree(c->q.range);
-    cudaFree(c->q.meta);
+    cudaFree(c->q.words);
     cudaFree(c->q.seq);
-    cudaFree(c->q.pts);
-    cudaFree(c->q.path);
     c->q = Queue{};
-    CK(dalloc(&c->q.range, cap));
-    CK(dalloc(&c->q.meta, cap));
+    CK(dalloc(&c->q.words, cap * kBundleWords));
     CK(dalloc(&c->q.seq, cap));
-    CK(dalloc(&c->q.pts, cap * kPtsPerSlot));
-    CK(dalloc(&c->q.path, cap));
     CK(cudaMemsetAsync(c->q.seq, 0, sizeof(unsigned) * (size_t)cap, c->stream));
     c->q.capacity = cap;
     return MP_OK;
@@ -319,6 +314,11 @@ mp_status check_status(mp_ctx* c, unsigned long long st) {
 
 unsigned long long hc(const mp_ctx* c, int w) { return c->h_ctrl[w * kCtrlStride]; }
 
+// Ranges bounded in the last batched frame: the roots and two per split.
+long long bounded_ranges(const mp_ctx* c) {
+    return (long long)hc(c, kRoots) + 2 * (long long)(hc(c, kOutstanding) >> 32);
+}
+
 mp_status read_ctrl(mp_ctx* c) {
     CK(cudaMemcpyAsync(c->h_ctrl, c->ctrl, sizeof(unsigned long long) * kNumCtrl * kCtrlStride,
                        cudaMemcpyDeviceToHost, c->stream));
@@ -350,7 +350,7 @@ mp_status ensure_plain(mp_ctx* c, long long need_stack) {
     }
     if (need_stack > c->stack.capacity) {
         long long cap = std::max(need_stack, c->stack.capacity * 2);
-        Queue n{};
+        RangeStack n{};
         CK(dalloc(&n.range, cap));
         CK(dalloc(&n.meta, cap));
         n.capacity = cap;
@@ -570,7 +570,7 @@ mp_status capture_frame(mp_ctx* c, int n, long long roots) {
     c->graph_draws = n;
     c->graph_roots = roots;
     c->graph_stale = false;
-    c->graph_key[0] = c->q.range;
+    c->graph_key[0] = c->q.words;
     c->graph_key[1] = c->sub.range;
     c->graph_key[2] = c->big;
     c->graph_key[3] = c->d_draws;
@@ -592,7 +592,9 @@ mp_status batched_frame(mp_ctx* c) {
         c->h_root_prefix[i + 1] = (int)roots;
     }
     if (roots >= (1LL << 31)) return fail(c, MP_ERR_INVALID_ARG, "more than 2^31 patches in one frame");
-    long long qcap = c->opt.queue_capacity > 0 ? c->opt.queue_capacity : auto_queue_cap(roots);
+    // queue_capacity counts ranges, the queue bundles of them
+    long long qcap = c->opt.queue_capacity > 0 ? (c->opt.queue_capacity + 2 * kBundlePairs - 1) / (2 * kBundlePairs)
+                                               : auto_queue_cap(roots);
     long long scap = c->opt.subpatch_capacity > 0 ? c->opt.subpatch_capacity : auto_sub_cap(roots);
     if ((st = grow_queue(c, qcap)) || (st = grow_sub(c, scap, false)) || (st = grow_big(c, 1 << 16)) ||
         (st = ensure_mshade(c)))
@@ -612,7 +614,7 @@ mp_status batched_frame(mp_ctx* c) {
             CK(cudaGetLastError());
         } else {
             if (!c->graph || c->graph_stale || c->graph_draws != n || c->graph_roots != roots ||
-                c->graph_key[0] != c->q.range || c->graph_key[1] != c->sub.range || c->graph_key[2] != c->big ||
+                c->graph_key[0] != c->q.words || c->graph_key[1] != c->sub.range || c->graph_key[2] != c->big ||
                 c->graph_key[3] != c->d_draws || c->graph_key[4] != c->mshade || c->graph_key[5] != c->sorted.range) {
                 st = capture_frame(c, n, roots);
                 if (st) return st;
@@ -629,7 +631,7 @@ mp_status batched_frame(mp_ctx* c) {
             break;
         }
         // regrow what overflowed and render the frame again
-        long long pushed = (long long)(hc(c, kQTail) >> 32) - roots;
+        long long pushed = (long long)hc(c, kQTail);
         long long outc = (long long)hc(c, kOutCount);
         long long bigc = (long long)hc(c, kBigCount);
         if (pushed > c->q.capacity && (st = grow_queue(c, pushed + pushed / 2))) return st;
@@ -639,7 +641,7 @@ mp_status batched_frame(mp_ctx* c) {
         if (attempt == 7) {
             char msg[256];
             std::snprintf(msg, sizeof(msg),
-                          "capacity still exceeded after regrowth (queue %lld/%lld, sub-patches %lld/%lld, "
+                          "capacity still exceeded after regrowth (queue bundles %lld/%lld, sub-patches %lld/%lld, "
                           "slow quads %lld/%lld)",
                           pushed, c->q.capacity, outc, c->sub.capacity, bigc, c->big_cap);
             return fail(c, MP_ERR_OVERFLOW, msg);
@@ -842,7 +844,7 @@ void mp_destroy(mp_ctx* c) {
     dfree(c->d_root_prefix);
     if (c->h_draws) cudaFreeHost(c->h_draws);
     if (c->h_root_prefix) cudaFreeHost(c->h_root_prefix);
-    dfree(c->q.range); dfree(c->q.meta); dfree(c->q.seq); dfree(c->q.pts); dfree(c->q.path);
+    dfree(c->q.words); dfree(c->q.seq);
     dfree(c->sub.range); dfree(c->sub.meta); dfree(c->sub.seq); dfree(c->sub.path);
     free_sorted(c);
     dfree(c->big);
@@ -1070,7 +1072,7 @@ mp_status mp_finish(mp_ctx* c) {
         st = batched_frame(c);
         if (st) return st;
         c->stats.subpatches = std::min((long long)hc(c, kOutCount), c->sub.capacity);
-        c->stats.bounds = (long long)(hc(c, kQTail) >> 32);
+        c->stats.bounds = bounded_ranges(c);
         c->stats.passes = 1;
         c->stats.kernels = batched_kernels(c);
     } else {
@@ -1160,8 +1162,7 @@ mp_status mp_dump_stats(mp_ctx* c, char* buf, size_t cap) {
         long long bytes;
     } mem[] = {
         {"control points", cp},
-        {"work queue", c->q.capacity * (long long)(sizeof(float4) * (1 + kPtsPerSlot) + sizeof(uint2) +
-                                                   2 * sizeof(unsigned))},
+        {"work queue", c->q.capacity * (long long)((kBundleWords + 1) * sizeof(unsigned))},
         {"sub-patch list", c->sub.capacity * (long long)(sizeof(float4) + sizeof(int2) + 2 * sizeof(unsigned))},
         {"canonical sub-patch list", c->sorted.capacity * (long long)(sizeof(float4) + sizeof(int2))},
         {"canonical order sort", c->sb.capacity * 2 * (long long)(sizeof(unsigned long long) + sizeof(unsigned)) +
@@ -1181,7 +1182,7 @@ mp_status mp_dump_stats(mp_ctx* c, char* buf, size_t cap) {
         if (m.bytes > 0) ok = ok && put(buf, cap, &pos, "opencl_mem@%s = %lld;\n", m.use, m.bytes);
     const long long max_patches = c->opt.path == MP_PATH_PLAIN
                                       ? c->plain_max_stack
-                                      : (long long)(hc(c, kQTail) >> 32) - (long long)hc(c, kRoots);
+                                      : bounded_ranges(c) - (long long)hc(c, kRoots);
     ok = ok && put(buf, cap, &pos, "opengl_mem = 0;\n");
     ok = ok && put(buf, cap, &pos, "max_patches = %lld;\n", max_patches);
     ok = ok && put(buf, cap, &pos, "patches_per_frame = %lld;\n", (long long)c->stats.subpatches);

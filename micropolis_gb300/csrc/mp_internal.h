@@ -12,9 +12,10 @@ namespace mp {
 // Control words of one frame, each on its own 128-byte line so that the hot
 // atomics of different roles land in different L2 slices.
 enum CtrlWord {
-    kQTail = 0,        // queue tickets ever filled (virtual roots included)
-    kQHead,            // queue tickets handed out
-    kOutstanding,      // items pushed but not finished
+    kQTail = 0,        // bundle slots reserved by warps that give pairs away
+    kQHead,            // bundle tickets taken by waiting warps (beyond the first, dealt by warp number)
+    kRootHead,         // roots taken (beyond the first, dealt by warp number)
+    kOutstanding,      // units of work not finished | ranges split << 32
     kOutCount,         // sub-patches emitted
     kDone,             // bound-and-split finished
     kStatus,           // first error code (mp_status values)
@@ -34,16 +35,20 @@ enum CtrlWord {
 };
 constexpr int kCtrlStride = 16;  // unsigned long long words per line
 
-struct Queue {              // bound-and-split work queue (structure of arrays)
+// Bound-and-split queue: bundles of up to kBundlePairs split pairs that warps
+// hand to each other (word layout: mp_bns_loop.cuh).
+constexpr int kBundlePairs = 8;
+constexpr int kBundleWords = 288;   // 34 words per pair, the pair count, padding to 128 bytes
+struct Queue {
+    unsigned* words;        // kBundleWords per bundle
+    unsigned* seq;          // epoch of the frame that filled the bundle
+    long long capacity;     // bundles
+};
+
+// Stack of ranges of the per-pass path.
+struct RangeStack {
     float4* range;          // (min.x, min.y, max.x, max.y)
     uint2* meta;            // (patch id, draw | depth << 24)
-    unsigned* seq;          // epoch of the frame that wrote the slot
-    // kPtsPerSlot float4 per slot: six of the item's nine bound samples, taken
-    // from its parent, and which three are missing (or nullptr: none kept)
-    float4* pts;
-    // split path of each range: bit 31 - d is 1 when the range is the high
-    // half of its depth-d ancestor's split (nullptr: not kept)
-    unsigned* path;
     long long capacity;
 };
 
@@ -52,7 +57,8 @@ struct SubPatches {         // emitted sub-patch list
     int2* meta;             // (patch id, draw)
     long long capacity;
     unsigned* seq;          // epoch of the frame that emitted the slot (frame kernel only)
-    unsigned* path;         // split path (Queue::path) of each sub-patch (nullptr: not kept)
+    unsigned* path;         // split path of each sub-patch: bit 31 - d is 1 when it lies in the high half of
+                            // its depth-d ancestor's split (nullptr: not kept)
 };
 
 // Canonical order of a frame's sub-patches: ascending (root, split path),
@@ -97,8 +103,8 @@ void launch_bns_persistent(const DrawDev* draws, const int* root_prefix, int n_d
                            long long spin_limit, cudaStream_t s);
 int bns_persistent_grid(int criterion);
 // plain per-pass bound-and-split (the reference's BOUNDED structure)
-void launch_bns_init_stack(const Queue& stack, int draw, int n_patches, cudaStream_t s);
-void launch_bns_pass(const DrawDev* draws, const FrameDev& fr, const Queue& stack, long long offset, int batch,
+void launch_bns_init_stack(const RangeStack& stack, int draw, int n_patches, cudaStream_t s);
+void launch_bns_pass(const DrawDev* draws, const FrameDev& fr, const RangeStack& stack, long long offset, int batch,
                      float4* pad_range, uint2* pad_meta, unsigned char* dec, unsigned long long* keys,
                      unsigned long long* scan_state, const SubPatches& out, long long out_base,
                      unsigned long long* ctrl, long long spin_limit, cudaStream_t s);

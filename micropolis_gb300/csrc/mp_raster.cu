@@ -474,14 +474,14 @@ __global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>()
 // has not started; a wait that runs out stops consumption and reports
 // MP_ERR_TIMEOUT.
 // Shared memory of the frame kernel: the raster's, or what its
-// bound-and-split blocks stage (draw records, nine samples per thread).
-constexpr int kFrameStagedDraws = 64;
+// bound-and-split blocks hold (draw records, samples and stacks of the warp loop).
+constexpr int kFrameStagedDraws = 8;
 constexpr size_t kFramePtsOffset = (kFrameStagedDraws * sizeof(DrawDev) + 15) / 16 * 16;
 template <int PS, int NS>
 constexpr size_t frame_smem() {
-    return sizeof(FusedSmem<PS, NS>) > kFramePtsOffset + 27 * fused_threads<NS>() * sizeof(float)
+    return sizeof(FusedSmem<PS, NS>) > kFramePtsOffset + bns_smem<fused_threads<NS>(), kStackPairsFrame>()
                ? sizeof(FusedSmem<PS, NS>)
-               : kFramePtsOffset + 27 * fused_threads<NS>() * sizeof(float);
+               : kFramePtsOffset + bns_smem<fused_threads<NS>(), kStackPairsFrame>();
 }
 
 template <int PS, int NS>
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>()
     using SM = FusedSmem<PS, NS>;
     FrameDev fr = frp;
     load_amplitude(fr);
-    // bound-and-split blocks: draw records, then the bound samples of each thread
+    // bound-and-split blocks: draw records, then the warp loop's buffers
     // (frame_smem() sizes the launch for both uses)
     constexpr int kStaged = kFrameStagedDraws;
     constexpr size_t kPtsOffset = kFramePtsOffset;
@@ -509,9 +509,10 @@ __global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>()
             __syncthreads();
         }
         // the CPU criterion only: the host runs the GPU criterion as two launches
-        float* pts = reinterpret_cast<float*>(smem_raw + kPtsOffset);
-        bns_warp_loop<0, fused_threads<NS>()>(staged ? sd : gdraws, root_prefix, n_draws, fr, q, sub, sub.seq, ctrl,
-                                        spin_limit, pts);
+        bns_warp_loop<0, kStackPairsFrame>(
+            staged ? sd : gdraws, root_prefix, n_draws, fr, q, sub, sub.seq, ctrl, spin_limit,
+            reinterpret_cast<float*>(smem_raw + kPtsOffset), (int)(blockIdx.x + n_bns_ctas * (threadIdx.x >> 5)),
+            n_bns_ctas * (fused_threads<NS>() / 32));
         __syncthreads();
     }
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
