@@ -5,8 +5,9 @@ not the rendered sub-patch set:
 
 - ``dice_group``: sub-patches one fused block claims from the emitted
   sub-patch queue, dices, shades and rasterizes at a time (the queue chunk of
-  the dice/raster stage; 8, 11, 16 or 22 for 8x8 dicing, 2, 3, 4 or 6 for
-  16x16; 11 and 3 run 128-thread blocks, the others 256);
+  the dice/raster stage; nominally 8, 11, 16 or 22 for 8x8 dicing, 2, 3, 4 or
+  6 for 16x16, each the block shape next to it: 7, 14, 18 or 21 sub-patches in
+  64, 128, 256 or 192 threads, and 2, 3, 4 or 5 in 64, 128, 128 or 128);
 - ``raster_tile``: the tile edge, in pixels, of the depth|id key buffer that
   the 64-bit atomicMin resolves visibility in (8, 16 or 32);
 - ``overlap``: bound-and-split and rasterization in one launch, with the

@@ -529,13 +529,11 @@ __device__ __forceinline__ float dice_param(float rmin, float rmax, int n, const
     return ffma(fsub(rmax, rmin), fmul((float)n, inv), rmin);
 }
 // Eye position from precomputed parameters and weights of one vertex.
-// DISP: 0 no displacement, 1 displaced, -1 as fr.displacement says.
-template <int DISP = -1>
 __device__ __forceinline__ float4 dice_eye_w(int type, const float* mv, const FrameDev& fr, const float4* P, float tx,
                                              float ty, float4 vw, float4 cw) {
     float4 o = (type == 0) ? eval_bezier_dice_w(P, vw, cw) : eval_gregory_dice_w(P, tx, ty, vw, cw);
     float4 pos = mul_m44v4(mv, o);
-    if (DISP > 0 || (DISP < 0 && fr.displacement)) pos = displace(pos, fr.fdisp);
+    if (fr.displacement) pos = displace(pos, fr.fdisp);
     return pos;
 }
 __device__ __forceinline__ float4 dice_eye_m(int type, const float* mv, const FrameDev& fr, const float4* P,
@@ -546,6 +544,89 @@ __device__ __forceinline__ float4 dice_eye_m(int type, const float* mv, const Fr
 __device__ __forceinline__ float4 dice_eye(const DrawDev& d, const FrameDev& fr, const float4* P, float4 r,
                                            int nu, int nv) {
     return dice_eye_m(d.type, d.mv, fr, P, r, nu, nv);
+}
+
+// The object-space positions of N dice vertices of one column (the same u),
+// each by the operations of eval_bezier_dice_w / eval_gregory_dice_w: every
+// control point is loaded once for the N vertices, and their N independent
+// chains hide each other's latency.
+template <int N>
+struct DiceColumn {
+    float2 xy[N], zw[N];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int n = 0; n < N; ++n) xy[n] = zw[n] = make_float2(0.f, 0.f);
+    }
+    // adds the same control point to every vertex
+    __device__ __forceinline__ void add(float vw, const float (&cw)[N], float4 c) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const float2 w = fmul2(dup2(vw), dup2(cw[n]));
+            xy[n] = ffma2(w, make_float2(c.x, c.y), xy[n]);
+            zw[n] = ffma2(w, make_float2(c.z, c.w), zw[n]);
+        }
+    }
+    // adds each vertex's face point (a A + b_n B) / den_n, NaN zeroed (blend4)
+    __device__ __forceinline__ void add_face(float vw, const float (&cw)[N], float a, float4 A, const float (&b)[N],
+                                             float4 B, const float (&den)[N]) {
+        const float2 axy = fmul2(dup2(a), make_float2(A.x, A.y)), azw = fmul2(dup2(a), make_float2(A.z, A.w));
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const float2 r = dup2(frcp(den[n])), b2 = dup2(b[n]), w = fmul2(dup2(vw), dup2(cw[n]));
+            const float2 fxy = fmul2(ffma2(b2, make_float2(B.x, B.y), axy), r);
+            const float2 fzw = fmul2(ffma2(b2, make_float2(B.z, B.w), azw), r);
+            xy[n] = ffma2(w, make_float2(sel_nan(fxy.x), sel_nan(fxy.y)), xy[n]);
+            zw[n] = ffma2(w, make_float2(sel_nan(fzw.x), sel_nan(fzw.y)), zw[n]);
+        }
+    }
+};
+
+template <int N>
+__device__ __forceinline__ void dice_column(DiceColumn<N>& d, int type, const float4* P, float tx,
+                                            const float (&ty)[N], float4 vw, const float4 (&cw)[N]) {
+    float c[4][N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        c[0][n] = cw[n].x;
+        c[1][n] = cw[n].y;
+        c[2][n] = cw[n].z;
+        c[3][n] = cw[n].w;
+    }
+    const float v[4] = {vw.x, vw.y, vw.z, vw.w};
+    d.clear();
+    if (type == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) d.add(v[i], c[j], P[4 * i + j]);
+        return;
+    }
+    const float u = tx, a = fsub(1.0f, tx);
+    float b[N], d0[N], d1[N], d2[N], d3[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        b[n] = fsub(1.0f, ty[n]);
+        d0[n] = fadd(u, ty[n]);
+        d1[n] = fadd(a, ty[n]);
+        d2[n] = fsub(fsub(2.0f, u), ty[n]);
+        d3[n] = fsub(fadd(1.0f, u), ty[n]);
+    }
+    d.add(v[0], c[0], P[0]);
+    d.add(v[0], c[1], P[4]);
+    d.add(v[0], c[2], P[9]);
+    d.add(v[0], c[3], P[1]);
+    d.add(v[1], c[0], P[8]);
+    d.add_face(v[1], c[1], u, P[12], ty, P[16], d0);
+    d.add_face(v[1], c[2], a, P[17], ty, P[13], d1);
+    d.add(v[1], c[3], P[5]);
+    d.add(v[2], c[0], P[7]);
+    d.add_face(v[2], c[1], u, P[19], b, P[15], d3);
+    d.add_face(v[2], c[2], a, P[14], b, P[18], d2);
+    d.add(v[2], c[3], P[10]);
+    d.add(v[3], c[0], P[3]);
+    d.add(v[3], c[1], P[11]);
+    d.add(v[3], c[2], P[6]);
+    d.add(v[3], c[3], P[2]);
 }
 
 // Projection to fixed-point pixel coordinates and NDC depth (kernels/dice.cl:69-79).
@@ -564,22 +645,36 @@ __device__ __forceinline__ void project_vertex_m(const float* proj, const FrameD
     depth = fmul(p.z, rw);
 }
 // project_vertex_m for a glm::perspective matrix, whose only nonzero
-// entries are m0, m5, m10, m14 and m11 = -1 (the host builds every draw's
-// projection so).  For a finite position with eye z != 0 the general product
-// reduces exactly: each zero term adds a zero to a rounded product, which
-// changes at most the sign of a zero result, and the viewport transform
+// entries are pr = (m0, m5, m10, m14) and m11 = -1 (the host builds every
+// draw's projection so).  For a finite position with eye z != 0 the general
+// product reduces exactly: each zero term adds a zero to a rounded product,
+// which changes at most the sign of a zero result, and the viewport transform
 // (+ W/2, + H/2) and the depth clamp do not see that sign; p.w = -z.  Any
 // other position takes the general product.
-__device__ __forceinline__ void project_vertex_persp(const float* proj, const FrameDev& fr, float4 pos, int& px,
+static __device__ __noinline__ int4 project_vertex_general(float4 pr, int W, int H, int shift, float4 pos) {
+    const float m[16] = {pr.x, 0.f, 0.f, 0.f, 0.f, pr.y, 0.f, 0.f, 0.f, 0.f, pr.z, -1.f, 0.f, 0.f, pr.w, 0.f};
+    FrameDev fr{};
+    fr.W = W;
+    fr.H = H;
+    fr.shift = shift;
+    int px, py;
+    float depth;
+    project_vertex_m(m, fr, pos, px, py, depth);
+    return make_int4(px, py, __float_as_int(depth), 0);
+}
+__device__ __forceinline__ void project_vertex_persp(const float (&pr)[4], const FrameDev& fr, float4 pos, int& px,
                                                      int& py, float& depth) {
     const float mag = fadd(fadd(fabsf(pos.x), fabsf(pos.y)), fadd(fabsf(pos.z), fabsf(pos.w)));
     if (!(mag < __int_as_float(0x7f800000)) || pos.z == 0.0f) {
-        project_vertex_m(proj, fr, pos, px, py, depth);
+        const int4 r = project_vertex_general(make_float4(pr[0], pr[1], pr[2], pr[3]), fr.W, fr.H, fr.shift, pos);
+        px = r.x;
+        py = r.y;
+        depth = __int_as_float(r.z);
         return;
     }
     const int vsx = fr.W << fr.shift, vsy = fr.H << fr.shift;
-    const float2 pxy = fmul2(make_float2(proj[0], proj[5]), make_float2(pos.x, pos.y));
-    const float pz = ffma(proj[14], pos.w, fmul(proj[10], pos.z));
+    const float2 pxy = fmul2(make_float2(pr[0], pr[1]), make_float2(pos.x, pos.y));
+    const float pz = ffma(pr[3], pos.w, fmul(pr[2], pos.z));
     const float rw = frcp(-pos.z);
     float2 e = fmul2(pxy, dup2(rw));
     e = fmul2(e, make_float2((float)vsx, (float)vsy));

@@ -84,14 +84,6 @@ __device__ __forceinline__ bool quad_is_fast(const int* qx, const int* qy, int& 
     return (maxx - minx) <= kFastExtent && (maxy - miny) <= kFastExtent;
 }
 
-// A small quad whose two triangles both have the rejected winding covers
-// nothing (small quads: the products below cannot overflow).
-__device__ __forceinline__ bool quad_winding_ok(const int* qx, const int* qy) {
-    int d1x = qx[1] - qx[0], d1y = qy[1] - qy[0];
-    int d2x = qx[2] - qx[0], d2y = qy[2] - qy[0];
-    int d3x = qx[3] - qx[0], d3y = qy[3] - qy[0];
-    return d1x * d3y - d3x * d1y < 0 || d3x * d2y - d2x * d3y < 0;
-}
 // Pixels whose sample point lies in the fixed-point bbox, clipped to the
 // frame; false when there are none.
 __device__ __forceinline__ bool quad_pixels(const FrameDev& fr, int minx, int miny, int maxx, int maxy, int& x0,
@@ -104,24 +96,55 @@ __device__ __forceinline__ bool quad_pixels(const FrameDev& fr, int minx, int mi
     return x0 <= x1 && y0 <= y1;
 }
 
+// One triangle (a, b, c) of a quad at one sample, kernels/reyes.cl:240-265
+// with the vertices taken relative to the sample (r = sample - vertex): edge
+// a -> b's function (b.y - a.y) (t.x - a.x) + (a.x - b.x) (t.y - a.y) is
+// rb.x ra.y - rb.y ra.x, the reference's value exactly (wrapped int32 is a
+// ring), and the three functions add up to the barycentric denominator (see
+// tri_setup), so a quad that covers one pixel, the usual case, needs no edge
+// setup, and no reciprocal unless it covers it.
+__device__ __forceinline__ bool edge_inside(int v, int ax, int ay, int bx, int by) {
+    // V > C with C = -1 where Dx > 0 or (Dx == 0 and Dy > 0), else 0; Dx = ra.y - rb.y, Dy = rb.x - ra.x
+    return v > ((ay > by || (ay == by && bx > ax)) ? -1 : 0);
+}
+__device__ __forceinline__ float tri_depth(int va, int vb, int vc, float da, float db, float dc) {
+    // weights: edge b -> c's function for a, c -> a's for b, a -> b's for c (va, vb, vc: edges from a, b, c)
+    const float rdn = frcp((float)wadd(wadd(va, vb), vc));
+    return ffma(dc, fmul((float)va, rdn), ffma(db, fmul((float)vc, rdn), fmul(da, fmul((float)vb, rdn))));
+}
+
 // Fast path: rasterize one quad over its own pixel bbox (see file header).
+// The quad's triangles are (0, 1, 3) and (0, 3, 2).
 __device__ __forceinline__ int raster_quad_fast(const FrameDev& fr, unsigned long long* keys, const int* qx,
                                                 const int* qy, const float* qd, int minx, int miny, int maxx,
                                                 int maxy, unsigned mp_id) {
-    if (!quad_winding_ok(qx, qy)) return 0;
     int x0, y0, x1, y1;
     if (!quad_pixels(fr, minx, miny, maxx, maxy, x0, y0, x1, y1)) return 0;
-    Tri t1, t2;
-    tri_setup(t1, qx[0], qy[0], qd[0], qx[1], qy[1], qd[1], qx[3], qy[3], qd[3]);
-    tri_setup(t2, qx[0], qy[0], qd[0], qx[3], qy[3], qd[3], qx[2], qy[2], qd[2]);
     int frags = 0;
     for (int y = y0; y <= y1; ++y)
         for (int x = x0; x <= x1; ++x) {
-            int tx = x << fr.shift, ty = y << fr.shift;
-            float depth = 1.0f;
-            bool in1 = tri_test(t1, tx, ty, depth);
-            bool in2 = tri_test(t2, tx, ty, depth);
+            int rx[4], ry[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                rx[k] = (x << fr.shift) - qx[k];
+                ry[k] = (y << fr.shift) - qy[k];
+            }
+            auto edge = [&](int a, int b) { return wsub(wmul(rx[b], ry[a]), wmul(ry[b], rx[a])); };
+            auto in = [&](int v, int a, int b) { return edge_inside(v, rx[a], ry[a], rx[b], ry[b]); };
+            const int v01 = edge(0, 1), v13 = edge(1, 3), v30 = edge(3, 0), v32 = edge(3, 2), v20 = edge(2, 0);
+            const int v03 = wsub(0, v30);
+            const bool in1 = in(v01, 0, 1) && in(v13, 1, 3) && in(v30, 3, 0);
+            const bool in2 = in(v03, 0, 3) && in(v32, 3, 2) && in(v20, 2, 0);
             if (in1 || in2) {
+                float depth = 1.0f;
+                if (in1) {
+                    const float d = tri_depth(v01, v13, v30, qd[0], qd[1], qd[3]);
+                    if (d < depth) depth = d;
+                }
+                if (in2) {
+                    const float d = tri_depth(v03, v32, v20, qd[0], qd[3], qd[2]);
+                    if (d < depth) depth = d;
+                }
                 // the reference writes only depths below the cleared 0x7fffffff (kernels/reyes.cl:389)
                 const unsigned idp = idepth_of(depth);
                 if (idp < 0x7fffffffu) atomicMin(keys + key_index(fr, x, y), ((unsigned long long)idp << 32) | mp_id);
@@ -153,42 +176,65 @@ __device__ __forceinline__ void push_big(BigQuad* big, long long big_cap, unsign
     big[i] = b;
 }
 
-// The fused kernel works on groups of NS sub-patches per block:
-// NS * (PS+1)^2 dice vertices are spread over all threads (22 * 81 = 1782 =
-// 7 rounds of 256 at PS = 8), then the block bounds, then one thread per quad
-// that can touch a pixel.  The inputs of the next group (sub-patch records,
-// control points, matrices) are copied into the other half of a double
-// buffer with cp.async while the current group is diced and rasterized.
-// Groups of 11 (PS = 8) and 3 (PS = 16) run half-size blocks of 128 threads,
-// twice as many per SM, the others 256.
+// The fused kernel works on groups of NS sub-patches per block: their dice
+// vertices are spread over the threads in runs of kRun of one column
+// (27 runs a sub-patch at PS = 8), then the quads in strips of 8 of one
+// column (8 strips a sub-patch), then one thread per quad that can touch a
+// pixel.  The inputs of the next group (sub-patch records, control points,
+// matrices) are copied into the other half of a double buffer with cp.async
+// while the current group is diced and rasterized.
+//
+// Instruction issue and the latency of short chains bound the kernel (no
+// pipe is above 40 %, DRAM at 2 %).  Runs of 3 vertices load each control
+// point, matrix and column weight once for three independent chains: with one
+// vertex per thread the dice issued 209 instructions a vertex.  Strips load
+// two vertices a row instead of four a quad and skip the block bound.  Runs
+// take 96 registers, so the shapes hold 20 warps per SM; NS is chosen so that
+// both the runs and the strips of a group nearly fill whole rounds of its
+// threads (14 at 128 threads: 98 % and 88 %).  Dice+raster on the mixed
+// 4096-patch scene at 1920x1080: 1.72 ms (one vertex per thread, groups of 11
+// in 6 blocks of 128) -> 1.42 ms; groups of 13: 1.47, of 9: 1.57, of 11 in
+// 160 threads: 1.61, of 7 in 64: 1.59, of 18 in 256: 1.55, of 12 in 6 blocks
+// (80 registers, spills): 1.61.  At 16x16 dicing 5.63 -> 4.56 ms (groups of
+// 5; 4: 4.74, 6 in 256 threads: 4.92).
+constexpr int kRun = 3;
 template <int NS>
 constexpr int fused_threads() {
-    return (NS == 11 || NS == 3) ? 128 : 256;
+    return NS == 2 || NS == 7 ? 64 : NS == 18 ? 256 : NS == 21 ? 192 : 128;
+}
+// resident blocks per SM the kernels are compiled for
+template <int NS>
+constexpr int fused_blocks() {
+    return NS == 2 || NS == 7 ? 10 : NS == 18 || NS == 21 ? 3 : 5;
 }
 
 static_assert(offsetof(DrawDev, proj) == offsetof(DrawDev, mv) + 16 * sizeof(float), "mv, proj adjacent");
 static_assert(offsetof(DrawDev, mv) % 16 == 0 && sizeof(DrawDev) % 16 == 0, "16-byte copies of mv/proj");
 
-// Inputs of one group.
+// Inputs of one group.  Sub-patches of one draw follow each other in the
+// canonical list, so a group holds few runs of equal draws: the matrices are
+// staged once per run, the first kMatrixRuns runs of a group (later ones read
+// them from the draw records).
+constexpr int kMatrixRuns = 2;
 template <int NS>
 struct GroupStage {
     float4 cp[NS][20];
-    float mvp[NS][32];        // modelview, then projection
+    float mvp[kMatrixRuns][32];   // modelview, then projection
     float4 range[NS];
-    int2 meta[NS];            // (patch id, draw)
-    int tv[NS][2];            // draw type, view
+    int2 meta[NS];                // (patch id, draw)
+    int tv[NS][2];                // draw type, view
+    int run[NS];                  // run of equal draws
 };
 
 template <int PS, int NS_>
 struct FusedSmem {
-    static constexpr int NS = NS_, G = PS + 1, NV = G * G, NB = (PS / 8) * (PS / 8);
+    static constexpr int NS = NS_, G = PS + 1, NV = G * G;
     GroupStage<NS> st[2];
-    // per group state, double-buffered with st: block bounds, blocks with a
-    // vertex at eye z == 0, and the number of listed quads
-    int bound[2][NS][NB][4];
+    // per group state, double-buffered with st: blocks with a vertex at eye
+    // z == 0, and the number of listed quads
     unsigned zero[2][NS];
     unsigned n_live[2];
-    unsigned short live[NS * PS * PS];   // quads that may touch a pixel, in bound-phase order
+    unsigned short live[NS * PS * PS];   // quads that may touch a pixel
     float tx[NS][G], ty[NS][G];
     float4 vw[NS][G], cw[NS][G];
     float4 edep[NS * NV];     // eye position and NDC depth of each dice vertex
@@ -208,23 +254,45 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Copies, for the n sub-patches whose records are already in st.meta, their
+// Stores the records of a group's n sub-patches, one per thread of warp 0
+// (n <= 32), and numbers their runs of equal draws; called by whole warps.
+template <int NS>
+__device__ __forceinline__ void store_records(GroupStage<NS>& st, int n, float4 range, int2 meta) {
+    static_assert(NS <= 32, "one record per lane of warp 0");
+    const int tid = threadIdx.x;
+    if (tid >= 32) return;
+    const int before = __shfl_up_sync(0xffffffffu, meta.y, 1);
+    const unsigned starts = __ballot_sync(0xffffffffu, tid > 0 && tid < n && meta.y != before);
+    if (tid < n) {
+        st.range[tid] = range;
+        st.meta[tid] = meta;
+        st.run[tid] = __popc(starts & (lanemask_lt() | (1u << tid)));
+    }
+}
+
+// Copies, for the n sub-patches whose records are already in st, their
 // control points, matrices, type and view (asynchronous; the caller waits).
 template <int NS>
 __device__ __forceinline__ void stage_inputs(GroupStage<NS>& st, int n, const DrawDev* __restrict__ draws) {
-    for (int i = threadIdx.x; i < n * 32; i += fused_threads<NS>()) {
-        const int k = i >> 5, c = i & 31;
+    for (int i = threadIdx.x; i < n * 24; i += fused_threads<NS>()) {
+        const int k = i / 24, c = i % 24;
         const int2 m = st.meta[k];
         const DrawDev* d = draws + m.y;
         if (c < 20) {
             const int ncp = d->type == 0 ? 16 : 20;
             if (c < ncp) cp_async16(&st.cp[k][c], d->cp + (size_t)m.x * ncp + c);
-        } else if (c < 28) {
-            cp_async16(&st.mvp[k][4 * (c - 20)], d->mv + 4 * (c - 20));
-        } else if (c == 28) {
+        } else if (c == 20) {
             cp_async4(&st.tv[k][0], &d->type);
-        } else if (c == 29) {
+        } else if (c == 21) {
             cp_async4(&st.tv[k][1], &d->view);
+        } else {
+            // the run's first sub-patch copies its matrices, 64 bytes per lane
+            const int run = st.run[k];
+            if (run < kMatrixRuns && (k == 0 || st.run[k - 1] != run)) {
+                const int at = (c - 22) * 16;
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) cp_async16(&st.mvp[run][at + j], d->mv + at + j);
+            }
         }
     }
     cp_async_commit();
@@ -232,11 +300,10 @@ __device__ __forceinline__ void stage_inputs(GroupStage<NS>& st, int n, const Dr
 
 // Prepares the state of a group of n sub-patches whose records are in
 // sm.st[b]: the dice parameters and Bernstein weights of each row / column of
-// vertices, reset block bounds (viewport max, 0), eye-plane flags and listed
-// quad count.  This thread takes the items first, first + threads, ...
+// vertices, reset eye-plane flags and listed quad count.  This thread takes the items first, first + threads, ...
 template <int PS, int NS>
 __device__ __forceinline__ void prepare_group(FusedSmem<PS, NS>& sm, int b, int n, const FrameDev& fr, int first) {
-    constexpr int G = PS + 1, NB = (PS / 8) * (PS / 8);
+    constexpr int G = PS + 1;
     const GroupStage<NS>& st = sm.st[b];
     for (int i = first; i < n * 2 * G; i += fused_threads<NS>()) {
         const int k = i / (2 * G), c = i % (2 * G);
@@ -251,11 +318,6 @@ __device__ __forceinline__ void prepare_group(FusedSmem<PS, NS>& sm, int b, int 
             sm.cw[k][c - G] = col_weights(t);
         }
     }
-    const int vmaxx = (fr.W << fr.shift) - 1, vmaxy = (fr.H << fr.shift) - 1;
-    for (int i = first; i < n * NB; i += fused_threads<NS>()) {
-        int* bb = sm.bound[b][i / NB][i % NB];
-        bb[0] = vmaxx; bb[1] = vmaxy; bb[2] = 0; bb[3] = 0;
-    }
     if (first < n) sm.zero[b][first] = 0;
     if (first == 0) sm.n_live[b] = 0;
 }
@@ -266,10 +328,13 @@ template <int PS, int NS>
 __device__ __forceinline__ void stage_group(FusedSmem<PS, NS>& sm, long long base, int n, const SubPatches& sub,
                                             const DrawDev* __restrict__ draws, const FrameDev& fr) {
     GroupStage<NS>& st = sm.st[0];
+    float4 range = make_float4(0.f, 0.f, 0.f, 0.f);
+    int2 meta = make_int2(0, 0);
     if ((int)threadIdx.x < n) {
-        st.range[threadIdx.x] = sub.range[base + threadIdx.x];
-        st.meta[threadIdx.x] = sub.meta[base + threadIdx.x];
+        range = sub.range[base + threadIdx.x];
+        meta = sub.meta[base + threadIdx.x];
     }
+    store_records(st, n, range, meta);
     __syncthreads();
     stage_inputs(st, n, draws);
     prepare_group(sm, 0, n, fr, threadIdx.x);
@@ -277,12 +342,65 @@ __device__ __forceinline__ void stage_group(FusedSmem<PS, NS>& sm, long long bas
     __syncthreads();
 }
 
+// The 8x8 block bound over front-facing quads (kernels/reyes.cl:120-166) of a
+// block whose first vertex is pxy[0] (rows G apart), clamped, as its tile
+// range; x > z when is_empty (kernels/reyes.cl:287) skips the block.
+template <int G>
+__device__ __forceinline__ int4 group_block_tiles(const int2* pxy, int W, int H, int shift, int backface) {
+    FrameDev fr{};
+    fr.W = W;
+    fr.H = H;
+    fr.shift = shift;
+    fr.backface = backface;
+    int x0 = (W << shift) - 1, y0 = (H << shift) - 1, x1 = 0, y1 = 0;
+#pragma unroll 1
+    for (int q = 0; q < 64; ++q) {
+        const int2* at = pxy + (q & 7) + (q >> 3) * G;
+        const int2 c0 = at[0], c1 = at[1], c2 = at[G], c3 = at[G + 1];
+        const int qx[4] = {c0.x, c1.x, c2.x, c3.x}, qy[4] = {c0.y, c1.y, c2.y, c3.y};
+        const QuadBound qb = quad_block_bound(fr, qx, qy);
+        if (qb.ff) {
+            x0 = min(x0, qb.pminx);
+            y0 = min(y0, qb.pminy);
+            x1 = max(x1, qb.pmaxx);
+            y1 = max(y1, qb.pmaxy);
+        }
+    }
+    int t[4];
+    if (!block_tiles(fr, x0, y0, x1, y1, true, t)) return make_int4(1, 0, 0, 0);
+    return make_int4(t[0], t[1], t[2], t[3]);
+}
+
+// Modelview and the perspective matrix's entries 0, 5, 10, 14 from 32 floats
+// (modelview, projection; 16-byte aligned).
+__device__ __forceinline__ void load_matrices(const float* m, float (&mv)[16], float (&pr)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 v = reinterpret_cast<const float4*>(m)[j];
+        mv[4 * j] = v.x;
+        mv[4 * j + 1] = v.y;
+        mv[4 * j + 2] = v.z;
+        mv[4 * j + 3] = v.w;
+    }
+    pr[0] = m[16];
+    pr[1] = m[21];
+    pr[2] = m[26];
+    pr[3] = m[30];
+}
+
 // Dices, shades and rasterizes the n (<= NS) sub-patches at [base, base+n)
 // of the emitted list, whose inputs are staged and prepared in buffer b, with
 // the whole block; meanwhile stages and prepares the n_next sub-patches at
-// next_base in buffer b ^ 1.  Three phases (dice; block bounds and the list
-// of quads that can touch a pixel; raster), each ending with a barrier after
-// which both groups' buffers are complete.
+// next_base in buffer b ^ 1.  Three phases (dice; the list of quads that can
+// touch a pixel; raster), each ending with a barrier after which both groups'
+// buffers are complete.
+//
+// The 8x8 block bound decides only whether a block is skipped, and the tiles
+// of quads too large for the fast raster.  A small front-facing quad with a
+// pixel centre in its bbox has that centre inside the clamped bound, and the
+// bound is not empty unless every front-facing quad of the block ends at
+// x = 0, so only large quads and those with maxx <= 0 look at the bound, each
+// on its own (group_block_tiles); an eye-plane vertex still skips the block.
 // DISP is the frame's displacement option, compiled in: frames without it
 // carry neither its code nor its registers.
 template <int PS, int NS, bool DISP>
@@ -292,11 +410,10 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
                                              float* __restrict__ mshade, BigQuad* big, long long big_cap,
                                              unsigned long long* ctrl, const V3& light, long long& frags) {
     using SM = FusedSmem<PS, NS>;
-    constexpr int G = SM::G, NV = SM::NV, NQ = PS * PS, BPL = PS / 8, NB = SM::NB, TH = fused_threads<NS>();
+    constexpr int G = SM::G, NV = SM::NV, NQ = PS * PS, BPL = PS / 8, TH = fused_threads<NS>();
     GroupStage<NS>& cur = sm.st[b];
     GroupStage<NS>& nxt = sm.st[b ^ 1];
     const int tid = threadIdx.x, lane = tid & 31;
-    const int vmaxx = (fr.W << fr.shift) - 1, vmaxy = (fr.H << fr.shift) - 1;
     // the next group's records travel in registers until this group's
     // vertices are done
     float4 next_range = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -305,87 +422,130 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
         next_range = sub.range[next_base + tid];
         next_meta = sub.meta[next_base + tid];
     }
-    // dice vertices (kernels/dice.cl:37-80); vertex i is (k, nu, nv) with
-    // i = k * NV + nv * G + nu, stepped by TH without divisions
-    constexpr int DK = TH / NV, DNV = (TH % NV) / G, DNU = (TH % NV) % G;
-    int k = tid / NV, nv = (tid % NV) / G, nu = (tid % NV) % G;
-    for (int i = tid; i < n * NV; i += TH) {
-        const float* mvp = cur.mvp[k];
-        float4 pos = dice_eye_w<DISP ? 1 : 0>(cur.tv[k][0], mvp, fr, cur.cp[k], sm.tx[k][nu], sm.ty[k][nv], sm.vw[k][nu],
-                                sm.cw[k][nv]);
-        int px, py;
-        float dep;
-        project_vertex_persp(mvp + 16, fr, pos, px, py, dep);
-        sm.pxy[i] = make_int2(px, py);
-        sm.edep[i] = make_float4(pos.x, pos.y, pos.z, dep);
-        if (pos.z == 0.0f) {
-            // a vertex at eye z == 0 drops every 8x8 block it belongs to (kernels/reyes.cl:130-162)
-            unsigned zb = 0;
-            for (int bv = max(nv - 1, 0) / 8; bv <= min(nv, PS - 1) / 8; ++bv)
-                for (int bu = max(nu - 1, 0) / 8; bu <= min(nu, PS - 1) / 8; ++bu) zb |= 1u << (bu + bv * BPL);
-            atomicOr(&sm.zero[b][k], zb);
+    // dice vertices (kernels/dice.cl:37-80): run i of a sub-patch holds the
+    // vertices (nu, nv0 .. nv0 + kRun - 1), nu = i % G, nv0 = kRun (i / G)
+    constexpr int NR = (G + kRun - 1) / kRun, RPS = G * NR;
+    for (int i = tid; i < n * RPS; i += TH) {
+        const int k = i / RPS, c = i - k * RPS, nv0 = c / G * kRun, nu = c % G;
+        float4 cw[kRun];
+        float ty[kRun];
+#pragma unroll
+        for (int v = 0; v < kRun; ++v) {
+            // (a run past the last row repeats it)
+            const int nv = G % kRun ? min(nv0 + v, G - 1) : nv0 + v;
+            cw[v] = sm.cw[k][nv];
+            ty[v] = sm.ty[k][nv];
         }
-        k += DK;
-        nv += DNV;
-        nu += DNU;
-        if (nu >= G) { nu -= G; ++nv; }
-        if (nv >= G) { nv -= G; ++k; }
+        DiceColumn<kRun> d;
+        dice_column<kRun>(d, cur.tv[k][0], cur.cp[k], sm.tx[k][nu], ty, sm.vw[k][nu], cw);
+        // the draw's modelview, and the perspective's entries 0, 5, 10, 14
+        float mv[16], pr[4];
+        const int run = cur.run[k];
+        if (run < kMatrixRuns) {
+            load_matrices(cur.mvp[run], mv, pr);
+        } else {
+            load_matrices(draws[cur.meta[k].y].mv, mv, pr);
+        }
+        float4 pos[kRun];
+#pragma unroll
+        for (int v = 0; v < kRun; ++v)
+            pos[v] = mul_m44v4(mv, make_float4(d.xy[v].x, d.xy[v].y, d.zw[v].x, d.zw[v].y));
+        if (DISP) {
+#pragma unroll
+            for (int v = 0; v < kRun; ++v) pos[v] = displace(pos[v], fr.fdisp);
+        }
+        int2 px[kRun];
+        float dep[kRun];
+#pragma unroll
+        for (int v = 0; v < kRun; ++v) project_vertex_persp(pr, fr, pos[v], px[v].x, px[v].y, dep[v]);
+        const int at = k * NV + nv0 * G + nu;
+#pragma unroll
+        for (int v = 0; v < kRun; ++v) {
+            if (G % kRun && nv0 + v >= G) break;
+            sm.pxy[at + v * G] = px[v];
+            sm.edep[at + v * G] = make_float4(pos[v].x, pos[v].y, pos[v].z, dep[v]);
+            if (pos[v].z == 0.0f) {
+                // a vertex at eye z == 0 drops every 8x8 block it belongs to (kernels/reyes.cl:130-162)
+                const int nv = nv0 + v;
+                unsigned zb = 0;
+                for (int bv = max(nv - 1, 0) / 8; bv <= min(nv, PS - 1) / 8; ++bv)
+                    for (int bu = max(nu - 1, 0) / 8; bu <= min(nu, PS - 1) / 8; ++bu) zb |= 1u << (bu + bv * BPL);
+                atomicOr(&sm.zero[b][k], zb);
+            }
+        }
     }
-    if (tid < n_next) {
-        nxt.range[tid] = next_range;
-        nxt.meta[tid] = next_meta;
-    }
+    if (n_next > 0) store_records(nxt, n_next, next_range, next_meta);
     __syncthreads();
     if (n_next > 0) stage_inputs(nxt, n_next, draws);
-    // Block bounds over front-facing quads (kernels/reyes.cl:120-166), and
-    // the list of quads that can touch a pixel: a quad with a large bbox, or
-    // a small one with an accepted winding and a pixel centre in its bbox.
-    // n * NQ is a multiple of 32, so whole warps run each round; the quads of
-    // one warp share a sub-patch, and their 8x8 blocks are fixed by the lane:
-    // one block at PS = 8, and at PS = 16 two, lanes with bit 3 clear / set.
-    for (int i = tid; i < n * NQ; i += TH) {
-        const int k = i / NQ, q = i % NQ;
-        const int nu = q % PS, nv = q / PS, i0 = k * NV + nu + nv * G;
-        const int2 c0 = sm.pxy[i0], c1 = sm.pxy[i0 + 1], c2 = sm.pxy[i0 + G], c3 = sm.pxy[i0 + G + 1];
-        const int qx[4] = {c0.x, c1.x, c2.x, c3.x};
-        const int qy[4] = {c0.y, c1.y, c2.y, c3.y};
-        const int minx = min(min(qx[0], qx[1]), min(qx[2], qx[3]));
-        const int maxx = max(max(qx[0], qx[1]), max(qx[2], qx[3]));
-        const int miny = min(min(qy[0], qy[1]), min(qy[2], qy[3]));
-        const int maxy = max(max(qy[0], qy[1]), max(qy[2], qy[3]));
-        // is_front_facing (kernels/reyes.cl:54-65) on wrapped int32
-        const int d1x = wsub(qx[1], qx[0]), d1y = wsub(qy[1], qy[0]);
-        const int d2x = wsub(qx[2], qx[0]), d2y = wsub(qy[2], qy[0]);
-        const int d3x = wsub(qx[3], qx[0]), d3y = wsub(qy[3], qy[0]);
-        const bool wind = wsub(wmul(d1x, d3y), wmul(d3x, d1y)) < 0 || wsub(wmul(d3x, d2y), wmul(d2x, d3y)) < 0;
-        const bool fast = minx >= -kFastCoord && maxx <= kFastCoord && miny >= -kFastCoord && maxy <= kFastCoord &&
-                          maxx - minx <= kFastExtent && maxy - miny <= kFastExtent;
-        // with backface culling, a warp whose quads are all small and face
-        // away lists none of them and leaves its block bound as it is (the
-        // steps below would add (viewport max, 0)): it skips them (about half
-        // the warps of a scene of randomly oriented patches)
-        if (fr.backface && __all_sync(0xffffffffu, fast && !wind)) continue;
-        int x0, y0, x1, y1;
-        const bool live = !fast || (wind && quad_pixels(fr, minx, miny, maxx, maxy, x0, y0, x1, y1));
-        const unsigned lm = __ballot_sync(0xffffffffu, live);
-        unsigned at = 0;
-        if (lane == 0 && lm) at = atomicAdd(&sm.n_live[b], (unsigned)__popc(lm));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (live) sm.live[at + __popc(lm & lanemask_lt())] = (unsigned short)i;
-        // the block bound starts at (viewport max, 0) and takes front-facing quads
-        const bool ff = !fr.backface || wind;
-        const unsigned grp = PS == 8 ? 0xffffffffu : ((lane & 8) ? 0xff00ff00u : 0x00ff00ffu);
-        const int bx0 = __reduce_min_sync(grp, ff ? min(vmaxx, minx) : vmaxx);
-        const int by0 = __reduce_min_sync(grp, ff ? min(vmaxy, miny) : vmaxy);
-        const int bx1 = __reduce_max_sync(grp, ff ? max(0, maxx) : 0);
-        const int by1 = __reduce_max_sync(grp, ff ? max(0, maxy) : 0);
-        if ((lane & (PS == 8 ? 31 : 23)) == 0) {
-            int* bb = sm.bound[b][k][(nu >> 3) + (nv >> 3) * BPL];
-            atomicMin(bb + 0, bx0);
-            atomicMin(bb + 1, by0);
-            atomicMax(bb + 2, bx1);
-            atomicMax(bb + 3, by1);
+    // The list of quads that can touch a pixel: a quad with a large bbox, or a
+    // small one with an accepted winding and a pixel centre in its bbox.  A
+    // thread walks a strip of 8 quads (column nu, rows 8 h .. 8 h + 7), so
+    // each row's two vertices and their bounds serve two quads.
+    constexpr int SPS = PS * BPL;   // strips of a sub-patch
+    for (int i0 = tid & ~31; i0 < n * SPS; i0 += TH) {
+        const int i = i0 + lane;
+        unsigned live = 0;   // bit r: quad of row 8 h + r
+        int first = 0;       // list entry of row 0
+        if (i < n * SPS) {
+            const int k = i / SPS, c = i % SPS, nu = c % PS, h = c / PS;
+            first = k * NQ + nu + 8 * h * PS;
+            const int2* at = sm.pxy + k * NV + nu + 8 * h * G;
+            const int one = (1 << fr.shift) - 1;
+            int2 a = at[0], q = at[1];
+            int lx = min(a.x, q.x), hx = max(a.x, q.x), ly = min(a.y, q.y), hy = max(a.y, q.y);
+            int slx = lx, shx = hx, sly = ly, shy = hy;   // the strip's bounds
+            unsigned inside = 0;                          // quads with a pixel centre in their bbox, frame ignored
+            unsigned wind = 0;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int2 c2 = at[(r + 1) * G], c3 = at[(r + 1) * G + 1];
+                const int nlx = min(c2.x, c3.x), nhx = max(c2.x, c3.x), nly = min(c2.y, c3.y), nhy = max(c2.y, c3.y);
+                const int minx = min(lx, nlx), maxx = max(hx, nhx), miny = min(ly, nly), maxy = max(hy, nhy);
+                if (((minx + one) >> fr.shift) <= (maxx >> fr.shift) && ((miny + one) >> fr.shift) <= (maxy >> fr.shift))
+                    inside |= 1u << r;
+                // is_front_facing (kernels/reyes.cl:54-65) on wrapped int32
+                const int d1x = wsub(q.x, a.x), d1y = wsub(q.y, a.y);
+                const int d2x = wsub(c2.x, a.x), d2y = wsub(c2.y, a.y);
+                const int d3x = wsub(c3.x, a.x), d3y = wsub(c3.y, a.y);
+                if (wsub(wmul(d1x, d3y), wmul(d3x, d1y)) < 0 || wsub(wmul(d3x, d2y), wmul(d2x, d3y)) < 0) wind |= 1u << r;
+                slx = min(slx, nlx);
+                shx = max(shx, nhx);
+                sly = min(sly, nly);
+                shy = max(shy, nhy);
+                lx = nlx; hx = nhx; ly = nly; hy = nhy;
+                a = c2;
+                q = c3;
+            }
+            if (slx >= 0 && sly >= 0 && shx < (fr.W << fr.shift) && shy < (fr.H << fr.shift) &&
+                shx - slx <= kFastExtent && shy - sly <= kFastExtent) {
+                // the strip is small and inside the frame, so every quad of it is
+                live = inside & wind;
+            } else {
+#pragma unroll 1
+                for (int r = 0; r < 8; ++r) {
+                    const int2 p0 = at[r * G], p1 = at[r * G + 1], p2 = at[(r + 1) * G], p3 = at[(r + 1) * G + 1];
+                    const int qx[4] = {p0.x, p1.x, p2.x, p3.x}, qy[4] = {p0.y, p1.y, p2.y, p3.y};
+                    int minx, miny, maxx, maxy, x0, y0, x1, y1;
+                    if (!quad_is_fast(qx, qy, minx, miny, maxx, maxy) ||
+                        (((wind >> r) & 1u) && quad_pixels(fr, minx, miny, maxx, maxy, x0, y0, x1, y1)))
+                        live |= 1u << r;
+                }
+            }
         }
+        // append the strips' quads: one shared add per warp, a prefix over the lanes
+        const int cnt = __popc(live);
+        const int total = __reduce_add_sync(0xffffffffu, cnt);
+        if (total == 0) continue;
+        int pre = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += y;
+        }
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(&sm.n_live[b], (unsigned)total);
+        at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)(pre - cnt);
+        for (unsigned m = live; m; m &= m - 1) sm.live[at++] = (unsigned short)(first + (__ffs(m) - 1) * PS);
     }
     __syncthreads();
     // the next group's weights and state, from the highest thread down (the
@@ -397,10 +557,7 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
         const int i = sm.live[j];
         const int k = i / NQ, q = i % NQ;
         const int nu = q % PS, nv = q / PS, blk = (nu >> 3) + (nv >> 3) * BPL;
-        // the block's tile range, or skip it (clamp, eye-plane flag, is_empty)
-        const int* bb = sm.bound[b][k][blk];
-        int tiles[4];
-        if (!block_tiles(fr, bb[0], bb[1], bb[2], bb[3], !((sm.zero[b][k] >> blk) & 1), tiles)) continue;
+        if ((sm.zero[b][k] >> blk) & 1) continue;   // an eye-plane vertex skips the block
         const int i0 = k * NV + nu + nv * G;
         const int idx[4] = {i0, i0 + 1, i0 + G, i0 + G + 1};
         int qx[4], qy[4];
@@ -420,10 +577,14 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
         unsigned long long* keys = fb.keys + (long long)view * fb.key_pixels;
         int minx, miny, maxx, maxy, f = 0;
         const bool fast = quad_is_fast(qx, qy, minx, miny, maxx, maxy);
-        if (fast)
-            f = raster_quad_fast(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id);
-        else
-            push_big(big, big_cap, ctrl, qx, qy, qd, mp_id, view, tiles);
+        if (!fast || maxx <= 0) {
+            const int4 t = group_block_tiles<G>(sm.pxy + k * NV + (nu & ~7) + (nv & ~7) * G, fr.W, fr.H, fr.shift,
+                                                fr.backface);
+            if (t.x > t.z) continue;
+            const int tiles[4] = {t.x, t.y, t.z, t.w};
+            if (!fast) push_big(big, big_cap, ctrl, qx, qy, qd, mp_id, view, tiles);
+        }
+        if (fast) f = raster_quad_fast(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id);
         if (f > 0 || !fast) {
             // the diffuse factor of a quad that may own pixels; resolve
             // turns it into the colour of kernels/reyes.cl:191
@@ -437,7 +598,7 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
 }
 
 template <int PS, int NS, bool DISP>
-__global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>())
+__global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     raster_fused_kernel(const DrawDev* __restrict__ draws, FrameDev frp, SubPatches sub, Framebuffer fb,
                         float* __restrict__ mshade, BigQuad* big, long long big_cap, unsigned long long* ctrl) {
     using SM = FusedSmem<PS, NS>;
@@ -485,7 +646,7 @@ constexpr size_t frame_smem() {
 }
 
 template <int PS, int NS>
-__global__ void __launch_bounds__(fused_threads<NS>(), 768 / fused_threads<NS>())
+__global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     frame_kernel(const DrawDev* __restrict__ gdraws, const int* __restrict__ root_prefix, int n_draws, FrameDev frp,
                  Queue q, SubPatches sub, Framebuffer fb, float* __restrict__ mshade, BigQuad* big, long long big_cap,
                  unsigned long long* ctrl, long long spin_limit, int n_bns_ctas) {
@@ -887,7 +1048,8 @@ int resident_grid(K kernel, size_t smem, int threads) {
     return sms * per_sm;
 }
 
-// Calls f(kernel instantiation tag) for the (PS, dice_group) pair.
+// Calls f(kernel instantiation tag) for the (PS, dice_group) pair: the shape
+// next to the nominal group whose threads the runs and strips fill.
 template <int PS, int NS>
 struct Tag {
     static constexpr int ps = PS, ns = NS;
@@ -898,12 +1060,12 @@ void dispatch_group(int PS, int group, F&& f) {
         if (group == 2) f(Tag<16, 2>{});
         else if (group == 3) f(Tag<16, 3>{});
         else if (group == 4) f(Tag<16, 4>{});
-        else f(Tag<16, 6>{});
+        else f(Tag<16, 5>{});
     } else {
-        if (group == 8) f(Tag<8, 8>{});
-        else if (group == 11) f(Tag<8, 11>{});
-        else if (group == 16) f(Tag<8, 16>{});
-        else f(Tag<8, 22>{});
+        if (group == 8) f(Tag<8, 7>{});
+        else if (group == 16) f(Tag<8, 18>{});
+        else if (group == 22) f(Tag<8, 21>{});
+        else f(Tag<8, 14>{});
     }
 }
 
