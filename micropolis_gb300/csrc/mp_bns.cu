@@ -32,11 +32,17 @@ template <int CRIT>
 __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev* __restrict__ gdraws,
                                                                    const int* __restrict__ root_prefix,
                                                                    int n_draws, FrameDev fr, Queue q,
-                                                                   SubPatches out, unsigned long long* ctrl,
-                                                                   long long spin_limit) {
+                                                                   SubPatches out, RootInfo* roots,
+                                                                   unsigned* __restrict__ table,
+                                                                   const unsigned* __restrict__ used,
+                                                                   unsigned long long* ctrl, long long spin_limit) {
     // draw constants staged in shared memory when they fit
     __shared__ DrawDev s_draws[kBnsSmemDraws];
     extern __shared__ __align__(16) float s_bns[];
+    // the last frame's entries of the sort's bucket table (whole uint4s), while the first ranges are on their way
+    const unsigned n_clear = __ldg(used) / 4;
+    for (unsigned i = blockIdx.x * kBnsBlock + threadIdx.x; i < n_clear; i += gridDim.x * kBnsBlock)
+        reinterpret_cast<uint4*>(table)[i] = make_uint4(0, 0, 0, 0);
     const bool staged = n_draws <= kBnsSmemDraws;
     if (staged) {
         const int words = n_draws * (int)(sizeof(DrawDev) / 4);
@@ -46,7 +52,7 @@ __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev
     }
     // consecutive warp numbers on different SMs: the first roots spread over the chip
     const int warp = (int)(blockIdx.x + gridDim.x * (threadIdx.x >> 5));
-    bns_warp_loop<CRIT, kStackPairs>(staged ? s_draws : gdraws, root_prefix, n_draws, fr, q, out, nullptr, ctrl,
+    bns_warp_loop<CRIT, kStackPairs>(staged ? s_draws : gdraws, root_prefix, n_draws, fr, q, out, nullptr, roots, ctrl,
                                      spin_limit, s_bns, warp, (int)(gridDim.x * (kBnsBlock / 32)));
 }
 
@@ -257,14 +263,14 @@ int bns_persistent_grid(int criterion) {
 }
 
 void launch_bns_persistent(const DrawDev* draws, const int* root_prefix, int n_draws, const FrameDev& fr,
-                           const Queue& q, const SubPatches& out, unsigned long long* ctrl, int grid,
-                           long long spin_limit, cudaStream_t s) {
+                           const Queue& q, const SubPatches& out, const SortBuffers& sb, unsigned long long* ctrl,
+                           int grid, long long spin_limit, cudaStream_t s) {
     if (fr.criterion == 1)
-        bns_persistent_kernel<1><<<grid, kBnsBlock, kBnsSmem, s>>>(draws, root_prefix, n_draws, fr, q, out, ctrl,
-                                                                    spin_limit);
+        bns_persistent_kernel<1><<<grid, kBnsBlock, kBnsSmem, s>>>(draws, root_prefix, n_draws, fr, q, out, sb.roots, sb.table, sb.used,
+                                                                    ctrl, spin_limit);
     else
-        bns_persistent_kernel<0><<<grid, kBnsBlock, kBnsSmem, s>>>(draws, root_prefix, n_draws, fr, q, out, ctrl,
-                                                                    spin_limit);
+        bns_persistent_kernel<0><<<grid, kBnsBlock, kBnsSmem, s>>>(draws, root_prefix, n_draws, fr, q, out, sb.roots, sb.table, sb.used,
+                                                                    ctrl, spin_limit);
 }
 
 void launch_bns_init_stack(const RangeStack& stack, int draw, int n_patches, cudaStream_t s) {

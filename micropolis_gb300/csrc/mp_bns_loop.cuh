@@ -55,6 +55,7 @@ __device__ __forceinline__ void bns_reset(unsigned long long* ctrl, long long ro
     *cw(ctrl, kGroupTicket) = 0;
     *cw(ctrl, kMaxDepth) = 0;
     *cw(ctrl, kSortDone) = 0;
+    *cw(ctrl, kSortMost) = 0;
 }
 
 __device__ __forceinline__ void set_status(unsigned long long* ctrl, int code) {
@@ -95,7 +96,9 @@ constexpr size_t bns_smem() {
 // Runs one warp's share of a frame's bound-and-split until the done flag is
 // raised.  Emitted sub-patches go to `out`; when out_seq is given, each
 // emitted slot is also marked with the frame's epoch (release) for consumers
-// that run concurrently.  CRIT selects the bound criterion (bns_decide).
+// that run concurrently; when roots is given, each root's record counts its
+// sub-patches and bounds their paths (for the canonical sort).  CRIT selects
+// the bound criterion (bns_decide).
 // `warp` is the warp's number among the n_warps that run the loop.
 //
 // A warp works depth first on a stack of its own: a step takes up to 16
@@ -116,7 +119,8 @@ constexpr size_t bns_smem() {
 template <int CRIT, int C>
 __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* __restrict__ root_prefix, int n_draws,
                                               const FrameDev& fr, const Queue& q, const SubPatches& out,
-                                              unsigned* out_seq, unsigned long long* ctrl, long long spin_limit,
+                                              unsigned* out_seq, RootInfo* roots, unsigned long long* ctrl,
+                                              long long spin_limit,
                                               float* smem, int warp, int n_warps) {
     static_assert(C >= 32, "a step adds up to 16 pairs, or 32 to an empty ring");
     // Pairs are given to waiting warps when more than kGiveAbove are left, and
@@ -310,6 +314,29 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
             // the sort packs the frame's keys into root bits above this many path bits
             max_depth = emit_depth;
             if (lane == 0) atomicMax(cw(ctrl, kMaxDepth), (unsigned long long)emit_depth);
+        }
+        if (roots && emask) {
+            // one update per warp while its emitted ranges share a root, as
+            // they do below the first levels of a tree, else one per root
+            const unsigned ri = (unsigned)(__ldg(root_prefix + draw) + pid);
+            const unsigned r0 = __shfl_sync(0xffffffffu, ri, __ffs(emask) - 1);
+            if (__all_sync(0xffffffffu, dec != kDraw || ri == r0)) {
+                const unsigned low = __reduce_min_sync(0xffffffffu, dec == kDraw ? path : 0xffffffffu);
+                const unsigned high = __reduce_max_sync(0xffffffffu, dec == kDraw ? path : 0u);
+                if (lane == 0) {
+                    atomicAdd(&roots[r0].count, (unsigned)__popc(emask));
+                    atomicMin(&roots[r0].low, low);
+                    atomicMax(&roots[r0].high, high);
+                }
+            } else if (dec == kDraw) {
+                const unsigned peers = __match_any_sync(emask, ri);
+                const unsigned low = __reduce_min_sync(peers, path), high = __reduce_max_sync(peers, path);
+                if ((peers & lanemask_lt()) == 0) {
+                    atomicAdd(&roots[ri].count, (unsigned)__popc(peers));
+                    atomicMin(&roots[ri].low, low);
+                    atomicMax(&roots[ri].high, high);
+                }
+            }
         }
         // split ranges: one pair each, once every lane has read the popped pairs
         __syncwarp();

@@ -66,6 +66,8 @@ struct mp_ctx {
     SubPatches sorted{};              // the same in canonical order (batched path, two launches)
     SortBuffers sb{};
     int sort_passes = 0;              // radix passes captured for this frame
+    RootInfo* root_info = nullptr;    // per root of the frame (sb.roots)
+    long long root_cap = 0;
     BigQuad* big = nullptr;
     long long big_cap = 0;
     float* mshade = nullptr;          // diffuse factor per micropolygon (batched path)
@@ -181,6 +183,9 @@ void free_sorted(mp_ctx* c) {
         dfree(c->sb.keys[k]);
         dfree(c->sb.vals[k]);
     }
+    dfree(c->sb.table);
+    dfree(c->sb.used);
+    dfree(c->sb.sums);
     dfree(c->sb.hist);
     dfree(c->sb.counts);
     dfree(c->sb.group_counts);
@@ -234,6 +239,7 @@ mp_status grow_sub(mp_ctx* c, long long need, bool keep) {
     o.capacity = cap;
     c->sorted = o;
     SortBuffers b{};
+    b.roots = c->root_info;
     b.capacity = cap;
     b.tiles = sort_tiles(cap);
     b.groups = (b.tiles + kSortGroup - 1) / kSortGroup;
@@ -242,10 +248,28 @@ mp_status grow_sub(mp_ctx* c, long long need, bool keep) {
         CK(dalloc(&c->sb.keys[k], cap));
         CK(dalloc(&c->sb.vals[k], cap));
     }
-    CK(dalloc(&c->sb.hist, 2 * kSortPasses * 256));
+    const long long entries = (cap + 7) / 4 * 4;   // and the end, in whole uint4s
+    CK(dalloc(&c->sb.table, entries));
+    CK(cudaMemsetAsync(c->sb.table, 0, sizeof(unsigned) * (size_t)entries, c->stream));
+    CK(dalloc(&c->sb.used, 1));
+    CK(cudaMemsetAsync(c->sb.used, 0, sizeof(unsigned), c->stream));
+    CK(dalloc(&c->sb.sums, kSortSums));
+    CK(dalloc(&c->sb.hist, kSortPasses * 256));
     CK(dalloc(&c->sb.counts, c->sb.tiles * 256));
     CK(dalloc(&c->sb.group_counts, kSortPasses * c->sb.groups * 256));
-    CK(cudaMemsetAsync(c->sb.hist, 0, sizeof(unsigned) * 2 * kSortPasses * 256, c->stream));
+    return MP_OK;
+}
+
+mp_status grow_roots(mp_ctx* c, long long need) {
+    if (need <= c->root_cap) return MP_OK;
+    c->graph_stale = true;
+    const long long cap = std::max(need, 2 * c->root_cap);
+    dfree(c->root_info);
+    c->root_info = c->sb.roots = nullptr;
+    c->root_cap = 0;
+    CK(dalloc(&c->root_info, cap));
+    c->root_cap = cap;
+    c->sb.roots = c->root_info;
     return MP_OK;
 }
 
@@ -515,7 +539,7 @@ void enqueue_frame(mp_ctx* c, int n, long long roots, bool capturing) {
     cudaMemcpyAsync(c->d_root_prefix, c->h_root_prefix, sizeof(int) * (size_t)(n + 1), cudaMemcpyHostToDevice,
                     c->stream);
     mark(c, 0, capturing);
-    launch_clear(c->fb, c->fr, 0, c->stream, c->ctrl, roots);
+    launch_clear(c->fb, c->fr, 0, c->stream, c->ctrl, roots, overlapped(c) ? nullptr : c->root_info);
     mark(c, 1, capturing);
     if (overlapped(c)) {
         // one launch, reported as dice+raster; bound-and-split and sort show 0
@@ -524,7 +548,7 @@ void enqueue_frame(mp_ctx* c, int n, long long roots, bool capturing) {
         launch_frame_kernel(c->d_draws, c->d_root_prefix, n, c->fr, c->q, c->sub, c->fb, c->mshade, c->big, c->big_cap,
                             c->ctrl, c->opt.spin_limit, c->frame_grid, bns_blocks(c), c->opt.dice_group, c->stream);
     } else {
-        launch_bns_persistent(c->d_draws, c->d_root_prefix, n, c->fr, c->q, c->sub, c->ctrl, c->bns_grid,
+        launch_bns_persistent(c->d_draws, c->d_root_prefix, n, c->fr, c->q, c->sub, c->sb, c->ctrl, c->bns_grid,
                               c->opt.spin_limit, c->stream);
         mark(c, 2, capturing);
         launch_sort(c);
@@ -596,7 +620,8 @@ mp_status batched_frame(mp_ctx* c) {
     long long qcap = c->opt.queue_capacity > 0 ? (c->opt.queue_capacity + 2 * kBundlePairs - 1) / (2 * kBundlePairs)
                                                : auto_queue_cap(roots);
     long long scap = c->opt.subpatch_capacity > 0 ? c->opt.subpatch_capacity : auto_sub_cap(roots);
-    if ((st = grow_queue(c, qcap)) || (st = grow_sub(c, scap, false)) || (st = grow_big(c, 1 << 16)) ||
+    if ((st = grow_queue(c, qcap)) || (st = grow_sub(c, scap, false)) ||
+        (st = grow_roots(c, std::max(roots, 4096LL))) || (st = grow_big(c, 1 << 16)) ||
         (st = ensure_mshade(c)))
         return st;
     const int passes = canonical_sort_passes(c->opt.max_split_depth, roots);
@@ -847,6 +872,7 @@ void mp_destroy(mp_ctx* c) {
     dfree(c->q.words); dfree(c->q.seq);
     dfree(c->sub.range); dfree(c->sub.meta); dfree(c->sub.seq); dfree(c->sub.path);
     free_sorted(c);
+    dfree(c->root_info);
     dfree(c->big);
     dfree(c->mshade);
     dfree(c->fb.keys); dfree(c->fb.color); dfree(c->fb.depth);
@@ -1166,7 +1192,8 @@ mp_status mp_dump_stats(mp_ctx* c, char* buf, size_t cap) {
         {"sub-patch list", c->sub.capacity * (long long)(sizeof(float4) + sizeof(int2) + 2 * sizeof(unsigned))},
         {"canonical sub-patch list", c->sorted.capacity * (long long)(sizeof(float4) + sizeof(int2))},
         {"canonical order sort", c->sb.capacity * 2 * (long long)(sizeof(unsigned long long) + sizeof(unsigned)) +
-                                     (c->sb.tiles + kSortPasses * c->sb.groups) * 256 * (long long)sizeof(unsigned)},
+                                     ((c->sb.tiles + kSortPasses * c->sb.groups) * 256 + c->sb.capacity) *
+                                         (long long)sizeof(unsigned)},
         {"diffuse factors", c->mshade_cap * (long long)sizeof(float)},
         {"framebuffer", c->fb.key_pixels * c->fb.views * 8 + c->fb.pixels * c->fb.views * 20},
         {"exact slow raster quads", c->big_cap * (long long)sizeof(BigQuad)},

@@ -31,6 +31,7 @@ enum CtrlWord {
     kMaxDepth,         // deepest split path of an emitted sub-patch (canonical sort keys)
     kSortTicket,       // tile tickets of the canonical sort, one word per radix pass (kSortPasses)
     kSortDone = kSortTicket + 8,   // grid-barrier arrivals of the sort kernel this frame
+    kSortMost,         // keys of the fullest bucket of the canonical sort, when it is too full
     kNumCtrl
 };
 constexpr int kCtrlStride = 16;  // unsigned long long words per line
@@ -61,6 +62,13 @@ struct SubPatches {         // emitted sub-patch list
                             // its depth-d ancestor's split (nullptr: not kept)
 };
 
+// A root's emitted sub-patches: how many, their lowest and highest split path,
+// and its first place in the canonical list.
+struct RootInfo {
+    unsigned count, low, high, start;
+};
+static_assert(sizeof(RootInfo) == 16, "read as one uint4");
+
 // Canonical order of a frame's sub-patches: ascending (root, split path),
 // root = the draw's first root + patch id.  Scratch of the radix sort that
 // establishes it (mp_sort.cu).
@@ -68,7 +76,11 @@ constexpr int kSortPasses = 8;          // 8-bit digits of the 64-bit key
 struct SortBuffers {
     unsigned long long* keys[2];        // ping-pong keys
     unsigned* vals[2];                  // ping-pong source slots
-    unsigned* hist;                     // 2 (frame parity) x kSortPasses x 256 digit counts
+    unsigned* table;                    // counts, then starts, of the buckets; zero where not in use
+    unsigned* used;                     // entries of the table the last sort used (bound-and-split clears them)
+    unsigned* sums;                     // keys in each block's stretch of the table
+    RootInfo* roots;                    // one per root of the frame
+    unsigned* hist;                     // kSortPasses x 256 digit counts
     unsigned* counts;                   // per pass: digit counts of each tile, tiles x 256
     unsigned* group_counts;             // kSortPasses x groups x 256: counts of groups of kSortGroup tiles
     long long capacity;                 // keys per buffer
@@ -76,6 +88,7 @@ struct SortBuffers {
     long long groups;                   // tile groups at capacity
 };
 constexpr int kSortGroup = 32;          // tiles per group of the pass's prefix
+constexpr int kSortSums = 4096;         // most blocks of the sort
 
 struct BigQuad {            // a quad rasterized by the exact tile emulation
     int px[4], py[4];
@@ -99,8 +112,8 @@ enum { kOk = 0, kErrInvalidArg = 1, kErrOutOfMemory = 2, kErrOverflow = 3, kErrT
 
 // ---- bound-and-split (mp_bns.cu)
 void launch_bns_persistent(const DrawDev* draws, const int* root_prefix, int n_draws, const FrameDev& fr,
-                           const Queue& q, const SubPatches& out, unsigned long long* ctrl, int grid,
-                           long long spin_limit, cudaStream_t s);
+                           const Queue& q, const SubPatches& out, const SortBuffers& sb, unsigned long long* ctrl,
+                           int grid, long long spin_limit, cudaStream_t s);
 int bns_persistent_grid(int criterion);
 // plain per-pass bound-and-split (the reference's BOUNDED structure)
 void launch_bns_init_stack(const RangeStack& stack, int draw, int n_patches, cudaStream_t s);
@@ -130,9 +143,10 @@ int canonical_sort_passes(int max_split_depth, long long roots);
 
 // ---- dice / shade / raster / resolve (mp_raster.cu)
 // clears the key buffer (and with_color: colour and depth); with reset_ctrl,
-// also resets the frame's bound-and-split control words for `roots` roots
+// also resets the frame's bound-and-split control words for `roots` roots and
+// (root_info not null) their records
 void launch_clear(const Framebuffer& fb, const FrameDev& fr, int with_color, cudaStream_t s,
-                  unsigned long long* reset_ctrl = nullptr, long long roots = 0);
+                  unsigned long long* reset_ctrl = nullptr, long long roots = 0, RootInfo* root_info = nullptr);
 void launch_raster_fused(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
                          float* mshade, BigQuad* big, long long big_cap, unsigned long long* ctrl, int grid, int group,
                          cudaStream_t s);

@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
         }
         // the CPU criterion only: the host runs the GPU criterion as two launches
         bns_warp_loop<0, kStackPairsFrame>(
-            staged ? sd : gdraws, root_prefix, n_draws, fr, q, sub, sub.seq, ctrl, spin_limit,
+            staged ? sd : gdraws, root_prefix, n_draws, fr, q, sub, sub.seq, nullptr, ctrl, spin_limit,
             reinterpret_cast<float*>(smem_raw + kPtsOffset), (int)(blockIdx.x + n_bns_ctas * (threadIdx.x >> 5)),
             n_bns_ctas * (fused_threads<NS>() / 32));
         __syncthreads();
@@ -795,12 +795,15 @@ __global__ void __launch_bounds__(kBigThreads) raster_big_kernel(FrameDev fr, Fr
 }
 
 __global__ void clear_kernel(Framebuffer fb, FrameDev fr, int with_color, unsigned long long* reset_ctrl,
-                             long long roots) {
+                             long long roots, RootInfo* root_info) {
     // the frame's bound-and-split reset rides along (one thread)
     if (reset_ctrl && blockIdx.x == 0 && threadIdx.x == 0) bns_reset(reset_ctrl, roots);
     const long long nk = fb.key_pixels * fb.views, n = fb.pixels * fb.views;
     const float4 cc = make_float4(fr.clear[0], fr.clear[1], fr.clear[2], fr.clear[3]);
     const long long stride = (long long)gridDim.x * blockDim.x;
+    if (root_info)
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < roots; i += stride)
+            reinterpret_cast<uint4*>(root_info)[i] = make_uint4(0u, 0xffffffffu, 0u, 0u);
     // the key buffer is a whole number of 32x32 tiles per view: two keys per 16-byte store
     ulonglong2* k2 = reinterpret_cast<ulonglong2*>(fb.keys);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nk / 2; i += stride)
@@ -1082,13 +1085,13 @@ int grid_for(long long n, int block) {
 // launchers
 
 void launch_clear(const Framebuffer& fb, const FrameDev& fr, int with_color, cudaStream_t s,
-                  unsigned long long* reset_ctrl, long long roots) {
+                  unsigned long long* reset_ctrl, long long roots, RootInfo* root_info) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long want = with_color ? fb.pixels * fb.views : fb.key_pixels * fb.views / 2;
-    clear_kernel<<<(int)std::min<long long>(grid_for(want, 256), (long long)sms * 8), 256, 0, s>>>(fb, fr, with_color,
-                                                                                             reset_ctrl, roots);
+    clear_kernel<<<(int)std::min<long long>(grid_for(want, 256), (long long)sms * 8), 256, 0, s>>>(
+        fb, fr, with_color, reset_ctrl, roots, root_info);
 }
 
 int raster_fused_grid(int PS, int group, int displacement) {

@@ -13,13 +13,31 @@
 // depth-first order of its split tree, low half first.  The oracle numbers
 // its sub-patches in the same order, so the two break ties identically.
 //
-// The sort is a least-significant-digit radix sort over 8-bit digits of a
-// key that packs the root above the frame's D path bits (D = the deepest
-// emitted sub-patch, which bound-and-split records; below bit 32 - D every
-// path is zero, so the order is that of (root << 32 | path)).  Keys are 32
-// bits wide when the frame's root and path bits fit, else 64.  It is one
-// launch of a resident grid, in phases separated by grid barriers (bounded
-// waits on a counter of the frame's control words):
+// The sort is one launch of a resident grid, in phases separated by grid
+// barriers (bounded waits on a counter of the frame's control words).
+// Bound-and-split has counted each root's sub-patches and their lowest and
+// highest path, so a root's place in the list is known after one prefix sum,
+// and its paths are spread over as many buckets as it has sub-patches:
+//   roots -- the roots' starts;
+//   count -- every sub-patch takes a place in its bucket, the leading bits of
+//            its path above the root's lowest (one atomic);
+//   scan  -- the buckets' starts (sums of each block's stretch, then prefixes);
+//   place -- path and source slot go to the bucket's next place;
+//   rank  -- each sub-patch counts the smaller paths of its bucket and its
+//            record is written to its final place.
+// Each phase is one or two round trips to L2 per sub-patch and a barrier
+// (about 4 us on a small frame).  Against the radix passes below, which cost
+// some 20 us each: 13,496 sub-patches 51 -> 23 us, the mixed scene's 1.38 M
+// 150 -> 61 us, 64 views' 5.66 M 593 -> 206 us, 2.73 M of the 512x512
+// heightfield 240 -> 100 us.  Buckets of one size for the whole frame
+// (leading bits of root and path) left thousands of a deeply split patch's
+// sub-patches in one bucket.  A frame whose fullest
+// bucket still holds more than kMaxBucket (a patch split deeply in a small
+// part of its visible range) is sorted by radix passes instead, whose cost
+// does not depend on the paths.  Their key packs the root above the frame's D
+// path bits (D = the deepest emitted sub-patch; below bit 32 - D every path
+// is zero, so the order is that of (root << 32 | path)); keys are 32 bits wide
+// when the frame's root and path bits fit, else 64:
 //   counts -- the digit counts of every pass at once (Adinets & Merrill's
 //             one-sweep radix sort; warp matches aggregate a warp's equal
 //             digits into one shared add), added to the frame's table;
@@ -42,7 +60,12 @@ namespace mp {
 
 namespace {
 
-constexpr int kKeysBlock = 1024;
+// The largest bucket that is ranked by counting: 2,048 paths cost each of them
+// 2,048 compares of words in L1, a few microseconds, less than a radix pass.
+constexpr unsigned kMaxBucket = 2048;
+// Up to this many entries each block adds up the stretches before its own
+// (32 loads a thread) instead of waiting for every block's sum.
+constexpr unsigned kSumAlone = 16384;
 constexpr int kSortBlock = 512;
 constexpr int kSortWarps = kSortBlock / 32;
 constexpr int kSortItems = 8;
@@ -55,16 +78,6 @@ __device__ __forceinline__ long long sort_count(const unsigned long long* ctrl, 
     if (n > in.capacity) n = in.capacity;
     if (n > sb.capacity) n = sb.capacity;
     return n;
-}
-
-__device__ __forceinline__ unsigned frame_epoch(const unsigned long long* ctrl) {
-    return (unsigned)*(volatile const unsigned long long*)(ctrl + kEpoch * kCtrlStride);
-}
-
-// Counts of the frame's passes: one table per frame parity, so that a
-// frame clears the next frame's table while its own is read.
-__device__ __forceinline__ unsigned* hist_of(const SortBuffers& sb, unsigned epoch) {
-    return sb.hist + (epoch & 1u) * kSortPasses * kDigits;
 }
 
 template <typename K>
@@ -349,11 +362,234 @@ __device__ __forceinline__ bool pass_body(PassSmem& sm, const int* __restrict__ 
     return true;
 }
 
+// Sum over the block (every thread calls it and gets the sum; ends with a barrier).
+__device__ __forceinline__ unsigned block_sum(unsigned v, unsigned* warp_sum) {
+    const int tid = threadIdx.x;
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((tid & 31) == 0) warp_sum[tid >> 5] = v;
+    __syncthreads();
+    unsigned t = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) t += warp_sum[w];
+    __syncthreads();
+    return t;
+}
+
+// How many of keys[from, to) are below `key`: eight at a time, so that a
+// bucket of hundreds costs a few cycles a key and not a load's latency each
+// (the sort of the mixed 4,096-patch scene: 0.31 -> 0.12 ms).
+__device__ __forceinline__ unsigned count_below(const unsigned* keys, unsigned from, unsigned to, unsigned key) {
+    unsigned c = 0, j = from;
+    for (; j < to && (j & 3u); ++j) c += keys[j] < key;
+    for (; j + 8 <= to; j += 8) {
+        const uint4 a = *reinterpret_cast<const uint4*>(keys + j), b = *reinterpret_cast<const uint4*>(keys + j + 4);
+        c += (a.x < key) + (a.y < key) + (a.z < key) + (a.w < key) + (b.x < key) + (b.y < key) + (b.z < key) +
+             (b.w < key);
+    }
+    for (; j < to; ++j) c += keys[j] < key;
+    return c;
+}
+
+// A root's bucket of a path: the root's start and the leading bits of the
+// path above its lowest, at most as many buckets as it has sub-patches.
+__device__ __forceinline__ unsigned bucket_of(const RootInfo& ri, unsigned path) {
+    const int range_bits = 32 - __clz((int)(ri.high - ri.low));
+    const int shift = max(0, range_bits - (31 - __clz((int)ri.count)));
+    return ri.start + ((path - ri.low) >> shift);
+}
+
+__device__ __forceinline__ RootInfo load_root(const RootInfo* r) {
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(r));
+    return RootInfo{v.x, v.y, v.z, v.w};
+}
+
+// Exclusive prefix over the block of each thread's v, from `run`; adds the
+// block's total to run (every thread calls it; ends with a barrier).
+__device__ __forceinline__ unsigned block_prefix(unsigned v, unsigned& run, unsigned* warp_sum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sum[warp] = x;
+    __syncthreads();
+    unsigned pre = run, all = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+        if (w < warp) pre += warp_sum[w];
+        all += warp_sum[w];
+    }
+    __syncthreads();
+    run += all;
+    return pre + x - v;
+}
+
+// The sum of all entries before this block's stretch: `entry(i)` reads one,
+// lo is the stretch's begin, per its length, own its sum.  Long tables go
+// through every block's sum and a barrier; false when that wait ran out.
+template <typename F>
+__device__ __forceinline__ bool sum_before(F entry, unsigned total, unsigned lo, unsigned own, unsigned* sums,
+                                           unsigned long long* ctrl, int nblk, unsigned long long& barrier,
+                                           long long spin_limit, unsigned* warp_sum, int* s_flag, unsigned& before) {
+    const int tid = threadIdx.x;
+    unsigned v = 0;
+    if (total <= kSumAlone) {
+        for (unsigned i = tid; i < lo; i += kSortBlock) v += entry(i);
+    } else {
+        own = block_sum(own, warp_sum);
+        if (tid == 0) sums[blockIdx.x] = own;
+        if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return false;
+        for (int j = tid; j < (int)blockIdx.x; j += kSortBlock) v += __ldcg(sums + j);
+    }
+    before = block_sum(v, warp_sum);
+    return true;
+}
+
+// The bucket sort (file header).  Returns 1 when done, 0 when a bucket is too
+// full (nothing is written to `out`), -1 when a wait ran out.
+__device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, const SubPatches& in,
+                                           const SubPatches& out, const SortBuffers& sb, unsigned long long* ctrl,
+                                           long long n, int nblk, unsigned long long& barrier, long long spin_limit,
+                                           unsigned* warp_sum, int* s_flag) {
+    constexpr int kBatch = 4;   // sub-patches a thread handles at a time, their loads in flight together
+    const int tid = threadIdx.x;
+    const long long gt = (long long)blockIdx.x * kSortBlock + tid, stride = (long long)nblk * kSortBlock;
+    const unsigned R = (unsigned)*(volatile unsigned long long*)cw(ctrl, kRoots);
+    RootInfo* roots = sb.roots;
+    unsigned* table = sb.table;
+    unsigned* place = sb.vals[0];
+    unsigned* slot_path = reinterpret_cast<unsigned*>(sb.keys[0]);
+    unsigned* slot_src = sb.vals[1];
+    // the next frame's bound-and-split clears what this one uses of the table
+    if (gt == 0) *sb.used = (unsigned)n + 4;
+    {
+        // roots
+        const unsigned per = (R + nblk - 1) / nblk, lo = min(per * blockIdx.x, R), hi = min(lo + per, R);
+        unsigned own = 0, run = 0;
+        if (R > kSumAlone)
+            for (unsigned i = lo + tid; i < hi; i += kSortBlock) own += __ldcg(&roots[i].count);
+        if (!sum_before([&](unsigned i) { return __ldcg(&roots[i].count); }, R, lo, own, sb.sums, ctrl, nblk, barrier,
+                        spin_limit, warp_sum, s_flag, run))
+            return -1;
+        for (unsigned t0 = lo; t0 < hi; t0 += kSortBlock) {
+            const unsigned i = t0 + tid;
+            const unsigned pre = block_prefix(i < hi ? __ldcg(&roots[i].count) : 0u, run, warp_sum);
+            if (i < hi) roots[i].start = pre;
+        }
+    }
+    if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+    // count
+    for (long long i0 = gt; i0 < n; i0 += kBatch * stride) {
+        int2 m[kBatch];
+        unsigned p[kBatch], at[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const long long i = min(i0 + u * stride, n - 1);
+            m[u] = __ldcg(in.meta + i);
+            p[u] = __ldcg(in.path + i);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) at[u] = bucket_of(load_root(roots + __ldg(root_prefix + m[u].y) + m[u].x), p[u]);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (i0 + u * stride < n && at[u] < (unsigned)n) at[u] = atomicAdd(table + at[u], 1u);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (i0 + u * stride < n) place[i0 + u * stride] = at[u];
+    }
+    if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+    {
+        // scan: this block's stretch of the table, whole uint4s
+        const unsigned nb = (unsigned)n, per = ((nb + nblk - 1) / nblk + 3) & ~3u;
+        const unsigned lo = min(per * blockIdx.x, nb), hi = min(lo + per, nb);
+        unsigned own = 0, most = 0, run = 0;
+        for (unsigned i = lo + 4 * tid; i < hi; i += 4 * kSortBlock) {
+            const uint4 c = __ldcg(reinterpret_cast<const uint4*>(table + i));
+            own += c.x + c.y + c.z + c.w;
+            most = max(max(max(most, c.x), max(c.y, c.z)), c.w);
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        if ((tid & 31) == 0 && most > kMaxBucket) atomicMax(cw(ctrl, kSortMost), (unsigned long long)most);
+        if (!sum_before([&](unsigned i) { return __ldcg(table + i); }, nb, lo, own, sb.sums, ctrl, nblk, barrier,
+                        spin_limit, warp_sum, s_flag, run))
+            return -1;
+        // (short tables: every entry is read before any is written)
+        if (nb <= kSumAlone && !grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+        if (*(volatile unsigned long long*)cw(ctrl, kSortMost)) return 0;
+        for (unsigned t0 = lo; t0 < hi; t0 += 4 * kSortBlock) {
+            const unsigned i = t0 + 4 * tid;
+            uint4 c = make_uint4(0, 0, 0, 0);
+            if (i < hi) c = __ldcg(reinterpret_cast<const uint4*>(table + i));
+            const unsigned pre = block_prefix(c.x + c.y + c.z + c.w, run, warp_sum);
+            if (i < hi)
+                *reinterpret_cast<uint4*>(table + i) = make_uint4(pre, pre + c.x, pre + c.x + c.y, pre + c.x + c.y + c.z);
+        }
+        if (hi == nb && lo < nb && tid == 0) table[nb] = nb;
+    }
+    if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+    // place
+    for (long long i0 = gt; i0 < n; i0 += kBatch * stride) {
+        int2 m[kBatch];
+        unsigned p[kBatch], at[kBatch], b[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const long long i = min(i0 + u * stride, n - 1);
+            m[u] = __ldcg(in.meta + i);
+            p[u] = __ldcg(in.path + i);
+            at[u] = __ldcg(place + i);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) b[u] = bucket_of(load_root(roots + __ldg(root_prefix + m[u].y) + m[u].x), p[u]);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) at[u] += __ldcg(table + min(b[u], (unsigned)n));
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (i0 + u * stride < n && at[u] < (unsigned)n) {
+                slot_path[at[u]] = p[u];
+                slot_src[at[u]] = (unsigned)(i0 + u * stride);
+            }
+    }
+    if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+    // rank
+    constexpr int kRank = 2;
+    const bool ties = *(volatile unsigned long long*)cw(ctrl, kMaxDepth) >= 32;   // paths beyond 32 splits: by place
+    for (long long i0 = gt; i0 < n; i0 += kRank * stride) {
+        unsigned src[kRank], p[kRank], b[kRank];
+        int2 m[kRank];
+        float4 rg[kRank];
+#pragma unroll
+        for (int u = 0; u < kRank; ++u) src[u] = min(__ldcg(slot_src + min(i0 + u * stride, n - 1)), (unsigned)n - 1);
+#pragma unroll
+        for (int u = 0; u < kRank; ++u) {
+            m[u] = __ldcg(in.meta + src[u]);
+            p[u] = __ldcg(in.path + src[u]);
+            rg[u] = __ldcg(in.range + src[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kRank; ++u)
+            b[u] = min(bucket_of(load_root(roots + __ldg(root_prefix + m[u].y) + m[u].x), p[u]), (unsigned)n - 1);
+#pragma unroll
+        for (int u = 0; u < kRank; ++u) {
+            if (i0 + u * stride >= n) break;
+            const unsigned start = __ldcg(table + b[u]), end = min(__ldcg(table + b[u] + 1), (unsigned)n);
+            unsigned to = start;
+            if (end - start > 1) {
+                to += count_below(slot_path, start, end, p[u]);
+                if (ties)
+                    for (unsigned j = start; j < (unsigned)(i0 + u * stride); ++j) to += slot_path[j] == p[u];
+            }
+            if (to < (unsigned)n && (long long)to < out.capacity) {
+                out.range[to] = rg[u];
+                out.meta[to] = m[u];
+            }
+        }
+    }
+    return 1;
+}
+
 // The whole sort in one launch of a resident grid (see the file header).
-// A tile's start in digit bin d is the bin's start plus the counts of the
-// earlier tiles, read as the sums of whole groups of kSortGroup tiles
-// (accumulated as tiles publish) and the single counts of its own group's
-// earlier tiles.
 __global__ void __launch_bounds__(kSortBlock, 2) sort_kernel(const int* __restrict__ root_prefix, SubPatches in,
                                                              SubPatches out, SortBuffers sb, unsigned long long* ctrl,
                                                              int n_passes, long long spin_limit) {
@@ -362,29 +598,30 @@ __global__ void __launch_bounds__(kSortBlock, 2) sort_kernel(const int* __restri
     __shared__ int s_flag;
     const int tid = threadIdx.x, lane = tid & 31;
     const long long n = sort_count(ctrl, in, sb);
-    const unsigned epoch = frame_epoch(ctrl);
     unsigned D = 0;
     const int bits = key_bits(ctrl, &D);
+    // the working blocks: enough for a sub-patch and a root per thread, at most
+    // the grid; the others return at once and every barrier counts the working
+    // blocks only
+    const long long R = (long long)*(volatile unsigned long long*)cw(ctrl, kRoots);
+    const long long want = ((n > R ? n : R) + kSortBlock - 1) / kSortBlock;
+    const int nblk = (int)(want < 1 ? 1 : want < gridDim.x ? want : gridDim.x);
+    if ((int)blockIdx.x >= nblk || n == 0) return;
+    unsigned long long barrier = 0;
+    if (bucket_sort(root_prefix, in, out, sb, ctrl, n, nblk, barrier, spin_limit, sm.warp_sum, &s_flag) != 0) return;
+    // radix passes: a table and counters of zeros first
     const int active = (bits + 7) / 8 < n_passes ? (bits + 7) / 8 : n_passes;
-    unsigned* hist = hist_of(sb, epoch);
-    // the working blocks: one per tile of this frame's keys, at most the
-    // grid (a small frame leaves most of the resident grid idle); the others
-    // return at once and every barrier counts the working blocks only
-    const long long tiles = (n + kSortTile - 1) / kSortTile;
-    const int nblk = (int)(tiles < 1 ? 1 : tiles < gridDim.x ? tiles : gridDim.x);
-    if ((int)blockIdx.x >= nblk) return;
+    unsigned* hist = sb.hist;
     {
-        // counts: of this block's stripe of keys into shared memory (the
-        // front of the pass buffers), then into the frame's table; the next
-        // frame's table, the group counts and the passes' published-tile
-        // counters are cleared for later
-        unsigned* s_hist = reinterpret_cast<unsigned*>(smem_raw);
-        for (int i = tid; i < kSortPasses * kDigits; i += kSortBlock) s_hist[i] = 0;
-        unsigned* next = hist_of(sb, epoch + 1);
         const long long gt = (long long)blockIdx.x * kSortBlock + tid, gstride = (long long)nblk * kSortBlock;
-        for (long long i = gt; i < kSortPasses * kDigits; i += gstride) next[i] = 0;
+        for (long long i = gt; i < kSortPasses * kDigits; i += gstride) hist[i] = 0;
         for (long long i = gt; i < kSortPasses * sb.groups * kDigits; i += gstride) sb.group_counts[i] = 0;
         if (blockIdx.x == 0 && tid < kSortPasses) ctrl[(kSortTicket + tid) * kCtrlStride] = 0;
+        if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, &s_flag)) return;
+        // counts: of this block's stripe of keys into shared memory (the
+        // front of the pass buffers), then into the frame's table
+        unsigned* s_hist = reinterpret_cast<unsigned*>(smem_raw);
+        for (int i = tid; i < kSortPasses * kDigits; i += kSortBlock) s_hist[i] = 0;
         __syncthreads();
         const unsigned lt = (1u << lane) - 1u;
         // whole warps step together so that the warp matches below see every lane
@@ -408,7 +645,6 @@ __global__ void __launch_bounds__(kSortBlock, 2) sort_kernel(const int* __restri
             if (v) atomicAdd(hist + i, v);
         }
     }
-    unsigned long long barrier = 0;
     if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, &s_flag)) return;
     // plan: a pass moves keys unless one digit holds them all
     int moving = 0;
@@ -480,8 +716,8 @@ int canonical_sort_grid() {
 void launch_canonical_sort(const int* root_prefix, const SubPatches& in, const SubPatches& out, const SortBuffers& sb,
                            unsigned long long* ctrl, long long spin_limit, int n_passes, int resident_grid,
                            cudaStream_t s) {
-    const long long tiles = sb.tiles < 1 ? 1 : sb.tiles;
-    const int grid = (int)(tiles < resident_grid ? tiles : resident_grid);
+    const long long want = (sb.capacity + kSortBlock - 1) / kSortBlock;
+    const int grid = (int)(want < 1 ? 1 : want < resident_grid ? want : resident_grid);
     sort_kernel<<<grid, kSortBlock, sizeof(PassSmem), s>>>(root_prefix, in, out, sb, ctrl, n_passes, spin_limit);
 }
 
