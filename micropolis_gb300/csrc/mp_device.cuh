@@ -483,6 +483,32 @@ __device__ __forceinline__ float2 sin2_small(float x, float y) {
                        __uint_as_float(__float_as_uint(sn.y) ^ (__float_as_uint(km.y) << 31)));
 }
 
+// Sine and cosine together, for the adjoint: sin_small's reduction and sine,
+// and beside it, as the other half of the same packed chain, the even Taylor
+// polynomial of degree 12 (the next term is below 7e-9 on |r| <= pi/2).
+__device__ __forceinline__ float2 sincos_small(float x) {
+    const float km = fadd(fmul(x, 0x1.45f306p-2f), kRintMagic);
+    const float k = fsub(km, kRintMagic);
+    float r = ffma(k, -0x1.921fb6p+1f, x);
+    r = ffma(k, 0x1.777a5cp-24f, r);
+    r = ffma(k, 0x1.ee59dap-49f, r);
+    const float r2 = fmul(r, r);
+    float2 p = ffma2(dup2(r2), make_float2(0x1.612462p-33f, 0x1.1eed8ep-29f),
+                     make_float2(-0x1.ae6456p-26f, -0x1.27e4fcp-22f));
+    p = ffma2(dup2(r2), p, make_float2(0x1.71de3ap-19f, 0x1.a01a02p-16f));
+    p = ffma2(dup2(r2), p, make_float2(-0x1.a01a02p-13f, -0x1.6c16c2p-10f));
+    p = ffma2(dup2(r2), p, make_float2(0x1.111112p-7f, 0x1.555556p-5f));
+    p = ffma2(dup2(r2), p, make_float2(-0x1.555556p-3f, -0x1.0p-1f));
+    const float2 sc = ffma2(make_float2(fmul(r, r2), r2), p, make_float2(r, 1.0f));
+    const unsigned flip = __float_as_uint(km) << 31;
+    return make_float2(__uint_as_float(__float_as_uint(sc.x) ^ flip), __uint_as_float(__float_as_uint(sc.y) ^ flip));
+}
+// Whether every argument of the displacement of an eye position stays in the
+// range of the _small functions.
+__device__ __forceinline__ bool displace_is_small(float4 pos, const float* fd) {
+    return fadd(fadd(fabsf(pos.x), fabsf(pos.y)), fadd(fadd(fabsf(fd[0]), fabsf(fd[1])), fabsf(fd[2]))) < 262144.0f;
+}
+
 // kernels/dice.cl:51-67 -- eye-space displacement, updated coordinates used
 // immediately; fd are the three amplitudes.  The twelve sines form seven
 // dependent steps: sin(k x), sin(6 x) need the same x, and sin(k y) of one
@@ -490,8 +516,7 @@ __device__ __forceinline__ float2 sin2_small(float x, float y) {
 // packed pair.  Positions whose arguments could leave sin2_small's range
 // (more than 2^18 from the eye's axes, or not finite) take the general sine.
 __device__ __forceinline__ float4 displace(float4 pos, const float* fd) {
-    const float reach = fadd(fadd(fabsf(pos.x), fabsf(pos.y)), fadd(fadd(fabsf(fd[0]), fabsf(fd[1])), fabsf(fd[2])));
-    if (!(reach < 262144.0f)) {
+    if (!displace_is_small(pos, fd)) {
 #pragma unroll 1
         for (int i = 0; i < 3; ++i) {
             const float k = i == 0 ? 5.0f : i == 1 ? 7.0f : 11.0f, f = i == 0 ? fd[0] : i == 1 ? fd[1] : fd[2];
