@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev
     // draw constants staged in shared memory when they fit
     __shared__ DrawDev s_draws[kBnsSmemDraws];
     extern __shared__ __align__(16) float s_bns[];
+    stamp_start(ctrl, 1);
     // the last frame's entries of the sort's bucket table (whole uint4s), while the first ranges are on their way
     const unsigned n_clear = __ldg(used) / 4;
     for (unsigned i = blockIdx.x * kBnsBlock + threadIdx.x; i < n_clear; i += gridDim.x * kBnsBlock)

@@ -37,6 +37,18 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// Stage k of a batched frame starts: its kernel's first block notes the time.
+// (An event between every two kernels of the frame's graph cost 28 us a
+// frame, 19 % of the 8x8 heightfield's; the timer ticks every 32 ns.)
+__device__ __forceinline__ void stamp_start(unsigned long long* ctrl, int k) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *cw(ctrl, kStamp + k) = global_ns();
+}
+
 // The per-frame reset of the bound-and-split control words: every root
 // outstanding, counters cleared, the frame epoch advanced.
 __device__ __forceinline__ void bns_reset(unsigned long long* ctrl, long long roots) {
@@ -56,6 +68,7 @@ __device__ __forceinline__ void bns_reset(unsigned long long* ctrl, long long ro
     *cw(ctrl, kMaxDepth) = 0;
     *cw(ctrl, kSortDone) = 0;
     *cw(ctrl, kSortMost) = 0;
+    *cw(ctrl, kStampEnd) = 0;
 }
 
 __device__ __forceinline__ void set_status(unsigned long long* ctrl, int code) {

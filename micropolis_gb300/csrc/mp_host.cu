@@ -296,27 +296,29 @@ mp_status ensure_mshade(mp_ctx* c) {
     return MP_OK;
 }
 
+size_t draw_bytes(int cap) { return sizeof(DrawDev) * (size_t)cap + sizeof(int) * (size_t)(cap + 1); }
+
 mp_status ensure_draws(mp_ctx* c, int n) {
     if (n <= c->draws_cap) return MP_OK;
     c->graph_stale = true;
     int cap = std::max(n, std::max(4, c->draws_cap * 2));
     // earlier draws of a plain frame may still be read by queued kernels: keep them
     CK(cudaStreamSynchronize(c->stream));
+    // the root prefixes follow the draws: one copy uploads both
     DrawDev* nd = nullptr;
-    CK(dalloc(&nd, cap));
+    CK(cudaMalloc((void**)&nd, draw_bytes(cap)));
     if (c->d_draws && c->draws_cap > 0)
         CK(cudaMemcpy(nd, c->d_draws, sizeof(DrawDev) * (size_t)c->draws_cap, cudaMemcpyDeviceToDevice));
     cudaFree(c->d_draws);
-    cudaFree(c->d_root_prefix);
     cudaFreeHost(c->h_draws);
-    cudaFreeHost(c->h_root_prefix);
     c->d_draws = nd;
-    c->d_root_prefix = nullptr;
+    c->d_root_prefix = reinterpret_cast<int*>(nd + cap);
     c->h_draws = nullptr;
     c->h_root_prefix = nullptr;
-    CK(dalloc(&c->d_root_prefix, cap + 1));
-    CK(cudaMallocHost((void**)&c->h_draws, sizeof(DrawDev) * (size_t)cap));
-    CK(cudaMallocHost((void**)&c->h_root_prefix, sizeof(int) * (size_t)(cap + 1)));
+    c->draws_cap = 0;
+    CK(cudaMallocHost((void**)&c->h_draws, draw_bytes(cap)));
+    std::memset((void*)c->h_draws, 0, draw_bytes(cap));
+    c->h_root_prefix = reinterpret_cast<int*>(c->h_draws + cap);
     c->draws_cap = cap;
     return MP_OK;
 }
@@ -520,24 +522,18 @@ constexpr int kBatchedStages = 6;
 constexpr StageMark kStageMarks[kBatchedStages] = {{0, "clear framebuffer"}, {1, "bound & split"}, {5, "accumulate"},
                                                    {2, "dice"},              {3, "sample"},        {4, "shade"}};
 
-// Event sev[k] marks the end of stage k - 1 (sev[0] the start).  Inside a
-// stream capture the record becomes an event node of the graph.
+// With stage timing on, event sev[k] marks the end of stage k - 1 (sev[0]
+// the start); the graph's kernels note their own start times (kStamp).
 void mark(mp_ctx* c, int k, bool capturing) {
-    if (capturing)
-        cudaEventRecordWithFlags(c->sev[k], c->stream, cudaEventRecordExternal);
-    else
-        cudaEventRecord(c->sev[k], c->stream);
+    if (!capturing) cudaEventRecord(c->sev[k], c->stream);
 }
 
 // The device work of one batched frame, from the upload of the draw
-// constants to the read-back of the control words, with an event after each
-// stage: bound-and-split, canonical order and rasterization as separate
+// constants to the read-back of the control words: bound-and-split, canonical order and rasterization as separate
 // launches, or (option `overlap`) bound-and-split and rasterization as one
 // overlapped launch over the list in emission order.
 void enqueue_frame(mp_ctx* c, int n, long long roots, bool capturing) {
-    cudaMemcpyAsync(c->d_draws, c->h_draws, sizeof(DrawDev) * (size_t)n, cudaMemcpyHostToDevice, c->stream);
-    cudaMemcpyAsync(c->d_root_prefix, c->h_root_prefix, sizeof(int) * (size_t)(n + 1), cudaMemcpyHostToDevice,
-                    c->stream);
+    cudaMemcpyAsync(c->d_draws, c->h_draws, draw_bytes(c->draws_cap), cudaMemcpyHostToDevice, c->stream);
     mark(c, 0, capturing);
     launch_clear(c->fb, c->fr, 0, c->stream, c->ctrl, roots, overlapped(c) ? nullptr : c->root_info);
     mark(c, 1, capturing);
@@ -559,23 +555,30 @@ void enqueue_frame(mp_ctx* c, int n, long long roots, bool capturing) {
     mark(c, 4, capturing);
     launch_raster_big(c->d_draws, c->fr, c->fb, c->big, c->big_cap, c->ctrl, c->stream);
     mark(c, 5, capturing);
-    launch_resolve(c->d_draws, c->fr, final_list(c), c->fb, c->mshade, c->stream);
+    launch_resolve(c->d_draws, c->fr, final_list(c), c->fb, c->mshade, c->ctrl, c->stream);
     mark(c, 6, capturing);
     cudaMemcpyAsync(c->h_ctrl, c->ctrl, sizeof(unsigned long long) * kNumCtrl * kCtrlStride, cudaMemcpyDeviceToHost,
                     c->stream);
 }
 
-// Stage times and trace lines of the last batched frame (its events have completed).
-void read_stage_events(mp_ctx* c) {
+// Stage times and trace lines of the last batched frame (it has completed).
+void read_stage_times(mp_ctx* c) {
     c->trace.clear();
     for (double& v : c->stats.stage_ms) v = 0;
     float t = 0;
     for (int k = 0; k < kBatchedStages; ++k) {
+        const bool merged = overlapped(c) && (k == 1 || k == 2);   // part of the overlapped launch
         float ms = 0;
-        if (cudaEventElapsedTime(&ms, c->sev[k], c->sev[k + 1]) != cudaSuccess) ms = 0;
+        if (c->stage_timing) {
+            if (cudaEventElapsedTime(&ms, c->sev[k], c->sev[k + 1]) != cudaSuccess) ms = 0;
+        } else if (!merged) {
+            int next = k + 1;
+            while (overlapped(c) && (next == 1 || next == 2)) ++next;
+            const unsigned long long t0 = hc(c, kStamp + k), t1 = hc(c, kStamp + next);
+            ms = t1 > t0 ? (float)((double)(t1 - t0) * 1e-6) : 0.0f;
+        }
         c->stats.stage_ms[kStageMarks[k].slot] = ms;
-        if (!(overlapped(c) && (k == 1 || k == 2)))
-            c->trace.push_back({kStageMarks[k].name, (long long)(t * 1e6), (long long)((t + ms) * 1e6)});
+        if (!merged) c->trace.push_back({kStageMarks[k].name, (long long)(t * 1e6), (long long)((t + ms) * 1e6)});
         t += ms;
     }
     cudaGetLastError();
@@ -649,7 +652,7 @@ mp_status batched_frame(mp_ctx* c) {
             CK(cudaEventRecord(c->ev1, c->stream));
             CK(cudaStreamSynchronize(c->stream));
         }
-        read_stage_events(c);
+        read_stage_times(c);
         unsigned long long status = hc(c, kStatus);
         if (status != kErrOverflow) {
             if (status) return check_status(c, status);
@@ -866,9 +869,7 @@ void mp_destroy(mp_ctx* c) {
     if (c->staging) cudaFreeHost(c->staging);
     dfree(c->xyz_dev);
     dfree(c->d_draws);
-    dfree(c->d_root_prefix);
     if (c->h_draws) cudaFreeHost(c->h_draws);
-    if (c->h_root_prefix) cudaFreeHost(c->h_root_prefix);
     dfree(c->q.words); dfree(c->q.seq);
     dfree(c->sub.range); dfree(c->sub.meta); dfree(c->sub.seq); dfree(c->sub.path);
     free_sorted(c);

@@ -32,6 +32,8 @@ enum CtrlWord {
     kSortTicket,       // tile tickets of the canonical sort, one word per radix pass (kSortPasses)
     kSortDone = kSortTicket + 8,   // grid-barrier arrivals of the sort kernel this frame
     kSortMost,         // keys of the fullest bucket of the canonical sort, when it is too full
+    kStamp,            // start of each stage of a batched frame and the end of the last, ns (kStamps words)
+    kStampEnd = kStamp + 6,
     kNumCtrl
 };
 constexpr int kCtrlStride = 16;  // unsigned long long words per line
@@ -162,7 +164,7 @@ int frame_kernel_grid(int PS, int group);
 void launch_raster_big(const DrawDev* draws, const FrameDev& fr, const Framebuffer& fb, const BigQuad* big,
                        long long big_cap, unsigned long long* ctrl, cudaStream_t s);
 void launch_resolve(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
-                    const float* mshade, cudaStream_t s);
+                    const float* mshade, unsigned long long* ctrl, cudaStream_t s);
 // plain per-pass path
 void launch_dice_grid(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, long long base, int count,
                       float4* pos, int2* pxl, float* depth, cudaStream_t s);

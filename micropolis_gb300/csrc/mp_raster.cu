@@ -606,6 +606,7 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     load_amplitude(fr);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
+    stamp_start(ctrl, 3);
     // an earlier stage of the frame failed (the host reports it): the list
     // may be incomplete, so nothing is rasterized
     if (*(volatile unsigned long long*)cw(ctrl, kStatus) != 0) return;
@@ -659,6 +660,7 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     constexpr size_t kPtsOffset = kFramePtsOffset;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ long long s_group;
+    stamp_start(ctrl, 3);
     if ((int)blockIdx.x < n_bns_ctas) {
         // draw constants staged in the (not yet used) raster buffer
         DrawDev* sd = reinterpret_cast<DrawDev*>(smem_raw);
@@ -735,6 +737,7 @@ __global__ void __launch_bounds__(kBigThreads) raster_big_kernel(FrameDev fr, Fr
     __shared__ short s_x[kBigMaxAxis], s_y[kBigMaxAxis];
     __shared__ int s_nx, s_ny;
     __shared__ int s_frags;
+    stamp_start(ctrl, 4);
     long long n = (long long)*(volatile unsigned long long*)cw(ctrl, kBigCount);
     if (n > big_cap) n = big_cap;
     const int maxl = (8 << fr.shift) - 1;
@@ -798,6 +801,7 @@ __global__ void clear_kernel(Framebuffer fb, FrameDev fr, int with_color, unsign
                              long long roots, RootInfo* root_info) {
     // the frame's bound-and-split reset rides along (one thread)
     if (reset_ctrl && blockIdx.x == 0 && threadIdx.x == 0) bns_reset(reset_ctrl, roots);
+    if (reset_ctrl) stamp_start(reset_ctrl, 0);
     const long long nk = fb.key_pixels * fb.views, n = fb.pixels * fb.views;
     const float4 cc = make_float4(fr.clear[0], fr.clear[1], fr.clear[2], fr.clear[3]);
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -831,7 +835,8 @@ __device__ __forceinline__ unsigned long long key_of(const FrameDev& fr, const F
 constexpr int kResolvePixels = 4;
 template <int PS>
 __global__ void resolve_kernel(const DrawDev* __restrict__ draws, FrameDev fr, SubPatches sub, Framebuffer fb,
-                               const float* __restrict__ mshade) {
+                               const float* __restrict__ mshade, unsigned long long* ctrl) {
+    stamp_start(ctrl, 5);
     const long long n = fb.pixels * fb.views;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kResolvePixels * stride) {
@@ -866,6 +871,7 @@ __global__ void resolve_kernel(const DrawDev* __restrict__ draws, FrameDev fr, S
             }
         }
     }
+    if (threadIdx.x == 0) atomicMax(cw(ctrl, kStampEnd), global_ns());
 }
 
 // ---------------------------------------------------------------------------
@@ -1151,12 +1157,12 @@ void launch_raster_big(const DrawDev*, const FrameDev& fr, const Framebuffer& fb
 }
 
 void launch_resolve(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
-                    const float* mshade, cudaStream_t s) {
+                    const float* mshade, unsigned long long* ctrl, cudaStream_t s) {
     int g = grid_for((fb.pixels * fb.views + kResolvePixels - 1) / kResolvePixels, 256);
     if (fr.PS == 16)
-        resolve_kernel<16><<<g, 256, 0, s>>>(draws, fr, sub, fb, mshade);
+        resolve_kernel<16><<<g, 256, 0, s>>>(draws, fr, sub, fb, mshade, ctrl);
     else
-        resolve_kernel<8><<<g, 256, 0, s>>>(draws, fr, sub, fb, mshade);
+        resolve_kernel<8><<<g, 256, 0, s>>>(draws, fr, sub, fb, mshade, ctrl);
 }
 
 void launch_dice_grid(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, long long base, int count,

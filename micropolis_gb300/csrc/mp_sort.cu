@@ -596,6 +596,7 @@ __global__ void __launch_bounds__(kSortBlock, 2) sort_kernel(const int* __restri
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PassSmem& sm = *reinterpret_cast<PassSmem*>(smem_raw);
     __shared__ int s_flag;
+    stamp_start(ctrl, 2);
     const int tid = threadIdx.x, lane = tid & 31;
     const long long n = sort_count(ctrl, in, sb);
     unsigned D = 0;
