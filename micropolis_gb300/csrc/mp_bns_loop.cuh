@@ -13,6 +13,14 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -23,13 +31,6 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 }
 __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-// A release fence followed by relaxed stores: each store publishes every
-// write this thread made before the fence (the PTX release pattern), so two
-// flags need one fence.
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ void st_relaxed_u32(unsigned* p, unsigned v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
@@ -89,8 +90,14 @@ constexpr unsigned long long kLow32 = 0xffffffffull;
 //   word 31      patch id | split direction << 31 (1: x halved), GPU criterion
 //   word 32      draw | parent's depth << 24
 //   word 33      the parent's split path
-// Bundles of the global queue hold kBundlePairs pairs with the same words,
-// word w of pair p at kBundlePairs * w + p, then the number of pairs.
+// Bundles of the global queue hold up to kBundlePairs pairs with the same
+// words, word w of pair p at kBundlePairs * w + p, and the number of pairs in
+// the last one.  Every word carries the frame's epoch in its upper half, so a
+// reader knows each word valid by itself and neither side needs a fence: a
+// gpu-scope acquire empties the SM's L1 of the patches its other warps work
+// on and made the receiver's next loads wait some 5,000 cycles.  (The count of
+// unfinished units needs none either: a giver still holds a unit of its own
+// when it adds the bundle's, and its own updates of one word stay in order.)
 constexpr int kPairWords = 34;
 constexpr int kStackPairs = 64;        // ring size of the standalone kernel
 constexpr int kStackPairsFrame = 32;   // and of the overlapped kernel, whose blocks also hold the raster's buffers
@@ -171,7 +178,9 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
             roots_left = root < root_end;
         }
         if (n == 0 && root >= root_end) {
-            // out of work: report, then wait (bounded) for a bundle
+            // out of work: report, then wait (bounded) for a bundle: first for
+            // its pair count, then for its words, each valid once it carries
+            // this frame's epoch
             long long slot = warp - busy;
             int got = 0;
             if (lane == 0) {
@@ -184,9 +193,12 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
                 long long idle = 0;
                 unsigned sleep_ns = 32;
                 while (true) {
-                    if (slot < q.capacity && ld_acquire_u32(q.seq + slot) == epoch) {
-                        got = 1;
-                        break;
+                    if (slot < q.capacity) {
+                        const unsigned long long v = ld_relaxed_u64(q.words + slot * kBundleWords + kBundleWords - 1);
+                        if ((unsigned)(v >> 32) == epoch) {
+                            got = (int)(unsigned)v;
+                            break;
+                        }
                     }
                     if (*(volatile unsigned long long*)cw(ctrl, kDone)) break;
                     if (++idle > spin_limit) {
@@ -198,17 +210,33 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
                     if (sleep_ns < 512) sleep_ns <<= 1;
                 }
             }
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) break;
+            n = __shfl_sync(0xffffffffu, got, 0);
+            if (n == 0) break;
             slot = __shfl_sync(0xffffffffu, slot, 0);
             first_ticket = false;
             units = 1;
             splits = 0;
-            const unsigned* rec = q.words + slot * kBundleWords;
-            n = (int)__ldcg(rec + kPairWords * kBundlePairs);
             bottom = 0;
-            for (int i = lane; i < kPairWords * kBundlePairs; i += 32)
-                ring[(i / kBundlePairs) * S + (i % kBundlePairs)] = __uint_as_float(__ldcg(rec + i));
+            const unsigned long long* rec = q.words + slot * kBundleWords;
+            long long tries = 0;
+            bool valid;
+            do {
+                valid = true;
+                for (int i = lane; i < kPairWords * kBundlePairs; i += 32)
+                    if (i % kBundlePairs < n) {
+                        const unsigned long long v = ld_relaxed_u64(rec + i);
+                        valid = valid && (unsigned)(v >> 32) == epoch;
+                        ring[(i / kBundlePairs) * S + (i % kBundlePairs)] = __uint_as_float((unsigned)v);
+                    }
+                valid = __all_sync(0xffffffffu, valid);
+            } while (!valid && ++tries <= spin_limit);
+            if (!valid) {
+                if (lane == 0) {
+                    set_status(ctrl, kErrTimeout);
+                    st_release_u64(cw(ctrl, kDone), 1ull);
+                }
+                break;
+            }
             __syncwarp();
         }
         // this step's ranges: pairs from the top of the ring, then roots
@@ -403,18 +431,13 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
             }
             slot = __shfl_sync(0xffffffffu, slot, 0);
             if ((long long)slot < q.capacity) {
-                unsigned* rec = q.words + slot * kBundleWords;
+                unsigned long long* rec = q.words + slot * kBundleWords;
+                const unsigned long long tag = (unsigned long long)epoch << 32;
                 for (int i = lane; i < kPairWords * kBundlePairs; i += 32)
                     if (i % kBundlePairs < give)
-                        rec[i] = __float_as_uint(
-                            ring[(i / kBundlePairs) * S + wrap(bottom + i % kBundlePairs)]);
-                if (lane == 0) rec[kPairWords * kBundlePairs] = (unsigned)give;
-                __syncwarp();
-                if (lane == 0) {
-                    // release: the pairs and the outstanding count are visible before the slot's epoch
-                    fence_acq_rel_gpu();
-                    st_relaxed_u32(q.seq + slot, epoch);
-                }
+                        st_relaxed_u64(rec + i, tag | __float_as_uint(ring[(i / kBundlePairs) * S +
+                                                                           wrap(bottom + i % kBundlePairs)]));
+                if (lane == 0) st_relaxed_u64(rec + kBundleWords - 1, tag | (unsigned)give);
             } else if (n > kFull) {
                 set_status(ctrl, kErrOverflow);   // no room: the pairs are lost, the host grows the queue
             } else {

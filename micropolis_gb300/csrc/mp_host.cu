@@ -197,11 +197,9 @@ mp_status grow_queue(mp_ctx* c, long long need) {
     c->graph_stale = true;
     long long cap = std::max(need, c->q.capacity * 2);
     cudaFree(c->q.words);
-    cudaFree(c->q.seq);
     c->q = Queue{};
     CK(dalloc(&c->q.words, cap * kBundleWords));
-    CK(dalloc(&c->q.seq, cap));
-    CK(cudaMemsetAsync(c->q.seq, 0, sizeof(unsigned) * (size_t)cap, c->stream));
+    CK(cudaMemsetAsync(c->q.words, 0, sizeof(unsigned long long) * kBundleWords * (size_t)cap, c->stream));
     c->q.capacity = cap;
     return MP_OK;
 }
@@ -870,7 +868,7 @@ void mp_destroy(mp_ctx* c) {
     dfree(c->xyz_dev);
     dfree(c->d_draws);
     if (c->h_draws) cudaFreeHost(c->h_draws);
-    dfree(c->q.words); dfree(c->q.seq);
+    dfree(c->q.words);
     dfree(c->sub.range); dfree(c->sub.meta); dfree(c->sub.seq); dfree(c->sub.path);
     free_sorted(c);
     dfree(c->root_info);
@@ -1189,7 +1187,7 @@ mp_status mp_dump_stats(mp_ctx* c, char* buf, size_t cap) {
         long long bytes;
     } mem[] = {
         {"control points", cp},
-        {"work queue", c->q.capacity * (long long)((kBundleWords + 1) * sizeof(unsigned))},
+        {"work queue", c->q.capacity * (long long)(kBundleWords * sizeof(unsigned long long))},
         {"sub-patch list", c->sub.capacity * (long long)(sizeof(float4) + sizeof(int2) + 2 * sizeof(unsigned))},
         {"canonical sub-patch list", c->sorted.capacity * (long long)(sizeof(float4) + sizeof(int2))},
         {"canonical order sort", c->sb.capacity * 2 * (long long)(sizeof(unsigned long long) + sizeof(unsigned)) +

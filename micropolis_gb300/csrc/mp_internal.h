@@ -41,10 +41,9 @@ constexpr int kCtrlStride = 16;  // unsigned long long words per line
 // Bound-and-split queue: bundles of up to kBundlePairs split pairs that warps
 // hand to each other (word layout: mp_bns_loop.cuh).
 constexpr int kBundlePairs = 8;
-constexpr int kBundleWords = 288;   // 34 words per pair, the pair count, padding to 128 bytes
+constexpr int kBundleWords = 288;   // 34 words per pair, padding to 128 bytes, the pair count
 struct Queue {
-    unsigned* words;        // kBundleWords per bundle
-    unsigned* seq;          // epoch of the frame that filled the bundle
+    unsigned long long* words;   // kBundleWords per bundle, the epoch of the frame that wrote each above its value
     long long capacity;     // bundles
 };
 
