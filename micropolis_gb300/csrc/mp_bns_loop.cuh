@@ -136,12 +136,14 @@ constexpr size_t bns_smem() {
 //   a step of ten ranges takes a third of the time of a full one and lanes
 //   do not diverge by split direction;
 //   each lane bounds its range's nine points.
+// With the GPU criterion all nine samples of every range are dealt.
 template <int CRIT, int C>
 __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* __restrict__ root_prefix, int n_draws,
                                               const FrameDev& fr, const Queue& q, const SubPatches& out,
                                               unsigned* out_seq, RootInfo* roots, unsigned long long* ctrl,
                                               long long spin_limit,
                                               float* smem, int warp, int n_warps) {
+    static_assert(stack_stride<C>() > C + 32 && kPairWords > 27 && C >= 32, "scratch columns");
     static_assert(C >= 32, "a step adds up to 16 pairs, or 32 to an empty ring");
     // Pairs are given to waiting warps when more than kGiveAbove are left, and
     // kKeep stay (a step of 16 ranges: on 1,024 Gregory patches bound-and-split
@@ -340,8 +342,49 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
                     }
                 dec = bns_decide_points(draws[draw], fr, pts, depth);
             }
-        } else if (active) {
-            dec = bns_decide<CRIT>(draws[draw], fr, pid, r, depth);
+        } else {
+            // nine samples of five words each, word w of sample k of lane l's
+            // range: pairs keep no samples under this criterion, so words past
+            // the scratch column's rows go to the unused rows of the ring
+            auto word = [&](int l, int k, int w) {
+                const int j = 5 * k + w;
+                return j < 27 ? j * S + C + l : (j - 27) * S + l;
+            };
+            const int n_t = 9 * (2 * pop + n_root);
+#pragma unroll 1
+            for (int t0 = 0; t0 < n_t; t0 += 32) {
+                const int t = t0 + lane, q = (t / 9) & 31, k = t % 9;   // sample k of lane q's range
+                const float4 rq = make_float4(__shfl_sync(0xffffffffu, r.x, q), __shfl_sync(0xffffffffu, r.y, q),
+                                              __shfl_sync(0xffffffffu, r.z, q), __shfl_sync(0xffffffffu, r.w, q));
+                const int pq = __shfl_sync(0xffffffffu, pid, q), dq = __shfl_sync(0xffffffffu, draw, q);
+                if (t < n_t) {
+                    const GpuSample g = gpu_sample(draws[dq], pq, rq, k / 3, k % 3);
+                    ring[word(q, k, 0)] = g.x;
+                    ring[word(q, k, 1)] = g.y;
+                    ring[word(q, k, 2)] = g.z;
+                    ring[word(q, k, 3)] = g.s.x;
+                    ring[word(q, k, 4)] = g.s.y;
+                }
+            }
+            __syncwarp();
+            if (active) {
+                dec = kCull;
+                if (depth < fr.max_depth - 1) {
+                    GpuBound b;
+                    b.clear();
+#pragma unroll
+                    for (int u = 0; u < 3; ++u) {
+                        GpuSample c[3];
+#pragma unroll
+                        for (int v = 0; v < 3; ++v)
+                            c[v] = GpuSample{ring[word(lane, 3 * u + v, 0)], ring[word(lane, 3 * u + v, 1)],
+                                             ring[word(lane, 3 * u + v, 2)],
+                                             make_float2(ring[word(lane, 3 * u + v, 3)], ring[word(lane, 3 * u + v, 4)])};
+                        b.add(c, u == 0);
+                    }
+                    dec = b.decide(draws[draw], fr, r);
+                }
+            }
         }
         root += n_root;
         // emitted sub-patches: slots from one atomic, whose round trip the pushes below overlap

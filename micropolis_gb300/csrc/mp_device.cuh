@@ -840,72 +840,97 @@ __device__ __forceinline__ long long key_index(const FrameDev& fr, int x, int y)
 }
 
 // The reference's GPU bound criterion (kernels/bound_n_split.h:8-100), in the
-// kernel arithmetic (R1-R6).  The nine screen positions pp[v][u] are consumed
-// as they are produced: the sum along u of row v and the sum along v of
-// column u accumulate in the reference's order, so only the previous column
-// is kept.
-__device__ __forceinline__ int bns_decide_gpu(const DrawDev& d, const FrameDev& fr, int pid, float4 r, int depth) {
-    if (depth >= fr.max_depth - 1) return kCull;
-    const float inf = __int_as_float(0x7f800000);
-    float mnx = inf, mny = inf, mnz = inf, mxx = -inf, mxy = -inf, mxz = -inf;
-    float2 prev[3];                                  // pp[v][u - 1]
-    float hsum[3] = {0.0f, 0.0f, 0.0f};              // along u, per row v
-    float vlen = 0.0f;
+// kernel arithmetic (R1-R6): nine samples (u, v), each an eye position and a
+// screen position.
+struct GpuSample {
+    float x, y, z;   // eye
+    float2 s;        // screen
+};
+__device__ __forceinline__ GpuSample gpu_sample(const DrawDev& d, int pid, float4 r, int u, int v) {
+    // uv = mix(rmin, rmax, (u, v) * (1 / (RES - 1)))
     const float4* P = d.cp + (size_t)pid * (d.type == 0 ? 16 : 20);
-#pragma unroll 1
-    for (int u = 0; u < 3; ++u) {
-        float vsum = 0.0f;                           // along v, column u
-        float2 above = make_float2(0.0f, 0.0f);      // pp[v - 1][u]
+    const float tx = ffma(fsub(r.z, r.x), fmul((float)u, 0.5f), r.x);
+    const float ty = ffma(fsub(r.w, r.y), fmul((float)v, 0.5f), r.y);
+    const float4 o = d.type == 0 ? eval_bezier_dice(P, tx, ty) : eval_gregory_dice(P, tx, ty);
+    const float4 p = mul_m44v4(d.mv, o);
+    const float4 q = mul_m44v4(d.proj, p);
+    const float rw = frcp(q.w);
+    const float x = fmul(q.x, rw), y = fmul(q.y, rw);
+    // mul_cm2v2(screen_matrix = diag(vp), (x, y)): m0 * x + m1 * y per component
+    return GpuSample{p.x, p.y, p.z, make_float2(ffma(0.0f, y, fmul(d.vpx, x)), ffma(d.vpy, y, fmul(0.0f, x)))};
+}
+// The running sums over the samples, taken with u outer and v inner: the sum
+// along u of row v and the sum along v of column u accumulate in the
+// reference's order, so only the previous column is kept.
+struct GpuBound {
+    float mnx, mny, mnz, mxx, mxy, mxz;
+    float2 prev[3];   // pp[v][u - 1]
+    float hsum[3];    // along u, per row v
+    float vlen;
+    __device__ __forceinline__ void clear() {
+        const float inf = __int_as_float(0x7f800000);
+        mnx = mny = mnz = inf;
+        mxx = mxy = mxz = -inf;
+        hsum[0] = hsum[1] = hsum[2] = 0.0f;
+        vlen = 0.0f;
+    }
+    // column u (c[v] its samples)
+    __device__ __forceinline__ void add(const GpuSample (&c)[3], bool first) {
+        float vsum = 0.0f;   // along v, column u
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            // uv = mix(rmin, rmax, (u, v) * (1 / (RES - 1)))
-            const float tx = ffma(fsub(r.z, r.x), fmul((float)u, 0.5f), r.x);
-            const float ty = ffma(fsub(r.w, r.y), fmul((float)v, 0.5f), r.y);
-            const float4 o = d.type == 0 ? eval_bezier_dice(P, tx, ty) : eval_gregory_dice(P, tx, ty);
-            const float4 p = mul_m44v4(d.mv, o);
-            mnx = fminf(mnx, p.x); mny = fminf(mny, p.y); mnz = fminf(mnz, p.z);
-            mxx = fmaxf(mxx, p.x); mxy = fmaxf(mxy, p.y); mxz = fmaxf(mxz, p.z);
-            const float4 q = mul_m44v4(d.proj, p);
-            const float rw = frcp(q.w);
-            const float x = fmul(q.x, rw), y = fmul(q.y, rw);
-            // mul_cm2v2(screen_matrix = diag(vp), (x, y)): m0 * x + m1 * y per component
-            const float2 s = make_float2(ffma(0.0f, y, fmul(d.vpx, x)), ffma(d.vpy, y, fmul(0.0f, x)));
+            mnx = fminf(mnx, c[v].x); mny = fminf(mny, c[v].y); mnz = fminf(mnz, c[v].z);
+            mxx = fmaxf(mxx, c[v].x); mxy = fmaxf(mxy, c[v].y); mxz = fmaxf(mxz, c[v].z);
             // distance(a, b) = sqrt(dot(a - b, a - b)), R1: fma(dx, dx, dy*dy)
             if (v > 0) {
-                const float dx = fsub(above.x, s.x), dy = fsub(above.y, s.y);
+                const float dx = fsub(c[v - 1].s.x, c[v].s.x), dy = fsub(c[v - 1].s.y, c[v].s.y);
                 vsum = fadd(vsum, __fsqrt_rn(ffma(dx, dx, fmul(dy, dy))));
             }
-            if (u > 0) {
-                const float dx = fsub(prev[v].x, s.x), dy = fsub(prev[v].y, s.y);
+            if (!first) {
+                const float dx = fsub(prev[v].x, c[v].s.x), dy = fsub(prev[v].y, c[v].s.y);
                 hsum[v] = fadd(hsum[v], __fsqrt_rn(ffma(dx, dx, fmul(dy, dy))));
             }
-            above = s;
-            prev[v] = s;
+            prev[v] = c[v].s;
         }
         vlen = fmaxf(vsum, vlen);
     }
-    // outside_frustum (kernels/bound_n_split.h:8-30)
-    float n = -mxz;
-    const float f = -mnz;
-    if (f < d.near_plane || n > 1000.0f) return kCull;
-    n = fmaxf(d.near_plane, n);
-    // `x / n * f.x + screen_size.x * 0.5`: the 0.5 is a double literal, so the
-    // product is rounded to float before a double addition of W/2, which is
-    // exact, then rounded to float: one float multiply and one float add.
-    const float sminx = fadd(fmul(kdiv(mnx, mnx < 0 ? n : f), d.fx), d.vpx);
-    const float sminy = fadd(fmul(kdiv(mny, mny < 0 ? n : f), d.fy), d.vpy);
-    const float smaxx = fadd(fmul(kdiv(mxx, mxx > 0 ? n : f), d.fx), d.vpx);
-    const float smaxy = fadd(fmul(kdiv(mxy, mxy > 0 ? n : f), d.fy), d.vpy);
-    if (sminx > fadd((float)(d.vx - 1), d.cull_ribbon) || smaxx < -d.cull_ribbon ||
-        sminy > fadd((float)(d.vy - 1), d.cull_ribbon) || smaxy < -d.cull_ribbon)
-        return kCull;
-    // straddles the eye plane: split the shorter parametric side (VSPLIT halves x)
-    if (mnz < d.near_eps && mxz > d.near_plane) return fsub(r.z, r.x) < fsub(r.w, r.y) ? kSplitX : kSplitY;
-    float hlen = 0.0f;
+    __device__ __forceinline__ int decide(const DrawDev& d, const FrameDev& fr, float4 r) const {
+        // outside_frustum (kernels/bound_n_split.h:8-30)
+        float n = -mxz;
+        const float f = -mnz;
+        if (f < d.near_plane || n > 1000.0f) return kCull;
+        n = fmaxf(d.near_plane, n);
+        // `x / n * f.x + screen_size.x * 0.5`: the 0.5 is a double literal, so the
+        // product is rounded to float before a double addition of W/2, which is
+        // exact, then rounded to float: one float multiply and one float add.
+        const float sminx = fadd(fmul(kdiv(mnx, mnx < 0 ? n : f), d.fx), d.vpx);
+        const float sminy = fadd(fmul(kdiv(mny, mny < 0 ? n : f), d.fy), d.vpy);
+        const float smaxx = fadd(fmul(kdiv(mxx, mxx > 0 ? n : f), d.fx), d.vpx);
+        const float smaxy = fadd(fmul(kdiv(mxy, mxy > 0 ? n : f), d.fy), d.vpy);
+        if (sminx > fadd((float)(d.vx - 1), d.cull_ribbon) || smaxx < -d.cull_ribbon ||
+            sminy > fadd((float)(d.vy - 1), d.cull_ribbon) || smaxy < -d.cull_ribbon)
+            return kCull;
+        // straddles the eye plane: split the shorter parametric side (VSPLIT halves x)
+        if (mnz < d.near_eps && mxz > d.near_plane) return fsub(r.z, r.x) < fsub(r.w, r.y) ? kSplitX : kSplitY;
+        float hlen = 0.0f;
 #pragma unroll
-    for (int v = 0; v < 3; ++v) hlen = fmaxf(hsum[v], hlen);
-    if (hlen <= fr.limit && vlen <= fr.limit) return kDraw;
-    return hlen > vlen ? kSplitX : kSplitY;
+        for (int v = 0; v < 3; ++v) hlen = fmaxf(hsum[v], hlen);
+        if (hlen <= fr.limit && vlen <= fr.limit) return kDraw;
+        return hlen > vlen ? kSplitX : kSplitY;
+    }
+};
+__device__ __forceinline__ int bns_decide_gpu(const DrawDev& d, const FrameDev& fr, int pid, float4 r, int depth) {
+    if (depth >= fr.max_depth - 1) return kCull;
+    GpuBound b;
+    b.clear();
+#pragma unroll 1
+    for (int u = 0; u < 3; ++u) {
+        GpuSample c[3];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) c[v] = gpu_sample(d, pid, r, u, v);
+        b.add(c, u == 0);
+    }
+    return b.decide(d, fr, r);
 }
 
 // ---------------------------------------------------------------------------
