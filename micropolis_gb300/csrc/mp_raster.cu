@@ -2,7 +2,7 @@
 //
 // Batched path: raster_fused dices groups of sub-patches into shared memory
 // (a block per group, the group's control points and matrices staged with
-// cp.async while the previous group is processed), applies the
+// bulk copies while the previous group is processed), applies the
 // reference's per-8x8-block rules (a block with a vertex at eye z == 0 is
 // dropped, kernels/reyes.cl:130-162; the block bound over front-facing quads
 // and its is_empty test of kernels/reyes.cl:287) and rasterizes every quad
@@ -181,8 +181,8 @@ __device__ __forceinline__ void push_big(BigQuad* big, long long big_cap, unsign
 // (27 runs a sub-patch at PS = 8), then the quads in strips of 8 of one
 // column (8 strips a sub-patch), then one thread per quad that can touch a
 // pixel.  The inputs of the next group (sub-patch records, control points,
-// matrices) are copied into the other half of a double buffer with cp.async
-// while the current group is diced and rasterized.
+// matrices) are copied into the other half of a double buffer with bulk
+// copies, one per sub-patch, while the current group is diced and rasterized.
 //
 // Instruction issue and the latency of short chains bound the kernel (no
 // pipe is above 40 %, DRAM at 2 %).  Runs of 3 vertices load each control
@@ -196,7 +196,10 @@ __device__ __forceinline__ void push_big(BigQuad* big, long long big_cap, unsign
 // in 6 blocks of 128) -> 1.42 ms; groups of 13: 1.47, of 9: 1.57, of 11 in
 // 160 threads: 1.61, of 7 in 64: 1.59, of 18 in 256: 1.55, of 12 in 6 blocks
 // (80 registers, spills): 1.61.  At 16x16 dicing 5.63 -> 4.56 ms (groups of
-// 5; 4: 4.74, 6 in 256 threads: 4.92).
+// 5; 4: 4.74, 6 in 256 threads: 4.92).  Bulk copies by the lanes of one warp
+// instead of a 16-byte copy per thread and point, and the registers freed by
+// 32-bit list positions and the light in shared memory (no spills):
+// 1.41 -> 1.36 ms, 64 views 5.14 -> 4.90 ms.
 constexpr int kRun = 3;
 template <int NS>
 constexpr int fused_threads() {
@@ -230,6 +233,8 @@ template <int PS, int NS_>
 struct FusedSmem {
     static constexpr int NS = NS_, G = PS + 1, NV = G * G;
     GroupStage<NS> st[2];
+    unsigned long long full[2];   // mbarriers: the copies into st[b] have arrived
+    V3 light;                     // light_dir(), here because the dice needs every register
     // per group state, double-buffered with st: blocks with a vertex at eye
     // z == 0, and the number of listed quads
     unsigned zero[2][NS];
@@ -241,61 +246,60 @@ struct FusedSmem {
     int2 pxy[NS * NV];        // fixed-point pixel coordinates
 };
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    const size_t ga = __cvta_generic_to_global(gmem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(ga) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    const size_t ga = __cvta_generic_to_global(gmem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(ga) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-// Stores the records of a group's n sub-patches, one per thread of warp 0
-// (n <= 32), and numbers their runs of equal draws; called by whole warps.
+// Starts a copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
+// that completes on the mbarrier.
+__device__ __forceinline__ void bulk_copy(void* smem, const void* gmem, unsigned bytes, unsigned long long* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(smem)),
+                 "l"(__cvta_generic_to_global(gmem)), "r"(bytes), "r"(smem_addr(bar))
+                 : "memory");
+}
+// Waits (bounded) for the mbarrier's phase; false when the wait ran out.
+__device__ __forceinline__ bool bulk_wait(unsigned long long* bar, unsigned parity) {
+    for (int tries = 0; tries < (1 << 20); ++tries) {
+        unsigned done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(smem_addr(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// Stores the records of a group's n sub-patches, one per lane of warp 0 (its
+// callers), numbers their runs of equal draws, and starts the copies of their
+// control points (one per sub-patch) and of the runs' matrices.
 template <int NS>
-__device__ __forceinline__ void store_records(GroupStage<NS>& st, int n, float4 range, int2 meta) {
+__device__ __forceinline__ void stage_inputs(GroupStage<NS>& st, unsigned long long* full, int n, float4 range, int2 meta,
+                                             const DrawDev* __restrict__ draws) {
     static_assert(NS <= 32, "one record per lane of warp 0");
-    const int tid = threadIdx.x;
-    if (tid >= 32) return;
+    const int lane = threadIdx.x;
     const int before = __shfl_up_sync(0xffffffffu, meta.y, 1);
-    const unsigned starts = __ballot_sync(0xffffffffu, tid > 0 && tid < n && meta.y != before);
-    if (tid < n) {
-        st.range[tid] = range;
-        st.meta[tid] = meta;
-        st.run[tid] = __popc(starts & (lanemask_lt() | (1u << tid)));
+    const bool starts = lane > 0 && lane < n && meta.y != before;
+    const int run = __popc(__ballot_sync(0xffffffffu, starts) & (lanemask_lt() | (1u << lane)));
+    const bool copies_matrices = lane < n && run < kMatrixRuns && (lane == 0 || starts);
+    unsigned bytes = 0;
+    const DrawDev* d = draws + meta.y;
+    if (lane < n) {
+        const int type = d->type;
+        bytes = type == 0 ? 16 * sizeof(float4) : 20 * sizeof(float4);
+        st.range[lane] = range;
+        st.meta[lane] = meta;
+        st.run[lane] = run;
+        st.tv[lane][0] = type;
+        st.tv[lane][1] = d->view;
     }
-}
-
-// Copies, for the n sub-patches whose records are already in st, their
-// control points, matrices, type and view (asynchronous; the caller waits).
-template <int NS>
-__device__ __forceinline__ void stage_inputs(GroupStage<NS>& st, int n, const DrawDev* __restrict__ draws) {
-    for (int i = threadIdx.x; i < n * 24; i += fused_threads<NS>()) {
-        const int k = i / 24, c = i % 24;
-        const int2 m = st.meta[k];
-        const DrawDev* d = draws + m.y;
-        if (c < 20) {
-            const int ncp = d->type == 0 ? 16 : 20;
-            if (c < ncp) cp_async16(&st.cp[k][c], d->cp + (size_t)m.x * ncp + c);
-        } else if (c == 20) {
-            cp_async4(&st.tv[k][0], &d->type);
-        } else if (c == 21) {
-            cp_async4(&st.tv[k][1], &d->view);
-        } else {
-            // the run's first sub-patch copies its matrices, 64 bytes per lane
-            const int run = st.run[k];
-            if (run < kMatrixRuns && (k == 0 || st.run[k - 1] != run)) {
-                const int at = (c - 22) * 16;
-#pragma unroll
-                for (int j = 0; j < 16; j += 4) cp_async16(&st.mvp[run][at + j], d->mv + at + j);
-            }
-        }
-    }
-    cp_async_commit();
+    const unsigned total = __reduce_add_sync(0xffffffffu, bytes + (copies_matrices ? 32 * (unsigned)sizeof(float) : 0u));
+    if (lane == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(full)), "r"(total)
+                     : "memory");
+    __syncwarp();
+    if (lane < n)
+        bulk_copy(&st.cp[lane][0], reinterpret_cast<const char*>(d->cp) + (size_t)meta.x * bytes, bytes, full);
+    if (copies_matrices) bulk_copy(st.mvp[run], d->mv, 32 * sizeof(float), full);
 }
 
 // Prepares the state of a group of n sub-patches whose records are in
@@ -322,24 +326,44 @@ __device__ __forceinline__ void prepare_group(FusedSmem<PS, NS>& sm, int b, int 
     if (first == 0) sm.n_live[b] = 0;
 }
 
-// Stages the group [base, base + n) into sm.st[0] from scratch (records,
-// then inputs) and prepares it; ends with a barrier.
+// Initializes the mbarriers and the light; ends with a barrier.
 template <int PS, int NS>
-__device__ __forceinline__ void stage_group(FusedSmem<PS, NS>& sm, long long base, int n, const SubPatches& sub,
-                                            const DrawDev* __restrict__ draws, const FrameDev& fr) {
-    GroupStage<NS>& st = sm.st[0];
-    float4 range = make_float4(0.f, 0.f, 0.f, 0.f);
-    int2 meta = make_int2(0, 0);
-    if ((int)threadIdx.x < n) {
-        range = sub.range[base + threadIdx.x];
-        meta = sub.meta[base + threadIdx.x];
+__device__ __forceinline__ void init_stages(FusedSmem<PS, NS>& sm) {
+    if (threadIdx.x == 0) {
+        sm.light = light_dir();
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.full[0])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.full[1])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    store_records(st, n, range, meta);
     __syncthreads();
-    stage_inputs(st, n, draws);
-    prepare_group(sm, 0, n, fr, threadIdx.x);
-    cp_async_wait_all();
+}
+
+// The record of list entry base + lane, for lane < n.
+struct GroupRecord {
+    float4 range;
+    int2 meta;
+};
+__device__ __forceinline__ GroupRecord load_record(const SubPatches& sub, int base, int n) {
+    GroupRecord g{make_float4(0.f, 0.f, 0.f, 0.f), make_int2(0, 0)};
+    if ((int)threadIdx.x < n) {
+        g.range = sub.range[base + threadIdx.x];
+        g.meta = sub.meta[base + threadIdx.x];
+    }
+    return g;
+}
+
+// Stages the group [base, base + n) into sm.st[b] from scratch and prepares
+// it; parity: the phase of its mbarrier.  Ends with a barrier; false when the
+// copies did not arrive.
+template <int PS, int NS>
+__device__ __forceinline__ bool stage_group(FusedSmem<PS, NS>& sm, int b, unsigned parity, int base, int n,
+                                            const SubPatches& sub, const DrawDev* __restrict__ draws,
+                                            const FrameDev& fr) {
+    const GroupRecord g = load_record(sub, base, n);
+    if (threadIdx.x < 32) stage_inputs(sm.st[b], &sm.full[b], n, g.range, g.meta, draws);
     __syncthreads();
+    prepare_group(sm, b, n, fr, threadIdx.x);
+    return __syncthreads_and(bulk_wait(&sm.full[b], parity));
 }
 
 // The 8x8 block bound over front-facing quads (kernels/reyes.cl:120-166) of a
@@ -391,9 +415,9 @@ __device__ __forceinline__ void load_matrices(const float* m, float (&mv)[16], f
 // Dices, shades and rasterizes the n (<= NS) sub-patches at [base, base+n)
 // of the emitted list, whose inputs are staged and prepared in buffer b, with
 // the whole block; meanwhile stages and prepares the n_next sub-patches at
-// next_base in buffer b ^ 1.  Three phases (dice; the list of quads that can
-// touch a pixel; raster), each ending with a barrier after which both groups'
-// buffers are complete.
+// next_base in buffer b ^ 1, next_parity the phase of its mbarrier.  Three phases (dice; the list of quads that can
+// touch a pixel; raster), each ending with a barrier; after the last one the
+// next group's buffer is complete, or the result is false.
 //
 // The 8x8 block bound decides only whether a block is skipped, and the tiles
 // of quads too large for the fast raster.  A small front-facing quad with a
@@ -404,24 +428,23 @@ __device__ __forceinline__ void load_matrices(const float* m, float (&mv)[16], f
 // DISP is the frame's displacement option, compiled in: frames without it
 // carry neither its code nor its registers.
 template <int PS, int NS, bool DISP>
-__device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long long base, int n,
-                                             long long next_base, int n_next, const DrawDev* __restrict__ draws,
-                                             const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
+__device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int base, int n, int next_base, int n_next,
+                                             unsigned next_parity, const DrawDev* __restrict__ draws, const FrameDev& fr,
+                                             const SubPatches& sub, const Framebuffer& fb,
                                              float* __restrict__ mshade, BigQuad* big, long long big_cap,
-                                             unsigned long long* ctrl, const V3& light, long long& frags) {
+                                             unsigned long long* ctrl, int& frags) {
     using SM = FusedSmem<PS, NS>;
     constexpr int G = SM::G, NV = SM::NV, NQ = PS * PS, BPL = PS / 8, TH = fused_threads<NS>();
     GroupStage<NS>& cur = sm.st[b];
     GroupStage<NS>& nxt = sm.st[b ^ 1];
     const int tid = threadIdx.x, lane = tid & 31;
-    // the next group's records travel in registers until this group's
-    // vertices are done
-    float4 next_range = make_float4(0.f, 0.f, 0.f, 0.f);
-    int2 next_meta = make_int2(0, 0);
-    if (tid < n_next) {
-        next_range = sub.range[next_base + tid];
-        next_meta = sub.meta[next_base + tid];
-    }
+    // The next group's records travel in registers until this group's vertices
+    // are done (8x8 dicing; staging them at once costs 0.5-1 % there: warp 0
+    // waits for them); a 16x16 group has 5 and dices longer, and there
+    // staging at once is 0.7 % faster.
+    const GroupRecord next = load_record(sub, next_base, n_next);
+    if (PS == 16 && n_next > 0 && tid < 32)
+        stage_inputs(nxt, &sm.full[b ^ 1], n_next, next.range, next.meta, draws);
     // dice vertices (kernels/dice.cl:37-80): run i of a sub-patch holds the
     // vertices (nu, nv0 .. nv0 + kRun - 1), nu = i % G, nv0 = kRun (i / G)
     constexpr int NR = (G + kRun - 1) / kRun, RPS = G * NR;
@@ -474,9 +497,9 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
             }
         }
     }
-    if (n_next > 0) store_records(nxt, n_next, next_range, next_meta);
+    if (PS != 16 && n_next > 0 && tid < 32)
+        stage_inputs(nxt, &sm.full[b ^ 1], n_next, next.range, next.meta, draws);
     __syncthreads();
-    if (n_next > 0) stage_inputs(nxt, n_next, draws);
     // The list of quads that can touch a pixel: a quad with a large bbox, or a
     // small one with an accepted winding and a pixel centre in its bbox.  A
     // thread walks a strip of 8 quads (column nu, rows 8 h .. 8 h + 7), so
@@ -571,8 +594,7 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
             qy[c] = q.y;
             qd[c] = e[c].w;
         }
-        const long long s = base + k;
-        const unsigned mp_id = (unsigned)(s * NQ + nu + nv * PS);
+        const unsigned mp_id = (unsigned)(base + k) * NQ + nu + nv * PS;
         const int view = cur.tv[k][1];
         unsigned long long* keys = fb.keys + (long long)view * fb.key_pixels;
         int minx, miny, maxx, maxy, f = 0;
@@ -588,13 +610,12 @@ __device__ __forceinline__ void raster_group(FusedSmem<PS, NS>& sm, int b, long 
         if (f > 0 || !fast) {
             // the diffuse factor of a quad that may own pixels; resolve
             // turns it into the colour of kernels/reyes.cl:191
-            mshade[mp_id] = shade_m_l(light, e[0].x, e[0].y, e[0].z, e[1].x, e[1].y, e[1].z, e[2].x, e[2].y, e[2].z,
+            mshade[mp_id] = shade_m_l(sm.light, e[0].x, e[0].y, e[0].z, e[1].x, e[1].y, e[1].z, e[2].x, e[2].y, e[2].z,
                                       e[3].x, e[3].y, e[3].z);
         }
         frags += f;
     }
-    cp_async_wait_all();
-    __syncthreads();
+    return __syncthreads_and(n_next == 0 || bulk_wait(&sm.full[b ^ 1], next_parity));
 }
 
 template <int PS, int NS, bool DISP>
@@ -610,18 +631,20 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     // an earlier stage of the frame failed (the host reports it): the list
     // may be incomplete, so nothing is rasterized
     if (*(volatile unsigned long long*)cw(ctrl, kStatus) != 0) return;
-    long long S = (long long)*(volatile unsigned long long*)cw(ctrl, kOutCount);
-    if (S > sub.capacity) S = sub.capacity;
-    const V3 light = light_dir();
-    long long frags = 0;
-    const long long stride = (long long)gridDim.x * NS;
-    long long base = (long long)blockIdx.x * NS;
-    if (base < S) stage_group(sm, base, (int)min((long long)NS, S - base), sub, draws, fr);
-    for (int b = 0; base < S; base += stride, b ^= 1) {
-        const long long next = base + stride;
-        raster_group<PS, NS, DISP>(sm, b, base, (int)min((long long)NS, S - base), next,
-                             next < S ? (int)min((long long)NS, S - next) : 0, draws, fr, sub, fb, mshade, big,
-                             big_cap, ctrl, light, frags);
+    // (list positions fit 32 bits: micropolygon ids do)
+    const int S = (int)min((long long)*(volatile unsigned long long*)cw(ctrl, kOutCount), sub.capacity);
+    int frags = 0;
+    const int stride = (int)gridDim.x * NS;
+    int base = (int)blockIdx.x * NS;
+    auto count = [&](int at) { return at < S ? min(NS, S - at) : 0; };
+    if (base < S) {
+        init_stages(sm);
+        bool ok = stage_group(sm, 0, 0, base, count(base), sub, draws, fr);
+        for (unsigned it = 0; ok && base < S; ++it, base += stride)
+            ok = raster_group<PS, NS, DISP>(sm, it & 1, base, count(base), base + stride, count(base + stride),
+                                            ((it + 1) >> 1) & 1, draws, fr, sub, fb, mshade, big, big_cap, ctrl, frags);
+        // (a copy that never arrives: the frame reports it, like every wait that runs out)
+        if (!ok && threadIdx.x == 0) set_status(ctrl, kErrTimeout);
     }
     frags = __reduce_add_sync(0xffffffffu, (unsigned)frags);
     if ((threadIdx.x & 31) == 0 && frags) atomicAdd(cw(ctrl, kFragments), (unsigned long long)frags);
@@ -680,8 +703,9 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     }
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
     const unsigned epoch = (unsigned)*(volatile unsigned long long*)cw(ctrl, kEpoch);
-    const V3 light = light_dir();
-    long long frags = 0;
+    int frags = 0;
+    init_stages(sm);
+    unsigned parity = 0;
     while (true) {
         if (threadIdx.x == 0) s_group = (long long)atomicAdd(cw(ctrl, kGroupTicket), 1ull);
         __syncthreads();
@@ -712,13 +736,18 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
         }
         const int n = __syncthreads_count(ready);
         if (n == 0 || __syncthreads_or(gave_up)) break;
-        stage_group(sm, base, n, sub, gdraws, fr);
-        if (fr.displacement)
-            raster_group<PS, NS, true>(sm, 0, base, n, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl, light,
-                                       frags);
-        else
-            raster_group<PS, NS, false>(sm, 0, base, n, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl, light,
-                                        frags);
+        bool ok = stage_group(sm, 0, parity, (int)base, n, sub, gdraws, fr);
+        parity ^= 1;
+        if (ok && fr.displacement)
+            ok = raster_group<PS, NS, true>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
+                                            frags);
+        else if (ok)
+            ok = raster_group<PS, NS, false>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
+                                             frags);
+        if (!ok) {
+            if (threadIdx.x == 0) set_status(ctrl, kErrTimeout);
+            break;
+        }
     }
     frags = __reduce_add_sync(0xffffffffu, (unsigned)frags);
     if ((threadIdx.x & 31) == 0 && frags) atomicAdd(cw(ctrl, kFragments), (unsigned long long)frags);
