@@ -252,6 +252,8 @@ mp_status mp_set_displacement_amplitude(mp_ctx* ctx, float amplitude);
 mp_status mp_set_displacement_amplitude_device(mp_ctx* ctx, const void* amp_dev);
 /* Replaces the control points of a loaded handle in place from device memory (same count). */
 mp_status mp_update_patches_device(mp_ctx* ctx, uint64_t handle, const void* dev_xyz1);
+/* Same from xyz triples in device memory, widened to (x, y, z, 1) on the way. */
+mp_status mp_update_patches_xyz_device(mp_ctx* ctx, uint64_t handle, const void* dev_xyz);
 
 /* Inclusive prefix sum on the device (the decoupled look-back scan used by the
  * plain path; the reference's CL::PrefixSum, src/CL/PrefixSum.cpp:33-80). */

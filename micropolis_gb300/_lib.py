@@ -84,6 +84,7 @@ SIGNATURES = [
     ("mp_read_framebuffer_async", ctypes.c_int, [c_void_p, i32, c_void_p, c_void_p]),
     ("mp_wait_read_framebuffer", ctypes.c_int, [c_void_p]),
     ("mp_update_patches_device", ctypes.c_int, [c_void_p, u64, c_void_p]),
+    ("mp_update_patches_xyz_device", ctypes.c_int, [c_void_p, u64, c_void_p]),
     ("mp_inclusive_scan", ctypes.c_int, [c_void_p, P(i32), P(i32), i64]),
     ("mp_inclusive_scan_noalloc", ctypes.c_int, [c_void_p, c_void_p, i64, c_void_p]),
     ("mp_atomic_bench", ctypes.c_int, [c_void_p, i64, i64, i32, P(ctypes.c_double)]),
@@ -101,6 +102,7 @@ SIGNATURES = [
 ]
 
 _lib = None
+_draw = None
 
 
 def lib():
@@ -117,6 +119,19 @@ def lib():
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+def draw_call():
+    """mp_draw_patches_view taking the matrix and colour as addresses: a frame
+    makes this call once per object, and building two ctypes pointers took
+    half of its time."""
+    global _draw
+    if _draw is None:
+        fn = lib()["mp_draw_patches_view"]
+        fn.restype = ctypes.c_int
+        fn.argtypes = [c_void_p, u64, c_void_p, P(MpProjection), c_void_p, i32]
+        _draw = fn
+    return _draw
 
 
 class MpError(RuntimeError):

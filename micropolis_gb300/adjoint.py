@@ -58,14 +58,21 @@ class DiffRenderer:
         """Tiled RGBA image (W*H, 4) for control points cp (n, per, 3) and
         the displacement amplitude multiplier amp: a tensor on the device
         (read there, no host synchronization) or a number."""
-        xyz1 = torch.cat([cp.detach().float().reshape(-1, 3),
-                          torch.ones(cp.numel() // 3, 1, device=cp.device)], dim=1).contiguous()
+        xyz = cp.detach().float().reshape(-1, 3).contiguous()
+        if len(xyz) < self.n_patches * self.per:
+            raise ValueError("control points of %d patches of %d points expected" % (self.n_patches, self.per))
+        on_gpu = xyz.is_cuda   # widened by the renderer's kernel, else here
+        if not on_gpu:
+            xyz = torch.cat([xyz, torch.ones(len(xyz), 1)], dim=1).contiguous()
         amp_dev = None
         if isinstance(amp, torch.Tensor):
             amp_dev = amp.detach().to(device=cp.device, dtype=torch.float32).reshape(1).contiguous()
         img = torch.empty((self.npx, 4), dtype=torch.float32, device=cp.device)
         cur, side = self._stream_in()
-        self.r.update_patches_device(self.handle, xyz1.data_ptr())
+        if on_gpu:
+            self.r.update_patches_xyz_device(self.handle, xyz.data_ptr())
+        else:
+            self.r.update_patches_device(self.handle, xyz.data_ptr())
         if amp_dev is not None:
             self.r.set_displacement_amplitude_device(amp_dev.data_ptr())
         else:
@@ -74,7 +81,7 @@ class DiffRenderer:
         self.r.draw_patches(self.handle, self.draw.mv, self.proj, self.draw.color)
         self.r.finish()
         self.r.copy_framebuffer_device(0, img.data_ptr())
-        self._stream_out(cur, side, img, xyz1, *([amp_dev] if amp_dev is not None else []))
+        self._stream_out(cur, side, img, xyz, *([amp_dev] if amp_dev is not None else []))
         return img
 
     def backward(self, grad_img: torch.Tensor, cp_shape, device):

@@ -1021,6 +1021,15 @@ mp_status mp_update_patches_device(mp_ctx* c, uint64_t handle, const void* dev_x
     return MP_OK;
 }
 
+mp_status mp_update_patches_xyz_device(mp_ctx* c, uint64_t handle, const void* dev_xyz) {
+    if (!c || !dev_xyz) return MP_ERR_INVALID_ARG;
+    auto it = c->meshes.find(handle);
+    if (it == c->meshes.end()) return fail(c, MP_ERR_NOT_LOADED, "handle not loaded");
+    launch_widen_points((const float*)dev_xyz, it->second.cp, (long long)it->second.n_points, c->stream);
+    CK(cudaGetLastError());
+    return MP_OK;
+}
+
 mp_status mp_delete_patches(mp_ctx* c, uint64_t handle) {
     if (!c) return MP_ERR_INVALID_ARG;
     if (c->in_frame) return fail(c, MP_ERR_STATE, "delete_patches inside a frame");

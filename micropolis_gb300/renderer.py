@@ -123,14 +123,17 @@ class Renderer:
     def update_patches_device(self, handle: int, dev_ptr: int) -> None:
         self._ck(lib().mp_update_patches_device(self._ctx, handle, ctypes.c_void_p(dev_ptr)))
 
+    def update_patches_xyz_device(self, handle: int, dev_ptr: int) -> None:
+        """Replaces a loaded handle's control points from xyz float32 triples in device memory."""
+        self._ck(lib().mp_update_patches_xyz_device(self._ctx, handle, ctypes.c_void_p(dev_ptr)))
+
     def delete_patches(self, handle: int) -> None:
         self._ck(lib().mp_delete_patches(self._ctx, handle))
 
     def draw_patches(self, handle: int, modelview, projection: Projection, color=(1, 1, 1, 1), view: int = 0) -> None:
         mv = np.ascontiguousarray(modelview, np.float32).reshape(16)
         col = np.ascontiguousarray(color, np.float32).reshape(4)
-        p = projection.c()
-        self._ck(lib().mp_draw_patches_view(self._ctx, handle, _f32p(mv), ctypes.byref(p), _f32p(col), view))
+        self._ck(_lib.draw_call()(self._ctx, handle, mv.ctypes.data, projection.c(), col.ctypes.data, view))
 
     def draw_views(self, items) -> None:
         """Many draws in one call: items of (handle, modelview, projection, colour, view)."""
@@ -184,7 +187,7 @@ class Renderer:
 
     def read_image(self, view: int = 0) -> np.ndarray:
         """The displayed image (gamma 1/2.2, 8-bit), (height, width, 3) RGB, top row first."""
-        rgb = np.zeros((self.height, self.width, 3), np.uint8)
+        rgb = np.empty((self.height, self.width, 3), np.uint8)   # (every byte is written)
         self._ck(lib().mp_read_image(self._ctx, view, rgb.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8))))
         return rgb
 
@@ -312,12 +315,12 @@ def render_scene(renderer: Renderer, scene, handles=None) -> None:
     """Scene::draw (src/micropolis/Scene.cpp:179-197): prepare, load on first
     use, draw every object, finish."""
     renderer.prepare()
+    proj = Projection(scene.fovy, scene.near, (scene.width, scene.height))
     for k, d in enumerate(scene.draws):
         h = handles[k] if handles else id(d.mesh)
         if not renderer.are_patches_loaded(h):
             renderer.load_patches(h, d.mesh.cp, d.mesh.type)
-        renderer.draw_patches(h, d.mv, Projection(scene.fovy, scene.near, (scene.width, scene.height)), d.color,
-                              view=d.view)
+        renderer.draw_patches(h, d.mv, proj, d.color, view=d.view)
     renderer.finish()
 
 
