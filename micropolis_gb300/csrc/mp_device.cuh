@@ -68,6 +68,7 @@ struct FrameDev {
     int kshift;            // depth|id key buffer tile: 1 << kshift pixels (8, 16 or 32)
     int kgx;               // key tiles per row
     int criterion;         // mp_bound_criterion
+    float vp[4];           // W << shift, H << shift, and their halves (whole numbers)
 };
 
 // Depth|id key stored per pixel: (idepth << 32) | mp_id.  The clear key keeps
@@ -519,35 +520,59 @@ __device__ __forceinline__ bool displace_is_small(float4 pos, const float* fd) {
 // step and sin(k' y) of the next the same y, so five of the steps evaluate a
 // packed pair.  Positions whose arguments could leave sin2_small's range
 // (more than 2^18 from the eye's axes, or not finite) take the general sine.
-__device__ __forceinline__ float4 displace(float4 pos, const float* fd) {
-    if (!displace_is_small(pos, fd)) {
+static __device__ __noinline__ float4 displace_general(float4 pos, float f0, float f1, float f2) {
 #pragma unroll 1
-        for (int i = 0; i < 3; ++i) {
-            const float k = i == 0 ? 5.0f : i == 1 ? 7.0f : 11.0f, f = i == 0 ? fd[0] : i == 1 ? fd[1] : fd[2];
-            pos.x = ffma(mp_sinf(fmul(fmul(pos.y, k), 2.0f)), f, pos.x);
-            pos.y = ffma(mp_sinf(fmul(fmul(pos.x, k), 2.0f)), f, pos.y);
-            pos.z = ffma(fmul(mp_sinf(fmul(fmul(pos.y, k), 2.0f)), mp_sinf(fmul(fmul(pos.x, 3.0f), 2.0f))), f, pos.z);
-        }
-        return pos;
-    }
-    const float k[3] = {5.0f, 7.0f, 11.0f};
-    float sy = sin_small(fmul(fmul(pos.y, k[0]), 2.0f));
-#pragma unroll
     for (int i = 0; i < 3; ++i) {
-        pos.x = ffma(sy, fd[i], pos.x);
-        const float2 sx = sin2_small(fmul(fmul(pos.x, k[i]), 2.0f), fmul(fmul(pos.x, 3.0f), 2.0f));
-        pos.y = ffma(sx.x, fd[i], pos.y);
-        float sz;
-        if (i < 2) {
-            const float2 s = sin2_small(fmul(fmul(pos.y, k[i]), 2.0f), fmul(fmul(pos.y, k[i < 2 ? i + 1 : 2]), 2.0f));
-            sz = s.x;
-            sy = s.y;
-        } else {
-            sz = sin_small(fmul(fmul(pos.y, k[i]), 2.0f));
-        }
-        pos.z = ffma(fmul(sz, sx.y), fd[i], pos.z);
+        const float k = i == 0 ? 5.0f : i == 1 ? 7.0f : 11.0f, f = i == 0 ? f0 : i == 1 ? f1 : f2;
+        pos.x = ffma(mp_sinf(fmul(fmul(pos.y, k), 2.0f)), f, pos.x);
+        pos.y = ffma(mp_sinf(fmul(fmul(pos.x, k), 2.0f)), f, pos.y);
+        pos.z = ffma(fmul(mp_sinf(fmul(fmul(pos.y, k), 2.0f)), mp_sinf(fmul(fmul(pos.x, 3.0f), 2.0f))), f, pos.z);
     }
     return pos;
+}
+// N positions at once: one test decides for all (the general sine gives the
+// same bits), so that their chains of seven steps run side by side.
+template <int N>
+__device__ __forceinline__ void displace_vertices(float4 (&pos)[N], const float* fd) {
+    bool small = true;
+#pragma unroll
+    for (int n = 0; n < N; ++n) small = small && displace_is_small(pos[n], fd);
+    if (!small) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) pos[n] = displace_general(pos[n], fd[0], fd[1], fd[2]);
+        return;
+    }
+    const float k[3] = {5.0f, 7.0f, 11.0f};
+    float sy[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) sy[n] = sin_small(fmul(fmul(pos[n].y, k[0]), 2.0f));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        float2 sx[N];
+        float sz[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            pos[n].x = ffma(sy[n], fd[i], pos[n].x);
+            sx[n] = sin2_small(fmul(fmul(pos[n].x, k[i]), 2.0f), fmul(fmul(pos[n].x, 3.0f), 2.0f));
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            pos[n].y = ffma(sx[n].x, fd[i], pos[n].y);
+            if (i < 2) {
+                const float2 s = sin2_small(fmul(fmul(pos[n].y, k[i]), 2.0f), fmul(fmul(pos[n].y, k[i < 2 ? i + 1 : 2]), 2.0f));
+                sz[n] = s.x;
+                sy[n] = s.y;
+            } else {
+                sz[n] = sin_small(fmul(fmul(pos[n].y, k[i]), 2.0f));
+            }
+            pos[n].z = ffma(fmul(sz[n], sx[n].y), fd[i], pos[n].z);
+        }
+    }
+}
+__device__ __forceinline__ float4 displace(float4 pos, const float* fd) {
+    float4 p[1] = {pos};
+    displace_vertices<1>(p, fd);
+    return p[0];
 }
 
 // Eye-space position of dice vertex (nu, nv) of a sub-patch (kernels/dice.cl:44-67).
@@ -691,27 +716,38 @@ static __device__ __noinline__ int4 project_vertex_general(float4 pr, int W, int
     project_vertex_m(m, fr, pos, px, py, depth);
     return make_int4(px, py, __float_as_int(depth), 0);
 }
-__device__ __forceinline__ void project_vertex_persp(const float (&pr)[4], const FrameDev& fr, float4 pos, int& px,
-                                                     int& py, float& depth) {
-    const float mag = fadd(fadd(fabsf(pos.x), fabsf(pos.y)), fadd(fabsf(pos.z), fabsf(pos.w)));
-    if (!(mag < __int_as_float(0x7f800000)) || pos.z == 0.0f) {
-        const int4 r = project_vertex_general(make_float4(pr[0], pr[1], pr[2], pr[3]), fr.W, fr.H, fr.shift, pos);
-        px = r.x;
-        py = r.y;
-        depth = __int_as_float(r.z);
+// N vertices at once: one test decides for all (the general product is right
+// for any position), so that their chains run side by side.
+template <int N>
+__device__ __forceinline__ void project_vertices_persp(const float (&pr)[4], const FrameDev& fr, const float4 (&pos)[N],
+                                                       int2 (&px)[N], float (&depth)[N]) {
+    float mag = 0.0f, zs = 1.0f;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        mag = fadd(mag, fadd(fadd(fabsf(pos[n].x), fabsf(pos[n].y)), fadd(fabsf(pos[n].z), fabsf(pos[n].w))));
+        zs = fmul(zs, pos[n].z);
+    }
+    if (!(mag < __int_as_float(0x7f800000)) || zs == 0.0f) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int4 r = project_vertex_general(make_float4(pr[0], pr[1], pr[2], pr[3]), fr.W, fr.H, fr.shift, pos[n]);
+            px[n] = make_int2(r.x, r.y);
+            depth[n] = __int_as_float(r.z);
+        }
         return;
     }
-    const int vsx = fr.W << fr.shift, vsy = fr.H << fr.shift;
-    const float2 pxy = fmul2(make_float2(pr[0], pr[1]), make_float2(pos.x, pos.y));
-    const float pz = ffma(pr[3], pos.w, fmul(pr[2], pos.z));
-    const float rw = frcp(-pos.z);
-    float2 e = fmul2(pxy, dup2(rw));
-    e = fmul2(e, make_float2((float)vsx, (float)vsy));
-    e = fmul2(e, dup2(0.5f));
-    e = fadd2(e, make_float2((float)(vsx / 2), (float)(vsy / 2)));
-    px = __float2int_rz(e.x);
-    py = __float2int_rz(e.y);
-    depth = fmul(pz, rw);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const float2 pxy = fmul2(make_float2(pr[0], pr[1]), make_float2(pos[n].x, pos[n].y));
+        const float pz = ffma(pr[3], pos[n].w, fmul(pr[2], pos[n].z));
+        const float rw = frcp(-pos[n].z);
+        float2 e = fmul2(pxy, dup2(rw));
+        e = fmul2(e, make_float2(fr.vp[0], fr.vp[1]));
+        e = fmul2(e, dup2(0.5f));
+        e = fadd2(e, make_float2(fr.vp[2], fr.vp[3]));
+        px[n] = make_int2(__float2int_rz(e.x), __float2int_rz(e.y));
+        depth[n] = fmul(pz, rw);
+    }
 }
 __device__ __forceinline__ void project_vertex(const DrawDev& d, const FrameDev& fr, float4 pos, int& px, int& py,
                                                float& depth) {

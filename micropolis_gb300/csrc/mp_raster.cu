@@ -199,7 +199,10 @@ __device__ __forceinline__ void push_big(BigQuad* big, long long big_cap, unsign
 // 5; 4: 4.74, 6 in 256 threads: 4.92).  Bulk copies by the lanes of one warp
 // instead of a 16-byte copy per thread and point, and the registers freed by
 // 32-bit list positions and the light in shared memory (no spills):
-// 1.41 -> 1.36 ms, 64 views 5.14 -> 4.90 ms.
+// 1.41 -> 1.36 ms, 64 views 5.14 -> 4.90 ms.  One range test for a run's three
+// projections (and displacements) instead of a branch each, so that their
+// chains run side by side: 1.36 -> 1.34 ms, 4.90 -> 4.82, displaced 512x512
+// heightfield at 3840x2160 3.76 -> 3.51.
 constexpr int kRun = 3;
 template <int NS>
 constexpr int fused_threads() {
@@ -473,14 +476,10 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
 #pragma unroll
         for (int v = 0; v < kRun; ++v)
             pos[v] = mul_m44v4(mv, make_float4(d.xy[v].x, d.xy[v].y, d.zw[v].x, d.zw[v].y));
-        if (DISP) {
-#pragma unroll
-            for (int v = 0; v < kRun; ++v) pos[v] = displace(pos[v], fr.fdisp);
-        }
+        if (DISP) displace_vertices<kRun>(pos, fr.fdisp);
         int2 px[kRun];
         float dep[kRun];
-#pragma unroll
-        for (int v = 0; v < kRun; ++v) project_vertex_persp(pr, fr, pos[v], px[v].x, px[v].y, dep[v]);
+        project_vertices_persp<kRun>(pr, fr, pos, px, dep);
         const int at = k * NV + nv0 * G + nu;
 #pragma unroll
         for (int v = 0; v < kRun; ++v) {
@@ -861,42 +860,52 @@ __device__ __forceinline__ unsigned long long key_of(const FrameDev& fr, const F
 // winning depth (kernels/reyes.cl:389).  Each thread takes kResolvePixels
 // pixels a grid apart and issues their key loads, then their gathers, before
 // any use, so the dependent loads of several pixels are in flight at once.
+// (Views go along the grid's y axis, so pixel indices are 32-bit; with one
+// 64-bit index over all views, its divisions made 64 views 107 us, now 96.)
 constexpr int kResolvePixels = 4;
 template <int PS>
 __global__ void resolve_kernel(const DrawDev* __restrict__ draws, FrameDev fr, SubPatches sub, Framebuffer fb,
                                const float* __restrict__ mshade, unsigned long long* ctrl) {
-    stamp_start(ctrl, 5);
-    const long long n = fb.pixels * fb.views;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kResolvePixels * stride) {
-        unsigned long long key[kResolvePixels];
+    if (blockIdx.y == 0) stamp_start(ctrl, 5);
+    const unsigned n = (unsigned)fb.pixels, stride = gridDim.x * blockDim.x;
+    for (int view = blockIdx.y; view < fb.views; view += gridDim.y) {
+        const unsigned long long* keys = fb.keys + (long long)view * fb.key_pixels;
+        float4* color = fb.color + (long long)view * fb.pixels;
+        int* depth = fb.depth + (long long)view * fb.pixels;
+        for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kResolvePixels * stride) {
+            unsigned long long key[kResolvePixels];
 #pragma unroll
-        for (int u = 0; u < kResolvePixels; ++u) {
-            const long long i = i0 + u * stride;
-            key[u] = i < n ? key_of(fr, fb, i) : kClearKey;
-        }
-        int draw[kResolvePixels];
-        float m[kResolvePixels];
-#pragma unroll
-        for (int u = 0; u < kResolvePixels; ++u) {
-            draw[u] = 0;
-            m[u] = 0.0f;
-            if (key[u] != kClearKey) {
-                const unsigned id = (unsigned)(key[u] & 0xffffffffu);
-                draw[u] = sub.meta[id / (PS * PS)].y;
-                m[u] = mshade[id];
+            for (int u = 0; u < kResolvePixels; ++u) {
+                const unsigned i = i0 + u * stride;
+                key[u] = kClearKey;
+                if (i < n) {
+                    const unsigned t = i >> 6, ty = t / (unsigned)fr.gx, tx = t - ty * (unsigned)fr.gx;
+                    key[u] = keys[key_index(fr, (int)((tx << 3) + (i & 7)), (int)((ty << 3) + ((i >> 3) & 7)))];
+                }
             }
-        }
+            int draw[kResolvePixels];
+            float m[kResolvePixels];
 #pragma unroll
-        for (int u = 0; u < kResolvePixels; ++u) {
-            const long long i = i0 + u * stride;
-            if (i >= n) break;
-            if (key[u] == kClearKey) {
-                fb.color[i] = make_float4(fr.clear[0], fr.clear[1], fr.clear[2], fr.clear[3]);
-                fb.depth[i] = 0x7fffffff;
-            } else {
-                fb.color[i] = shade_color(m[u], draws[draw[u]].color);
-                fb.depth[i] = (int)(key[u] >> 32);
+            for (int u = 0; u < kResolvePixels; ++u) {
+                draw[u] = 0;
+                m[u] = 0.0f;
+                if (key[u] != kClearKey) {
+                    const unsigned id = (unsigned)(key[u] & 0xffffffffu);
+                    draw[u] = sub.meta[id / (PS * PS)].y;
+                    m[u] = mshade[id];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kResolvePixels; ++u) {
+                const unsigned i = i0 + u * stride;
+                if (i >= n) break;
+                if (key[u] == kClearKey) {
+                    color[i] = make_float4(fr.clear[0], fr.clear[1], fr.clear[2], fr.clear[3]);
+                    depth[i] = 0x7fffffff;
+                } else {
+                    color[i] = shade_color(m[u], draws[draw[u]].color);
+                    depth[i] = (int)(key[u] >> 32);
+                }
             }
         }
     }
@@ -1187,7 +1196,8 @@ void launch_raster_big(const DrawDev*, const FrameDev& fr, const Framebuffer& fb
 
 void launch_resolve(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
                     const float* mshade, unsigned long long* ctrl, cudaStream_t s) {
-    int g = grid_for((fb.pixels * fb.views + kResolvePixels - 1) / kResolvePixels, 256);
+    const dim3 g((unsigned)grid_for((fb.pixels + kResolvePixels - 1) / kResolvePixels, 256),
+                 (unsigned)std::min(fb.views, 65535));
     if (fr.PS == 16)
         resolve_kernel<16><<<g, 256, 0, s>>>(draws, fr, sub, fb, mshade, ctrl);
     else
