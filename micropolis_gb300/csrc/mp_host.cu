@@ -243,7 +243,7 @@ mp_status grow_sub(mp_ctx* c, long long need, bool keep) {
     b.groups = (b.tiles + kSortGroup - 1) / kSortGroup;
     c->sb = b;
     for (int k = 0; k < 2; ++k) {
-        CK(dalloc(&c->sb.keys[k], cap));
+        CK(dalloc(&c->sb.keys[k], cap + 4));   // (as bucket starts: one more, in whole uint4s)
         CK(dalloc(&c->sb.vals[k], cap));
     }
     const long long entries = (cap + 7) / 4 * 4;   // and the end, in whole uint4s

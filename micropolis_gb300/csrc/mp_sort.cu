@@ -66,11 +66,15 @@ constexpr unsigned kMaxBucket = 2048;
 // Up to this many entries each block adds up the stretches before its own
 // (32 loads a thread) instead of waiting for every block's sum.
 constexpr unsigned kSumAlone = 16384;
+// Up to this many roots each block keeps all their starts in shared memory (16
+// loads a thread) instead of waiting for them to be written.
+constexpr unsigned kRootsAlone = 8192;
 constexpr int kSortBlock = 512;
 constexpr int kSortWarps = kSortBlock / 32;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortBlock * kSortItems;   // keys per tile
 constexpr int kDigits = 256;
+static_assert(kRootsAlone <= 2 * kSortTile, "the starts take the place of the radix passes' keys");
 
 __device__ __forceinline__ long long sort_count(const unsigned long long* ctrl, const SubPatches& in,
                                                 const SortBuffers& sb) {
@@ -452,7 +456,7 @@ __device__ __forceinline__ bool sum_before(F entry, unsigned total, unsigned lo,
 __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, const SubPatches& in,
                                            const SubPatches& out, const SortBuffers& sb, unsigned long long* ctrl,
                                            long long n, int nblk, unsigned long long& barrier, long long spin_limit,
-                                           unsigned* warp_sum, int* s_flag) {
+                                           unsigned* s_start, unsigned* warp_sum, int* s_flag) {
     constexpr int kBatch = 4;   // sub-patches a thread handles at a time, their loads in flight together
     const int tid = threadIdx.x;
     const long long gt = (long long)blockIdx.x * kSortBlock + tid, stride = (long long)nblk * kSortBlock;
@@ -462,10 +466,22 @@ __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, 
     unsigned* place = sb.vals[0];
     unsigned* slot_path = reinterpret_cast<unsigned*>(sb.keys[0]);
     unsigned* slot_src = sb.vals[1];
+    // the starts replace the counts, but of a short table other blocks still
+    // read the counts when this one writes
+    unsigned* starts = n <= kSumAlone ? reinterpret_cast<unsigned*>(sb.keys[1]) : table;
     // the next frame's bound-and-split clears what this one uses of the table
     if (gt == 0) *sb.used = (unsigned)n + 4;
-    {
-        // roots
+    // roots
+    const bool alone = R <= kRootsAlone;
+    if (alone) {
+        unsigned run = 0;
+        for (unsigned t0 = 0; t0 < R; t0 += kSortBlock) {
+            const unsigned i = t0 + tid;
+            const unsigned pre = block_prefix(i < R ? __ldcg(&roots[i].count) : 0u, run, warp_sum);
+            if (i < R) s_start[i] = pre;
+        }
+        __syncthreads();
+    } else {
         const unsigned per = (R + nblk - 1) / nblk, lo = min(per * blockIdx.x, R), hi = min(lo + per, R);
         unsigned own = 0, run = 0;
         if (R > kSumAlone)
@@ -478,8 +494,15 @@ __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, 
             const unsigned pre = block_prefix(i < hi ? __ldcg(&roots[i].count) : 0u, run, warp_sum);
             if (i < hi) roots[i].start = pre;
         }
+        if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
     }
-    if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+    // a record's bucket
+    auto bucket = [&](int2 m, unsigned path) {
+        const int r = __ldg(root_prefix + m.y) + m.x;
+        RootInfo ri = load_root(roots + r);
+        if (alone) ri.start = s_start[r];
+        return bucket_of(ri, path);
+    };
     // count
     for (long long i0 = gt; i0 < n; i0 += kBatch * stride) {
         int2 m[kBatch];
@@ -491,7 +514,7 @@ __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, 
             p[u] = __ldcg(in.path + i);
         }
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) at[u] = bucket_of(load_root(roots + __ldg(root_prefix + m[u].y) + m[u].x), p[u]);
+        for (int u = 0; u < kBatch; ++u) at[u] = bucket(m[u], p[u]);
 #pragma unroll
         for (int u = 0; u < kBatch; ++u)
             if (i0 + u * stride < n && at[u] < (unsigned)n) at[u] = atomicAdd(table + at[u], 1u);
@@ -515,20 +538,18 @@ __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, 
         if (!sum_before([&](unsigned i) { return __ldcg(table + i); }, nb, lo, own, sb.sums, ctrl, nblk, barrier,
                         spin_limit, warp_sum, s_flag, run))
             return -1;
-        // (short tables: every entry is read before any is written)
-        if (nb <= kSumAlone && !grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
-        if (*(volatile unsigned long long*)cw(ctrl, kSortMost)) return 0;
         for (unsigned t0 = lo; t0 < hi; t0 += 4 * kSortBlock) {
             const unsigned i = t0 + 4 * tid;
             uint4 c = make_uint4(0, 0, 0, 0);
             if (i < hi) c = __ldcg(reinterpret_cast<const uint4*>(table + i));
             const unsigned pre = block_prefix(c.x + c.y + c.z + c.w, run, warp_sum);
             if (i < hi)
-                *reinterpret_cast<uint4*>(table + i) = make_uint4(pre, pre + c.x, pre + c.x + c.y, pre + c.x + c.y + c.z);
+                *reinterpret_cast<uint4*>(starts + i) = make_uint4(pre, pre + c.x, pre + c.x + c.y, pre + c.x + c.y + c.z);
         }
-        if (hi == nb && lo < nb && tid == 0) table[nb] = nb;
+        if (hi == nb && lo < nb && tid == 0) starts[nb] = nb;
     }
     if (!grid_barrier(ctrl, ++barrier, nblk, spin_limit, s_flag)) return -1;
+    if (*(volatile unsigned long long*)cw(ctrl, kSortMost)) return 0;
     // place
     for (long long i0 = gt; i0 < n; i0 += kBatch * stride) {
         int2 m[kBatch];
@@ -541,9 +562,9 @@ __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, 
             at[u] = __ldcg(place + i);
         }
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) b[u] = bucket_of(load_root(roots + __ldg(root_prefix + m[u].y) + m[u].x), p[u]);
+        for (int u = 0; u < kBatch; ++u) b[u] = bucket(m[u], p[u]);
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) at[u] += __ldcg(table + min(b[u], (unsigned)n));
+        for (int u = 0; u < kBatch; ++u) at[u] += __ldcg(starts + min(b[u], (unsigned)n));
 #pragma unroll
         for (int u = 0; u < kBatch; ++u)
             if (i0 + u * stride < n && at[u] < (unsigned)n) {
@@ -568,12 +589,11 @@ __device__ __forceinline__ int bucket_sort(const int* __restrict__ root_prefix, 
             rg[u] = __ldcg(in.range + src[u]);
         }
 #pragma unroll
-        for (int u = 0; u < kRank; ++u)
-            b[u] = min(bucket_of(load_root(roots + __ldg(root_prefix + m[u].y) + m[u].x), p[u]), (unsigned)n - 1);
+        for (int u = 0; u < kRank; ++u) b[u] = min(bucket(m[u], p[u]), (unsigned)n - 1);
 #pragma unroll
         for (int u = 0; u < kRank; ++u) {
             if (i0 + u * stride >= n) break;
-            const unsigned start = __ldcg(table + b[u]), end = min(__ldcg(table + b[u] + 1), (unsigned)n);
+            const unsigned start = __ldcg(starts + b[u]), end = min(__ldcg(starts + b[u] + 1), (unsigned)n);
             unsigned to = start;
             if (end - start > 1) {
                 to += count_below(slot_path, start, end, p[u]);
@@ -609,7 +629,9 @@ __global__ void __launch_bounds__(kSortBlock, 2) sort_kernel(const int* __restri
     const int nblk = (int)(want < 1 ? 1 : want < gridDim.x ? want : gridDim.x);
     if ((int)blockIdx.x >= nblk || n == 0) return;
     unsigned long long barrier = 0;
-    if (bucket_sort(root_prefix, in, out, sb, ctrl, n, nblk, barrier, spin_limit, sm.warp_sum, &s_flag) != 0) return;
+    if (bucket_sort(root_prefix, in, out, sb, ctrl, n, nblk, barrier, spin_limit, reinterpret_cast<unsigned*>(sm.keys),
+                    sm.warp_sum, &s_flag) != 0)
+        return;
     // radix passes: a table and counters of zeros first
     const int active = (bits + 7) / 8 < n_passes ? (bits + 7) / 8 : n_passes;
     unsigned* hist = sb.hist;
