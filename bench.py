@@ -554,7 +554,7 @@ def main():
     # key clear, 8 B key + 16 B colour + 4 B depth per pixel for the resolve.
     cp_alg = sum(d.mesh.n_patches * d.mesh.cp.shape[1] * 12 for d in sc.draws)
     alg = {"dice_raster": cp_alg + S * 20,
-           "bound_split": cp_alg + S * 20 + stats["bounds"] * (28 + 80),
+           "bound_split": cp_alg + S * 20,   # its ranges stay in shared memory
            "resolve_or_shade": W * H * (8 + 16 + 4),
            "clear": W * H * 8,
            "raster_big": 0}

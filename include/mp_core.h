@@ -75,7 +75,7 @@ typedef struct {
     int32_t batch_views;            /* framebuffer layers (independent views) */
     int32_t path;                   /* mp_path */
     /* capacities (elements); 0 = automatic.  They grow on overflow. */
-    int64_t queue_capacity;         /* bound&split work items */
+    int64_t queue_capacity;         /* bound&split ranges that may change warps (batched path) */
     int64_t subpatch_capacity;      /* emitted sub-patches per frame */
     int64_t spin_limit;             /* bounded-wait iterations before MP_ERR_TIMEOUT */
     /* batched path: run bound&split and rasterization in one launch that
@@ -114,7 +114,7 @@ typedef struct {
     int64_t big_quads;              /* quads on the exact slow raster path */
     double gpu_ms;                  /* device time of the last frame (CUDA events) */
     /* per-stage device times of the last frame (batched path: always, from
-     * events inside its graph; plain path: with stage timing on,
+     * start times its kernels note; plain path: with stage timing on,
      * mp_set_stage_timing); stages: 0 clear+reset, 1 bound&split, 2 dice+raster
      * (plain: dice), 3 exact slow raster, 4 resolve (plain: shade), 5 canonical
      * order sort (plain: sample), 6 plain pass resolve, 7 plain host readback gaps */

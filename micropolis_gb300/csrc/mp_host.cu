@@ -109,7 +109,7 @@ struct mp_ctx {
     mp_stats stats{};
     long long plain_bounds = 0, plain_passes = 0, plain_out = 0, plain_kernels = 0;
     long long plain_max_stack = 0;
-    // stage events of the last frame (stage timing on): name, start, end in ns from the frame start
+    // stages of the last frame (plain path: stage timing on): name, start, end in ns from the frame start
     struct TraceEvent {
         const char* name;
         long long start, end;
@@ -508,7 +508,7 @@ void launch_sort(mp_ctx* c) {
 // Stages of a batched frame in launch order: the mp_stats.stage_ms slot
 // and the trace name of each.  Names are the reference's command names,
 // which its tools/trace_summary.py maps: bound-and-split is "bound & split";
-// the canonical-order sort, a radix sort built on prefix sums, takes the
+// the canonical-order sort, built on prefix sums, takes the
 // name of the reference's prefix-sum command, "accumulate" (both count as
 // subdivision there); the fused dice+shade+raster launch is "dice", the
 // exact slow raster "sample", the colour resolve "shade".
@@ -632,7 +632,7 @@ mp_status batched_frame(mp_ctx* c) {
     }
     for (int attempt = 0; attempt < 8; ++attempt) {
         if (c->stage_timing) {
-            // the graph's launches issued one by one (same events)
+            // the graph's launches issued one by one, an event after each
             CK(cudaEventRecord(c->ev0, c->stream));
             enqueue_frame(c, n, roots, false);
             CK(cudaEventRecord(c->ev1, c->stream));

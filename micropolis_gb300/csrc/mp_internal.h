@@ -71,12 +71,13 @@ struct RootInfo {
 static_assert(sizeof(RootInfo) == 16, "read as one uint4");
 
 // Canonical order of a frame's sub-patches: ascending (root, split path),
-// root = the draw's first root + patch id.  Scratch of the radix sort that
+// root = the draw's first root + patch id.  Scratch of the sort that
 // establishes it (mp_sort.cu).
 constexpr int kSortPasses = 8;          // 8-bit digits of the 64-bit key
 struct SortBuffers {
-    unsigned long long* keys[2];        // ping-pong keys
-    unsigned* vals[2];                  // ping-pong source slots
+    // bucket sort: paths by bucket place, bucket starts; radix passes: ping-pong keys
+    unsigned long long* keys[2];
+    unsigned* vals[2];                  // places in the buckets and source slots; ping-pong source slots
     unsigned* table;                    // counts, then starts, of the buckets; zero where not in use
     unsigned* used;                     // entries of the table the last sort used (bound-and-split clears them)
     unsigned* sums;                     // keys in each block's stretch of the table
