@@ -27,7 +27,7 @@ enum CtrlWord {
     kScanTotal,        // packed totals of the last scan (draws | splits << 32)
     kBigOverflow,      // big quads that did not fit
     kBigTotal,         // big quads rasterized over the frame
-    kGroupTicket,      // sub-patch groups claimed by the frame kernel's rasterizers
+    kGroupTicket,      // sub-patch groups claimed by the rasterizing blocks
     kMaxDepth,         // deepest split path of an emitted sub-patch (canonical sort keys)
     kSortTicket,       // tile tickets of the canonical sort, one word per radix pass (kSortPasses)
     kSortDone = kSortTicket + 8,   // grid-barrier arrivals of the sort kernel this frame

@@ -242,6 +242,7 @@ struct FusedSmem {
     // z == 0, and the number of listed quads
     unsigned zero[2][NS];
     unsigned n_live[2];
+    unsigned claimed;         // the group after the next one (raster_fused_kernel)
     unsigned short live[NS * PS * PS];   // quads that may touch a pixel
     float tx[NS][G], ty[NS][G];
     float4 vw[NS][G], cw[NS][G];
@@ -420,7 +421,8 @@ __device__ __forceinline__ void load_matrices(const float* m, float (&mv)[16], f
 // the whole block; meanwhile stages and prepares the n_next sub-patches at
 // next_base in buffer b ^ 1, next_parity the phase of its mbarrier.  Three phases (dice; the list of quads that can
 // touch a pixel; raster), each ending with a barrier; after the last one the
-// next group's buffer is complete, or the result is false.
+// next group's buffer is complete, or the result is false.  tickets, if not
+// null, counts claimed groups: one is claimed into sm.claimed.
 //
 // The 8x8 block bound decides only whether a block is skipped, and the tiles
 // of quads too large for the fast raster.  A small front-facing quad with a
@@ -435,7 +437,7 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
                                              unsigned next_parity, const DrawDev* __restrict__ draws, const FrameDev& fr,
                                              const SubPatches& sub, const Framebuffer& fb,
                                              float* __restrict__ mshade, BigQuad* big, long long big_cap,
-                                             unsigned long long* ctrl, int& frags) {
+                                             unsigned long long* ctrl, unsigned long long* tickets, int& frags) {
     using SM = FusedSmem<PS, NS>;
     constexpr int G = SM::G, NV = SM::NV, NQ = PS * PS, BPL = PS / 8, TH = fused_threads<NS>();
     GroupStage<NS>& cur = sm.st[b];
@@ -499,6 +501,8 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
     if (PS != 16 && n_next > 0 && tid < 32)
         stage_inputs(nxt, &sm.full[b ^ 1], n_next, next.range, next.meta, draws);
     __syncthreads();
+    unsigned claimed = 0;
+    if (tickets && tid == 0) claimed = (unsigned)atomicAdd(tickets, 1ull);   // used after the list
     // The list of quads that can touch a pixel: a quad with a large bbox, or a
     // small one with an accepted winding and a pixel centre in its bbox.  A
     // thread walks a strip of 8 quads (column nu, rows 8 h .. 8 h + 7), so
@@ -573,6 +577,7 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
     // the next group's weights and state, from the highest thread down (the
     // raster below occupies the lowest threads)
     prepare_group(sm, b ^ 1, n_next, fr, TH - 1 - tid);
+    if (tickets && tid == 0) sm.claimed = claimed;
     // rasterize the listed quads of live blocks
     const int n_live = (int)sm.n_live[b];
     for (int j = tid; j < n_live; j += TH) {
@@ -633,15 +638,24 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     // (list positions fit 32 bits: micropolygon ids do)
     const int S = (int)min((long long)*(volatile unsigned long long*)cw(ctrl, kOutCount), sub.capacity);
     int frags = 0;
-    const int stride = (int)gridDim.x * NS;
-    int base = (int)blockIdx.x * NS;
+    // The first two groups of a block are its own, the others claimed two
+    // ahead (thread 0 counts them between the dice and the raster, when its
+    // warp has nothing to wait for): groups differ in their patch type, matrix
+    // runs and covered quads, and with a fixed share of them the last block
+    // ended some 10 % after the average one.  Dice+raster: mixed 4096 patches
+    // 1.34 -> 1.23 ms, at 16x16 dicing 4.45 -> 4.04, 64 views 4.82 -> 4.40,
+    // displaced 512x512 heightfield at 3840x2160 3.51 -> 3.12.
+    int base = (int)blockIdx.x * NS, next = base + (int)gridDim.x * NS;
     auto count = [&](int at) { return at < S ? min(NS, S - at) : 0; };
     if (base < S) {
         init_stages(sm);
         bool ok = stage_group(sm, 0, 0, base, count(base), sub, draws, fr);
-        for (unsigned it = 0; ok && base < S; ++it, base += stride)
-            ok = raster_group<PS, NS, DISP>(sm, it & 1, base, count(base), base + stride, count(base + stride),
-                                            ((it + 1) >> 1) & 1, draws, fr, sub, fb, mshade, big, big_cap, ctrl, frags);
+        for (unsigned it = 0; ok && base < S; ++it) {
+            ok = raster_group<PS, NS, DISP>(sm, it & 1, base, count(base), next, count(next), ((it + 1) >> 1) & 1, draws,
+                                            fr, sub, fb, mshade, big, big_cap, ctrl, cw(ctrl, kGroupTicket), frags);
+            base = next;
+            next = (2 * (int)gridDim.x + (int)sm.claimed) * NS;
+        }
         // (a copy that never arrives: the frame reports it, like every wait that runs out)
         if (!ok && threadIdx.x == 0) set_status(ctrl, kErrTimeout);
     }
@@ -739,10 +753,10 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
         parity ^= 1;
         if (ok && fr.displacement)
             ok = raster_group<PS, NS, true>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
-                                            frags);
+                                            nullptr, frags);
         else if (ok)
             ok = raster_group<PS, NS, false>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
-                                             frags);
+                                             nullptr, frags);
         if (!ok) {
             if (threadIdx.x == 0) set_status(ctrl, kErrTimeout);
             break;
