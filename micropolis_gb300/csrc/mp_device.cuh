@@ -620,22 +620,29 @@ struct DiceColumn {
             zw[n] = ffma2(w, make_float2(c.z, c.w), zw[n]);
         }
     }
-    // adds each vertex's face point (a A + b_n B) / den_n, NaN zeroed (blend4)
+    // adds each vertex's face point (a A + b_n B) / den_n, NaN zeroed (blend4);
+    // EXACT false: only the NaN of 0 / 0 (a and b_n are 0 there), and any other
+    // NaN makes the sum one
+    template <bool EXACT>
     __device__ __forceinline__ void add_face(float vw, const float (&cw)[N], float a, float4 A, const float (&b)[N],
                                              float4 B, const float (&den)[N]) {
         const float2 axy = fmul2(dup2(a), make_float2(A.x, A.y)), azw = fmul2(dup2(a), make_float2(A.z, A.w));
 #pragma unroll
         for (int n = 0; n < N; ++n) {
-            const float2 r = dup2(frcp(den[n])), b2 = dup2(b[n]), w = fmul2(dup2(vw), dup2(cw[n]));
+            float rd = frcp(den[n]);
+            if (!EXACT && a == 0.0f && den[n] == 0.0f) rd = 0.0f;
+            const float2 r = dup2(rd), b2 = dup2(b[n]), w = fmul2(dup2(vw), dup2(cw[n]));
             const float2 fxy = fmul2(ffma2(b2, make_float2(B.x, B.y), axy), r);
             const float2 fzw = fmul2(ffma2(b2, make_float2(B.z, B.w), azw), r);
-            xy[n] = ffma2(w, make_float2(sel_nan(fxy.x), sel_nan(fxy.y)), xy[n]);
-            zw[n] = ffma2(w, make_float2(sel_nan(fzw.x), sel_nan(fzw.y)), zw[n]);
+            xy[n] = ffma2(w, EXACT ? make_float2(sel_nan(fxy.x), sel_nan(fxy.y)) : fxy, xy[n]);
+            zw[n] = ffma2(w, EXACT ? make_float2(sel_nan(fzw.x), sel_nan(fzw.y)) : fzw, zw[n]);
         }
     }
 };
 
-template <int N>
+// EXACT false: the same unless the result is not finite; sixteen selects a
+// Gregory vertex less.
+template <int N, bool EXACT>
 __device__ __forceinline__ void dice_column(DiceColumn<N>& d, int type, const float4* P, float tx,
                                             const float (&ty)[N], float4 vw, const float4 (&cw)[N]) {
     float c[4][N];
@@ -670,12 +677,12 @@ __device__ __forceinline__ void dice_column(DiceColumn<N>& d, int type, const fl
     d.add(v[0], c[2], P[9]);
     d.add(v[0], c[3], P[1]);
     d.add(v[1], c[0], P[8]);
-    d.add_face(v[1], c[1], u, P[12], ty, P[16], d0);
-    d.add_face(v[1], c[2], a, P[17], ty, P[13], d1);
+    d.template add_face<EXACT>(v[1], c[1], u, P[12], ty, P[16], d0);
+    d.template add_face<EXACT>(v[1], c[2], a, P[17], ty, P[13], d1);
     d.add(v[1], c[3], P[5]);
     d.add(v[2], c[0], P[7]);
-    d.add_face(v[2], c[1], u, P[19], b, P[15], d3);
-    d.add_face(v[2], c[2], a, P[14], b, P[18], d2);
+    d.template add_face<EXACT>(v[2], c[1], u, P[19], b, P[15], d3);
+    d.template add_face<EXACT>(v[2], c[2], a, P[14], b, P[18], d2);
     d.add(v[2], c[3], P[10]);
     d.add(v[3], c[0], P[3]);
     d.add(v[3], c[1], P[11]);
@@ -716,26 +723,22 @@ static __device__ __noinline__ int4 project_vertex_general(float4 pr, int W, int
     project_vertex_m(m, fr, pos, px, py, depth);
     return make_int4(px, py, __float_as_int(depth), 0);
 }
-// N vertices at once: one test decides for all (the general product is right
-// for any position), so that their chains run side by side.
+// Whether all N positions are finite and off the eye plane (false also for
+// some that overflow or underflow the one test made for all).
 template <int N>
-__device__ __forceinline__ void project_vertices_persp(const float (&pr)[4], const FrameDev& fr, const float4 (&pos)[N],
-                                                       int2 (&px)[N], float (&depth)[N]) {
+__device__ __forceinline__ bool positions_plain(const float4 (&pos)[N]) {
     float mag = 0.0f, zs = 1.0f;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
         mag = fadd(mag, fadd(fadd(fabsf(pos[n].x), fabsf(pos[n].y)), fadd(fabsf(pos[n].z), fabsf(pos[n].w))));
         zs = fmul(zs, pos[n].z);
     }
-    if (!(mag < __int_as_float(0x7f800000)) || zs == 0.0f) {
-#pragma unroll
-        for (int n = 0; n < N; ++n) {
-            const int4 r = project_vertex_general(make_float4(pr[0], pr[1], pr[2], pr[3]), fr.W, fr.H, fr.shift, pos[n]);
-            px[n] = make_int2(r.x, r.y);
-            depth[n] = __int_as_float(r.z);
-        }
-        return;
-    }
+    return mag < __int_as_float(0x7f800000) && zs != 0.0f;
+}
+// N plain positions at once, so that their chains run side by side.
+template <int N>
+__device__ __forceinline__ void project_vertices_plain(const float (&pr)[4], const FrameDev& fr, const float4 (&pos)[N],
+                                                       int2 (&px)[N], float (&depth)[N]) {
 #pragma unroll
     for (int n = 0; n < N; ++n) {
         const float2 pxy = fmul2(make_float2(pr[0], pr[1]), make_float2(pos[n].x, pos[n].y));

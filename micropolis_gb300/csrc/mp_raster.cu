@@ -416,6 +416,53 @@ __device__ __forceinline__ void load_matrices(const float* m, float (&mv)[16], f
     pr[3] = m[30];
 }
 
+// The vertices of run i (raster_group's numbering) for any positions: every
+// NaN of a face point zeroed, the general projection where a position is not
+// plain, and the blocks of a vertex on the eye plane noted.
+// The dice takes a run here when one of its positions is not finite or lies
+// on the eye plane, so its own loop carries none of this: dice+raster, mixed
+// 4096 patches 1.23 -> 1.17 ms, at 16x16 dicing 4.04 -> 3.78, 64 views
+// 4.40 -> 4.30, displaced 512x512 heightfield at 3840x2160 3.12 -> 3.03 (with
+// a flag per sub-patch and a second dice after the barrier the 64 views and
+// the heightfield lost 1.4 %).
+template <int PS, int NS, bool DISP>
+__device__ __noinline__ void dice_run_general(FusedSmem<PS, NS>& sm, int b, int i, const DrawDev* __restrict__ draws,
+                                              FrameDev fr) {
+    constexpr int G = PS + 1, NR = (G + kRun - 1) / kRun, RPS = G * NR, BPL = PS / 8;
+    const GroupStage<NS>& cur = sm.st[b];
+    const int k = i / RPS, c = i - k * RPS, nv0 = c / G * kRun, nu = c % G;
+#pragma unroll 1
+    for (int nv = nv0; nv < min(nv0 + kRun, G); ++nv) {
+        const float ty[1] = {sm.ty[k][nv]};
+        const float4 cw[1] = {sm.cw[k][nv]};
+        DiceColumn<1> d;
+        dice_column<1, true>(d, cur.tv[k][0], cur.cp[k], sm.tx[k][nu], ty, sm.vw[k][nu], cw);
+        float mv[16], pr[4];
+        load_matrices(draws[cur.meta[k].y].mv, mv, pr);
+        float4 pos[1] = {mul_m44v4(mv, make_float4(d.xy[0].x, d.xy[0].y, d.zw[0].x, d.zw[0].y))};
+        if (DISP) displace_vertices<1>(pos, fr.fdisp);
+        int2 px[1];
+        float dep[1];
+        if (positions_plain<1>(pos)) {
+            project_vertices_plain<1>(pr, fr, pos, px, dep);
+        } else {
+            const int4 r = project_vertex_general(make_float4(pr[0], pr[1], pr[2], pr[3]), fr.W, fr.H, fr.shift, pos[0]);
+            px[0] = make_int2(r.x, r.y);
+            dep[0] = __int_as_float(r.z);
+        }
+        const int at = k * G * G + nv * G + nu;
+        sm.pxy[at] = px[0];
+        sm.edep[at] = make_float4(pos[0].x, pos[0].y, pos[0].z, dep[0]);
+        if (pos[0].z == 0.0f) {
+            // a vertex at eye z == 0 drops every 8x8 block it belongs to (kernels/reyes.cl:130-162)
+            unsigned zb = 0;
+            for (int bv = max(nv - 1, 0) / 8; bv <= min(nv, PS - 1) / 8; ++bv)
+                for (int bu = max(nu - 1, 0) / 8; bu <= min(nu, PS - 1) / 8; ++bu) zb |= 1u << (bu + bv * BPL);
+            atomicOr(&sm.zero[b][k], zb);
+        }
+    }
+}
+
 // Dices, shades and rasterizes the n (<= NS) sub-patches at [base, base+n)
 // of the emitted list, whose inputs are staged and prepared in buffer b, with
 // the whole block; meanwhile stages and prepares the n_next sub-patches at
@@ -465,7 +512,7 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
             ty[v] = sm.ty[k][nv];
         }
         DiceColumn<kRun> d;
-        dice_column<kRun>(d, cur.tv[k][0], cur.cp[k], sm.tx[k][nu], ty, sm.vw[k][nu], cw);
+        dice_column<kRun, false>(d, cur.tv[k][0], cur.cp[k], sm.tx[k][nu], ty, sm.vw[k][nu], cw);
         // the draw's modelview, and the perspective's entries 0, 5, 10, 14
         float mv[16], pr[4];
         const int run = cur.run[k];
@@ -479,23 +526,19 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
         for (int v = 0; v < kRun; ++v)
             pos[v] = mul_m44v4(mv, make_float4(d.xy[v].x, d.xy[v].y, d.zw[v].x, d.zw[v].y));
         if (DISP) displace_vertices<kRun>(pos, fr.fdisp);
+        if (!positions_plain<kRun>(pos)) {
+            dice_run_general<PS, NS, DISP>(sm, b, i, draws, fr);
+            continue;
+        }
         int2 px[kRun];
         float dep[kRun];
-        project_vertices_persp<kRun>(pr, fr, pos, px, dep);
+        project_vertices_plain<kRun>(pr, fr, pos, px, dep);
         const int at = k * NV + nv0 * G + nu;
 #pragma unroll
         for (int v = 0; v < kRun; ++v) {
             if (G % kRun && nv0 + v >= G) break;
             sm.pxy[at + v * G] = px[v];
             sm.edep[at + v * G] = make_float4(pos[v].x, pos[v].y, pos[v].z, dep[v]);
-            if (pos[v].z == 0.0f) {
-                // a vertex at eye z == 0 drops every 8x8 block it belongs to (kernels/reyes.cl:130-162)
-                const int nv = nv0 + v;
-                unsigned zb = 0;
-                for (int bv = max(nv - 1, 0) / 8; bv <= min(nv, PS - 1) / 8; ++bv)
-                    for (int bu = max(nu - 1, 0) / 8; bu <= min(nu, PS - 1) / 8; ++bu) zb |= 1u << (bu + bv * BPL);
-                atomicOr(&sm.zero[b][k], zb);
-            }
         }
     }
     if (PS != 16 && n_next > 0 && tid < 32)
