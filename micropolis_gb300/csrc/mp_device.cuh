@@ -68,7 +68,7 @@ struct FrameDev {
     int kshift;            // depth|id key buffer tile: 1 << kshift pixels (8, 16 or 32)
     int kgx;               // key tiles per row
     int criterion;         // mp_bound_criterion
-    float vp[4];           // W << shift, H << shift, and their halves (whole numbers)
+    float vp[4];           // half of W << shift and H << shift, and those rounded down
 };
 
 // Depth|id key stored per pixel: (idepth << 32) | mp_id.  The clear key keeps
@@ -379,14 +379,13 @@ __device__ __forceinline__ float4 col_weights(float ty) {
 // x/y and z/w chains run as packed pairs.
 template <typename Pts>
 __device__ __forceinline__ float4 accumulate16(const Pts& Q, float4 vw4, float4 cw4) {
-    const float2 vw[4] = {dup2(vw4.x), dup2(vw4.y), dup2(vw4.z), dup2(vw4.w)};
-    const float2 cw[4] = {dup2(cw4.x), dup2(cw4.y), dup2(cw4.z), dup2(cw4.w)};
+    const float vw[4] = {vw4.x, vw4.y, vw4.z, vw4.w}, cw[4] = {cw4.x, cw4.y, cw4.z, cw4.w};
     float2 pxy = make_float2(0.f, 0.f), pzw = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float2 w = fmul2(vw[i], cw[j]);
+            const float2 w = dup2(fmul(vw[i], cw[j]));
             const float4 c = Q[4 * i + j];
             pxy = ffma2(w, make_float2(c.x, c.y), pxy);
             pzw = ffma2(w, make_float2(c.z, c.w), pzw);
@@ -611,11 +610,16 @@ struct DiceColumn {
 #pragma unroll
         for (int n = 0; n < N; ++n) xy[n] = zw[n] = make_float2(0.f, 0.f);
     }
-    // adds the same control point to every vertex
+    // adds the same control point to every vertex.  The weight is one product
+    // copied into a pair: as a packed product of copied factors it took a copy
+    // per factor and two cycles of the FMA pipe (with half the viewport and the
+    // packed test below: dice+raster, mixed 4096 patches 1.17 -> 1.12 ms, at
+    // 16x16 dicing 3.78 -> 3.65, 64 views 4.30 -> 4.08, displaced 512x512
+    // heightfield at 3840x2160 3.03 -> 2.95).
     __device__ __forceinline__ void add(float vw, const float (&cw)[N], float4 c) {
 #pragma unroll
         for (int n = 0; n < N; ++n) {
-            const float2 w = fmul2(dup2(vw), dup2(cw[n]));
+            const float2 w = dup2(fmul(vw, cw[n]));
             xy[n] = ffma2(w, make_float2(c.x, c.y), xy[n]);
             zw[n] = ffma2(w, make_float2(c.z, c.w), zw[n]);
         }
@@ -631,7 +635,7 @@ struct DiceColumn {
         for (int n = 0; n < N; ++n) {
             float rd = frcp(den[n]);
             if (!EXACT && a == 0.0f && den[n] == 0.0f) rd = 0.0f;
-            const float2 r = dup2(rd), b2 = dup2(b[n]), w = fmul2(dup2(vw), dup2(cw[n]));
+            const float2 r = dup2(rd), b2 = dup2(b[n]), w = dup2(fmul(vw, cw[n]));
             const float2 fxy = fmul2(ffma2(b2, make_float2(B.x, B.y), axy), r);
             const float2 fzw = fmul2(ffma2(b2, make_float2(B.z, B.w), azw), r);
             xy[n] = ffma2(w, EXACT ? make_float2(sel_nan(fxy.x), sel_nan(fxy.y)) : fxy, xy[n]);
@@ -724,18 +728,28 @@ static __device__ __noinline__ int4 project_vertex_general(float4 pr, int W, int
     return make_int4(px, py, __float_as_int(depth), 0);
 }
 // Whether all N positions are finite and off the eye plane (false also for
-// some that overflow or underflow the one test made for all).
-template <int N>
+// some that overflow or underflow the one test made for all).  PACKED takes
+// two instructions a position less; with the displacement's registers around
+// it, the 512x512 heightfield was 0.3 % slower so.
+template <int N, bool PACKED>
 __device__ __forceinline__ bool positions_plain(const float4 (&pos)[N]) {
-    float mag = 0.0f, zs = 1.0f;
+    float2 mag = make_float2(0.f, 0.f);
+    float zs = 1.0f;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
-        mag = fadd(mag, fadd(fadd(fabsf(pos[n].x), fabsf(pos[n].y)), fadd(fabsf(pos[n].z), fabsf(pos[n].w))));
+        if (PACKED) {   // 0 times each component: NaN unless it is finite
+            mag = ffma2(make_float2(pos[n].x, pos[n].y), dup2(0.0f), mag);
+            mag = ffma2(make_float2(pos[n].z, pos[n].w), dup2(0.0f), mag);
+        } else {
+            mag.x = fadd(mag.x, fadd(fadd(fabsf(pos[n].x), fabsf(pos[n].y)), fadd(fabsf(pos[n].z), fabsf(pos[n].w))));
+        }
         zs = fmul(zs, pos[n].z);
     }
-    return mag < __int_as_float(0x7f800000) && zs != 0.0f;
+    return (PACKED ? fadd(mag.x, mag.y) == 0.0f : mag.x < __int_as_float(0x7f800000)) && zs != 0.0f;
 }
-// N plain positions at once, so that their chains run side by side.
+// N plain positions at once, so that their chains run side by side.  Times
+// the viewport, then halved, is one product with half the viewport: exact
+// unless it leaves the normal range, where sum and conversion give the same.
 template <int N>
 __device__ __forceinline__ void project_vertices_plain(const float (&pr)[4], const FrameDev& fr, const float4 (&pos)[N],
                                                        int2 (&px)[N], float (&depth)[N]) {
@@ -746,7 +760,6 @@ __device__ __forceinline__ void project_vertices_plain(const float (&pr)[4], con
         const float rw = frcp(-pos[n].z);
         float2 e = fmul2(pxy, dup2(rw));
         e = fmul2(e, make_float2(fr.vp[0], fr.vp[1]));
-        e = fmul2(e, dup2(0.5f));
         e = fadd2(e, make_float2(fr.vp[2], fr.vp[3]));
         px[n] = make_int2(__float2int_rz(e.x), __float2int_rz(e.y));
         depth[n] = fmul(pz, rw);

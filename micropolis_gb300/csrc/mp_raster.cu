@@ -443,7 +443,7 @@ __device__ __noinline__ void dice_run_general(FusedSmem<PS, NS>& sm, int b, int 
         if (DISP) displace_vertices<1>(pos, fr.fdisp);
         int2 px[1];
         float dep[1];
-        if (positions_plain<1>(pos)) {
+        if (positions_plain<1, !DISP>(pos)) {
             project_vertices_plain<1>(pr, fr, pos, px, dep);
         } else {
             const int4 r = project_vertex_general(make_float4(pr[0], pr[1], pr[2], pr[3]), fr.W, fr.H, fr.shift, pos[0]);
@@ -526,7 +526,7 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
         for (int v = 0; v < kRun; ++v)
             pos[v] = mul_m44v4(mv, make_float4(d.xy[v].x, d.xy[v].y, d.zw[v].x, d.zw[v].y));
         if (DISP) displace_vertices<kRun>(pos, fr.fdisp);
-        if (!positions_plain<kRun>(pos)) {
+        if (!positions_plain<kRun, !DISP>(pos)) {
             dice_run_general<PS, NS, DISP>(sm, b, i, draws, fr);
             continue;
         }
