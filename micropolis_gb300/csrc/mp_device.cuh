@@ -68,7 +68,7 @@ struct FrameDev {
     int kshift;            // depth|id key buffer tile: 1 << kshift pixels (8, 16 or 32)
     int kgx;               // key tiles per row
     int criterion;         // mp_bound_criterion
-    float vp[4];           // half of W << shift and H << shift, and those rounded down
+    float vp[4];           // W << shift, H << shift, and their halves (whole numbers)
 };
 
 // Depth|id key stored per pixel: (idepth << 32) | mp_id.  The clear key keeps
@@ -612,8 +612,8 @@ struct DiceColumn {
     }
     // adds the same control point to every vertex.  The weight is one product
     // copied into a pair: as a packed product of copied factors it took a copy
-    // per factor and two cycles of the FMA pipe (with half the viewport and the
-    // packed test below: dice+raster, mixed 4096 patches 1.17 -> 1.12 ms, at
+    // per factor and two cycles of the FMA pipe (with the packed test below:
+    // dice+raster, mixed 4096 patches 1.17 -> 1.12 ms, at
     // 16x16 dicing 3.78 -> 3.65, 64 views 4.30 -> 4.08, displaced 512x512
     // heightfield at 3840x2160 3.03 -> 2.95).
     __device__ __forceinline__ void add(float vw, const float (&cw)[N], float4 c) {
@@ -747,9 +747,10 @@ __device__ __forceinline__ bool positions_plain(const float4 (&pos)[N]) {
     }
     return (PACKED ? fadd(mag.x, mag.y) == 0.0f : mag.x < __int_as_float(0x7f800000)) && zs != 0.0f;
 }
-// N plain positions at once, so that their chains run side by side.  Times
-// the viewport, then halved, is one product with half the viewport: exact
-// unless it leaves the normal range, where sum and conversion give the same.
+// N plain positions at once, so that their chains run side by side.  (One
+// product with half the viewport would be the same number, but the compiler
+// fuses a packed product with the packed sum after it; fused with the exact
+// halving it rounds as it should.)
 template <int N>
 __device__ __forceinline__ void project_vertices_plain(const float (&pr)[4], const FrameDev& fr, const float4 (&pos)[N],
                                                        int2 (&px)[N], float (&depth)[N]) {
@@ -760,6 +761,7 @@ __device__ __forceinline__ void project_vertices_plain(const float (&pr)[4], con
         const float rw = frcp(-pos[n].z);
         float2 e = fmul2(pxy, dup2(rw));
         e = fmul2(e, make_float2(fr.vp[0], fr.vp[1]));
+        e = fmul2(e, dup2(0.5f));
         e = fadd2(e, make_float2(fr.vp[2], fr.vp[3]));
         px[n] = make_int2(__float2int_rz(e.x), __float2int_rz(e.y));
         depth[n] = fmul(pz, rw);

@@ -805,8 +805,8 @@ mp_status mp_create(const mp_options* opts, mp_ctx** out) {
     fr.clear[3] = 1000.0f;
     fr.gx = W / 8;
     fr.gy = H / 8;
-    fr.vp[0] = 0.5f * (float)(W << fr.shift);
-    fr.vp[1] = 0.5f * (float)(H << fr.shift);
+    fr.vp[0] = (float)(W << fr.shift);
+    fr.vp[1] = (float)(H << fr.shift);
     fr.vp[2] = (float)((W << fr.shift) / 2);
     fr.vp[3] = (float)((H << fr.shift) / 2);
     mp_status st = MP_OK;
