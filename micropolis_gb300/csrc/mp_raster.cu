@@ -549,7 +549,11 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
     // The list of quads that can touch a pixel: a quad with a large bbox, or a
     // small one with an accepted winding and a pixel centre in its bbox.  A
     // thread walks a strip of 8 quads (column nu, rows 8 h .. 8 h + 7), so
-    // each row's two vertices and their bounds serve two quads.
+    // each row's two vertices and their bounds serve two quads.  (Pixel
+    // centres by rounding the upper bound down, and the strip's bounds every
+    // second row: dice+raster, mixed 4096 patches 1.122 -> 1.114 ms, 64 views
+    // 4.08 -> 4.05, displaced 512x512 heightfield at 3840x2160 2.93 -> 2.90;
+    // the winding of only the quads with a pixel centre: 1.150, 4.27, 2.89.)
     constexpr int SPS = PS * BPL;   // strips of a sub-patch
     for (int i0 = tid & ~31; i0 < n * SPS; i0 += TH) {
         const int i = i0 + lane;
@@ -570,17 +574,18 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
                 const int2 c2 = at[(r + 1) * G], c3 = at[(r + 1) * G + 1];
                 const int nlx = min(c2.x, c3.x), nhx = max(c2.x, c3.x), nly = min(c2.y, c3.y), nhy = max(c2.y, c3.y);
                 const int minx = min(lx, nlx), maxx = max(hx, nhx), miny = min(ly, nly), maxy = max(hy, nhy);
-                if (((minx + one) >> fr.shift) <= (maxx >> fr.shift) && ((miny + one) >> fr.shift) <= (maxy >> fr.shift))
-                    inside |= 1u << r;
+                if ((maxx & ~one) >= minx && (maxy & ~one) >= miny) inside |= 1u << r;
                 // is_front_facing (kernels/reyes.cl:54-65) on wrapped int32
                 const int d1x = wsub(q.x, a.x), d1y = wsub(q.y, a.y);
                 const int d2x = wsub(c2.x, a.x), d2y = wsub(c2.y, a.y);
                 const int d3x = wsub(c3.x, a.x), d3y = wsub(c3.y, a.y);
                 if (wsub(wmul(d1x, d3y), wmul(d3x, d1y)) < 0 || wsub(wmul(d3x, d2y), wmul(d2x, d3y)) < 0) wind |= 1u << r;
-                slx = min(slx, nlx);
-                shx = max(shx, nhx);
-                sly = min(sly, nly);
-                shy = max(shy, nhy);
+                if (r & 1) {   // two rows at once
+                    slx = min(slx, minx);
+                    shx = max(shx, maxx);
+                    sly = min(sly, miny);
+                    shy = max(shy, maxy);
+                }
                 lx = nlx; hx = nhx; ly = nly; hy = nhy;
                 a = c2;
                 q = c3;
