@@ -51,13 +51,13 @@ KERNEL_SOURCES = {
     "canonical_sort_or_sample": ["mp_sort.cu", "mp_bns_loop.cuh", "mp_internal.h"],
 }
 NCU_FIGURES = {
-    # ncu --set full of one frame (profiles/raster_fused_mixed4096_1920x1080.md and the
+    # ncu of one frame (profiles/raster_fused_mixed4096_1920x1080.md and the
     # summaries beside it), sources as of the capture
-    "dice_raster": {"source": "29884bf2bd105b71", "traffic": 101_184_768 + 66_111_744, "inst": 1_036_109_842},
-    "bound_split": {"source": "83928645e25485d2", "traffic": 2_856_960 + 213_277_696, "inst": 171_051_632},
-    "resolve_or_shade": {"source": "29884bf2bd105b71", "traffic": 61_478_400 + 6_120_448, "inst": 10_215_932},
-    "canonical_sort_or_sample": {"source": "1b09df18b3732cc4", "traffic": 30_085_376 + 6_288_128,
-                                 "inst": 33_245_208},
+    "dice_raster": {"source": "62aea51f17c8749a", "traffic": 101_773_312 + 65_697_792, "inst": 686_423_965},
+    "bound_split": {"source": "d623e6a3bf979e5b", "traffic": 4_508_928 + 15_795_456, "inst": 136_367_102},
+    "resolve_or_shade": {"source": "62aea51f17c8749a", "traffic": 61_491_968 + 5_449_728, "inst": 7_686_845},
+    "canonical_sort_or_sample": {"source": "c963fb5b008b97ec", "traffic": 34_220_544 + 2_097_664,
+                                 "inst": 15_268_433},
 }
 
 
