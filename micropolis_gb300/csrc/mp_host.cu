@@ -340,7 +340,7 @@ unsigned long long hc(const mp_ctx* c, int w) { return c->h_ctrl[w * kCtrlStride
 
 // Ranges bounded in the last batched frame: the roots and two per split.
 long long bounded_ranges(const mp_ctx* c) {
-    return (long long)hc(c, kRoots) + 2 * (long long)(hc(c, kOutstanding) >> 32);
+    return (long long)hc(c, kRoots) + 2 * (long long)hc(c, kSplits);
 }
 
 mp_status read_ctrl(mp_ctx* c) {
@@ -654,10 +654,11 @@ mp_status batched_frame(mp_ctx* c) {
         unsigned long long status = hc(c, kStatus);
         if (status != kErrOverflow) {
             if (status) return check_status(c, status);
+            if (hc(c, kQTail) & kUnitMask) return fail(c, MP_ERR_STATE, "bound-and-split ended before its work");
             break;
         }
         // regrow what overflowed and render the frame again
-        long long pushed = (long long)hc(c, kQTail);
+        long long pushed = (long long)handover_slot(hc(c, kQTail));
         long long outc = (long long)hc(c, kOutCount);
         long long bigc = (long long)hc(c, kBigCount);
         if (pushed > c->q.capacity && (st = grow_queue(c, pushed + pushed / 2))) return st;

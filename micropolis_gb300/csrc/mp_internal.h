@@ -6,16 +6,18 @@
 #include <cuda_runtime.h>
 
 #include "mp_device.cuh"
+#include "mp_handover.h"
 
 namespace mp {
 
 // Control words of one frame, each on its own 128-byte line so that the hot
 // atomics of different roles land in different L2 slices.
 enum CtrlWord {
-    kQTail = 0,        // bundle slots reserved by warps that give pairs away
+    kQTail = 0,        // units of work not finished | bundle slots reserved << 32 (mp_handover.h)
     kQHead,            // bundle tickets taken by waiting warps (beyond the first, dealt by warp number)
     kRootHead,         // roots taken (beyond the first, dealt by warp number)
-    kOutstanding,      // units of work not finished | ranges split << 32
+    kSplits,           // ranges split
+    kGiven,            // bundles given so far, for the warps that decide whether to give
     kOutCount,         // sub-patches emitted
     kDone,             // bound-and-split finished
     kStatus,           // first error code (mp_status values)
