@@ -760,6 +760,9 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
             staged ? sd : gdraws, root_prefix, n_draws, fr, q, sub, sub.seq, nullptr, ctrl, spin_limit,
             reinterpret_cast<float*>(smem_raw + kPtsOffset), (int)(blockIdx.x + n_bns_ctas * (threadIdx.x >> 5)),
             n_bns_ctas * (fused_threads<NS>() / 32));
+        // the rings were written by ordinary stores, and bulk copies (another
+        // proxy) write the same bytes next: each thread orders its own before them
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
