@@ -681,8 +681,11 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
     stamp_start(ctrl, 3);
     // an earlier stage of the frame failed (the host reports it): the list
-    // may be incomplete, so nothing is rasterized
-    if (*(volatile unsigned long long*)cw(ctrl, kStatus) != 0) return;
+    // may be incomplete, so nothing is rasterized.  The whole block decides
+    // the same: blocks that already run can set the status meanwhile (the list
+    // of large quads overflows), and a block without its first warp would work
+    // on records that nobody staged.
+    if (__syncthreads_or(*(volatile unsigned long long*)cw(ctrl, kStatus) != 0)) return;
     // (list positions fit 32 bits: micropolygon ids do)
     const int S = (int)min((long long)*(volatile unsigned long long*)cw(ctrl, kOutCount), sub.capacity);
     int frags = 0;
