@@ -178,6 +178,10 @@ mp_status mp_finish(mp_ctx* ctx);
  * launches with CUDA events between them instead of one graph replay, and
  * mp_stats.stage_ms is filled (for profiling; the graph replay is faster). */
 mp_status mp_set_stage_timing(mp_ctx* ctx, int32_t on);
+/* Blocks of the separate bound-and-split launch; 0: as many as the device holds
+ * at once (the default).  The frame is the same for any number: the launch ends
+ * whatever part of its blocks the device holds (the tests ask for more). */
+mp_status mp_set_bns_blocks(mp_ctx* ctx, int32_t blocks);
 /* Renderer::dump_trace (Renderer.h:43): the last frame's device commands as
  * `name@queue:queued:submit:start:end:id:deps` lines (src/CL/Device.cpp:275-289),
  * times in ns from the start of the frame, deps '|'-separated ids, named with

@@ -69,6 +69,7 @@ SIGNATURES = [
     ("mp_draw_views", ctypes.c_int, [c_void_p, i32, P(MpView)]),
     ("mp_finish", ctypes.c_int, [c_void_p]),
     ("mp_set_stage_timing", ctypes.c_int, [c_void_p, i32]),
+    ("mp_set_bns_blocks", ctypes.c_int, [c_void_p, i32]),
     ("mp_dump_trace", ctypes.c_int, [c_void_p, ctypes.c_char_p, ctypes.c_size_t]),
     ("mp_framebuffer", ctypes.c_int, [c_void_p, P(c_void_p), P(c_void_p), P(i32), P(i32), P(i32)]),
     ("mp_read_framebuffer", ctypes.c_int, [c_void_p, i32, P(f32), P(i32), i32]),

@@ -28,6 +28,9 @@ constexpr int kBnsBlock = 128;
 constexpr int kBnsSmemDraws = 8;
 constexpr size_t kBnsSmem = bns_smem<kBnsBlock, kStackPairs>();
 
+// (128 registers, and shared memory, hold four blocks per SM.  A launch bound of
+// four made the compiler's schedule slower, the 8x8 heightfield 0.045 -> 0.053
+// ms, and one register more makes it take 168, which hold three.)
 template <int CRIT>
 __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev* __restrict__ gdraws,
                                                                    const int* __restrict__ root_prefix,
@@ -39,7 +42,9 @@ __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev
     // draw constants staged in shared memory when they fit
     __shared__ DrawDev s_draws[kBnsSmemDraws];
     extern __shared__ __align__(16) float s_bns[];
+    __shared__ unsigned s_claim;
     stamp_start(ctrl, 1);
+    if (threadIdx.x == 0) s_claim = bns_claim(ctrl);
     // the last frame's entries of the sort's bucket table (whole uint4s), while the first ranges are on their way
     const unsigned n_clear = __ldg(used) / 4;
     for (unsigned i = blockIdx.x * kBnsBlock + threadIdx.x; i < n_clear; i += gridDim.x * kBnsBlock)
@@ -49,12 +54,10 @@ __global__ void __launch_bounds__(kBnsBlock) bns_persistent_kernel(const DrawDev
         const int words = n_draws * (int)(sizeof(DrawDev) / 4);
         for (int i = threadIdx.x; i < words; i += blockDim.x)
             reinterpret_cast<int*>(s_draws)[i] = __ldg(reinterpret_cast<const int*>(gdraws) + i);
-        __syncthreads();
     }
-    // consecutive warp numbers on different SMs: the first roots spread over the chip
-    const int warp = (int)(blockIdx.x + gridDim.x * (threadIdx.x >> 5));
+    __syncthreads();
     bns_warp_loop<CRIT, kStackPairs>(staged ? s_draws : gdraws, root_prefix, n_draws, fr, q, out, nullptr, roots, ctrl,
-                                     spin_limit, s_bns, warp, (int)(gridDim.x * (kBnsBlock / 32)));
+                                     spin_limit, s_bns, s_claim, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------

@@ -55,6 +55,7 @@ __device__ __forceinline__ void stamp_start(unsigned long long* ctrl, int k) {
 __device__ __forceinline__ void bns_reset(unsigned long long* ctrl, long long roots) {
     *cw(ctrl, kQTail) = handover_start((unsigned long long)roots);
     *cw(ctrl, kQHead) = 0;
+    *cw(ctrl, kClaims) = 0;
     *cw(ctrl, kRootHead) = 0;
     *cw(ctrl, kSplits) = 0;
     *cw(ctrl, kGiven) = 0;
@@ -71,6 +72,11 @@ __device__ __forceinline__ void bns_reset(unsigned long long* ctrl, long long ro
     *cw(ctrl, kSortDone) = 0;
     *cw(ctrl, kSortMost) = 0;
     *cw(ctrl, kStampEnd) = 0;
+}
+
+// This block's claim, by its first thread: the number of claims before it.
+__device__ __forceinline__ unsigned bns_claim(unsigned long long* ctrl) {
+    return (unsigned)atomicAdd(cw(ctrl, kClaims), 1ull);
 }
 
 __device__ __forceinline__ void set_status(unsigned long long* ctrl, int code) {
@@ -114,7 +120,17 @@ constexpr size_t bns_smem() {
 // that run concurrently; when roots is given, each root's record counts its
 // sub-patches and bounds their paths (for the canonical sort).  CRIT selects
 // the bound criterion (bns_decide).
-// `warp` is the warp's number among the n_warps that run the loop.
+// `blocks` blocks run the loop; `claim` is this one's number in the order in
+// which they started (bns_claim).
+//
+// Roots are dealt in shares: share s to warp s / blocks of the block with claim
+// s % blocks, the rest with atomics.  A warp that has waited a microsecond takes
+// the claims of blocks that have not started, so every root that nobody works
+// on yet can be taken by any warp that runs, and a warp waits only for warps
+// that hold work: the launch ends whatever part of its blocks the device holds
+// at once.  (Against shares and tickets dealt by block number without atomics:
+// 64 views 0.91 -> 0.83 ms, the displaced 512x512 heightfield at 3840x2160
+// 0.443 -> 0.410, 24 objects 0.124 -> 0.126, the 8x8 heightfield 0.045 as before.)
 //
 // A warp works depth first on a stack of its own: a step takes up to 16
 // pairs (32 ranges, one per lane) and, while few pairs are left and roots
@@ -136,8 +152,7 @@ template <int CRIT, int C>
 __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* __restrict__ root_prefix, int n_draws,
                                               const FrameDev& fr, const Queue& q, const SubPatches& out,
                                               unsigned* out_seq, RootInfo* roots, unsigned long long* ctrl,
-                                              long long spin_limit,
-                                              float* smem, int warp, int n_warps) {
+                                              long long spin_limit, float* smem, unsigned claim, unsigned blocks) {
     static_assert(stack_stride<C>() > C + 32 && kPairWords > 27 && C >= 32, "scratch columns");
     static_assert(C >= 32, "a step adds up to 16 pairs, or 32 to an empty ring");
     // Pairs are given to waiting warps when more than kGiveAbove are left, and
@@ -151,51 +166,72 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
     const int lane = threadIdx.x & 31;
     float* ring = smem + (threadIdx.x >> 5) * (kPairWords * S);
     const unsigned epoch = (unsigned)*(volatile unsigned long long*)cw(ctrl, kEpoch);
-    const long long R = (long long)*(volatile unsigned long long*)cw(ctrl, kRoots);
-    // the first roots and tickets are dealt by warp number, without atomics:
-    // the lowest `busy` warps start with `share` roots each
-    const int share = (int)min(32ll, (R + n_warps - 1) / n_warps);
-    const long long busy = share > 0 ? min((long long)n_warps, (R + share - 1) / share) : 0;
-    const bool more_roots = (long long)n_warps * share < R;   // the rest is taken with atomics
-    long long root = (long long)warp * share;                 // this warp's next roots: [root, root_end)
-    long long root_end = max(root, min(root + share, R));
-    bool roots_left = more_roots;
-    unsigned units = (unsigned)(root_end - root);             // units taken since the last report
-    unsigned splits = 0;                                      // ranges split since the last report
-    bool first_ticket = warp >= busy;
+    const unsigned R = (unsigned)*(volatile unsigned long long*)cw(ctrl, kRoots);   // (below 2^31)
+    const unsigned warps = blockDim.x >> 5, n_warps = blocks * warps;
+    const unsigned share = min(32u, (R + n_warps - 1) / n_warps);
+    const unsigned dealt = n_warps * share;                   // roots from here on are taken with atomics
+    // the claims that have roots (share s holds some while s * share < R)
+    const unsigned busy = share ? min(blocks, (R + share - 1) / share) : 0;
+    unsigned sh = claim + blocks * (threadIdx.x >> 5);        // the next share of this warp
+    unsigned sh_left = claim < blocks ? 1 : 0;                // its shares left: sh, sh + blocks, ...
+    unsigned root = 0, root_end = 0;                          // its next roots: [root, root_end)
+    bool roots_left = dealt < R, claims_left = busy > 0;
+    unsigned units = 0;                                       // units taken since the last report
+    // in the words beside the scratch columns: ranges split since the last
+    // report (lane 0), the depth of the deepest sub-patch emitted so far
+    unsigned* kept = reinterpret_cast<unsigned*>(ring + C + 32);
+    if (lane == 0) kept[0] = kept[S] = 0;
+    __syncwarp();
+    unsigned slot = 0;                                        // of this warp's ticket
+    bool has_ticket = false;
     int bottom = 0, n = 0;    // ring: pairs bottom .. bottom + n - 1 (mod C)
-    unsigned max_depth = 0;   // deepest emitted sub-patch of this warp so far
     while (true) {
-        if (roots_left && root >= root_end && n < 8) {
-            unsigned long long t = 0;
-            if (lane == 0) t = atomicAdd(cw(ctrl, kRootHead), (unsigned long long)share);
-            root = (long long)n_warps * share + (long long)__shfl_sync(0xffffffffu, t, 0);
-            root_end = max(root, min(root + share, R));
-            units += (unsigned)(root_end - root);
-            roots_left = root < root_end;
+        if (root >= root_end && n < 8) {
+            if (sh_left) {
+                root = sh * share;
+                root_end = max(root, min(root + share, R));
+                sh += blocks;
+                --sh_left;
+                units += root_end - root;
+            } else if (roots_left) {
+                unsigned long long t = 0;
+                if (lane == 0) t = atomicAdd(cw(ctrl, kRootHead), (unsigned long long)share);
+                root = dealt + (unsigned)__shfl_sync(0xffffffffu, t, 0);
+                root_end = max(root, min(root + share, R));
+                units += root_end - root;
+                roots_left = root < root_end;
+            }
         }
         if (n == 0 && root >= root_end) {
             // out of work: report, then wait (bounded) for a bundle: first for
             // its pair count, then for its words, each valid once it carries
             // this frame's epoch
-            long long slot = warp - busy;
             int got = 0;
+            unsigned stolen = busy;
             if (lane == 0) {
-                if (splits) atomicAdd(cw(ctrl, kSplits), (unsigned long long)splits);
+                if (kept[0]) atomicAdd(cw(ctrl, kSplits), (unsigned long long)kept[0]);
+                kept[0] = 0;
                 if (units && handover_ended(atomicAdd(cw(ctrl, kQTail), handover_finish(units)), units))
                     st_release_u64(cw(ctrl, kDone), 1ull);
-                if (!first_ticket) slot = n_warps - busy + (long long)atomicAdd(cw(ctrl, kQHead), 1ull);
-                long long idle = 0;
+                if (!has_ticket) slot = (unsigned)atomicAdd(cw(ctrl, kQHead), 1ull);
+                unsigned idle = 0;
                 unsigned sleep_ns = 32;
                 while (true) {
-                    if (slot < q.capacity) {
-                        const unsigned long long v = ld_relaxed_u64(q.words + slot * kBundleWords + kBundleWords - 1);
+                    if ((long long)slot < q.capacity) {
+                        const unsigned long long v = ld_relaxed_u64(q.words + (size_t)slot * kBundleWords + kBundleWords - 1);
                         if ((unsigned)(v >> 32) == epoch) {
                             got = (int)(unsigned)v;
                             break;
                         }
                     }
                     if (*(volatile unsigned long long*)cw(ctrl, kDone)) break;
+                    if (sleep_ns == 512 && claims_left) {
+                        // a microsecond without work: blocks may not have started (claims only grow)
+                        if (*(volatile unsigned long long*)cw(ctrl, kClaims) < busy)
+                            stolen = (unsigned)atomicAdd(cw(ctrl, kClaims), 1ull);
+                        if (stolen < busy) break;
+                        claims_left = false;
+                    }
                     if (++idle > spin_limit) {
                         set_status(ctrl, kErrTimeout);
                         st_release_u64(cw(ctrl, kDone), 1ull);
@@ -205,15 +241,21 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
                     if (sleep_ns < 512) sleep_ns <<= 1;
                 }
             }
+            units = 0;
+            stolen = __shfl_sync(0xffffffffu, stolen, 0);
+            has_ticket = stolen < busy;   // (kept for the next wait)
+            if (has_ticket) {
+                sh = stolen;
+                sh_left = warps;
+                continue;
+            }
             n = __shfl_sync(0xffffffffu, got, 0);
             if (n == 0) break;
             slot = __shfl_sync(0xffffffffu, slot, 0);
-            first_ticket = false;
             units = 1;
-            splits = 0;
             bottom = 0;
-            const unsigned long long* rec = q.words + slot * kBundleWords;
-            long long tries = 0;
+            const unsigned long long* rec = q.words + (size_t)slot * kBundleWords;
+            unsigned tries = 0;
             bool valid;
             do {
                 valid = true;
@@ -236,17 +278,17 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
         }
         // this step's ranges: pairs from the top of the ring, then roots
         const int pop = min(n, 16);
-        const int n_root = (int)min((long long)(32 - 2 * pop), root_end - root);
+        const int n_root = (int)min((unsigned)(32 - 2 * pop), root_end - root);
         // tickets taken and bundles given so far, for the hand-over below
         // (loaded here so that the bounds cover the latency, and the bundles
         // from a word of their own: polled in kQTail, which every giver and
         // finisher updates, 64 views took 0.975 ms for 0.911, the 512x512
         // heightfield at 3840x2160 0.478 for 0.443)
         const bool may_give = n + pop + n_root > kGiveAbove;
-        unsigned long long taken = 0, filled = 0;
+        unsigned taken = 0, filled = 0;
         if (may_give && lane == 0) {
-            taken = *(volatile unsigned long long*)cw(ctrl, kQHead);
-            filled = *(volatile unsigned long long*)cw(ctrl, kGiven);
+            taken = (unsigned)*(volatile unsigned long long*)cw(ctrl, kQHead);
+            filled = (unsigned)*(volatile unsigned long long*)cw(ctrl, kGiven);
         }
         const int src = wrap(bottom + max(n - 1 - (lane >> 1), 0));
         const bool child = lane < 2 * pop, active = lane < 2 * pop + n_root;
@@ -278,14 +320,14 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
             if (half && depth <= 32) path |= 0x80000000u >> (depth - 1);
         } else if (active) {
             // root: find the draw whose patch range holds it
-            const long long rt = root + (lane - 2 * pop);
+            const int rt = (int)root + (lane - 2 * pop);
             int lo = 0, hi = n_draws - 1;
             while (lo < hi) {
                 int mid = (lo + hi + 1) >> 1;
                 if (__ldg(root_prefix + mid) <= rt) lo = mid; else hi = mid - 1;
             }
             draw = lo;
-            pid = (int)(rt - __ldg(root_prefix + lo));
+            pid = rt - __ldg(root_prefix + lo);
         }
         F3 pts[9];   // the range's samples, (iu, iv) at 3 * iv + iu (CPU criterion)
         if (samples) {
@@ -388,12 +430,15 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
         const bool split = dec == kSplitX || dec == kSplitY;
         const unsigned smask = __ballot_sync(0xffffffffu, split);
         const unsigned emit_depth = __reduce_max_sync(0xffffffffu, dec == kDraw ? (unsigned)depth : 0u);
-        unsigned long long obase = 0;
-        if (lane == 0 && emask) obase = atomicAdd(cw(ctrl, kOutCount), (unsigned long long)__popc(emask));
-        if (emit_depth > max_depth) {
+        unsigned obase = 0;
+        if (lane == 0 && emask) obase = (unsigned)atomicAdd(cw(ctrl, kOutCount), (unsigned long long)__popc(emask));
+        if (emit_depth > kept[S]) {
             // the sort packs the frame's keys into root bits above this many path bits
-            max_depth = emit_depth;
-            if (lane == 0) atomicMax(cw(ctrl, kMaxDepth), (unsigned long long)emit_depth);
+            __syncwarp();
+            if (lane == 0) {
+                kept[S] = emit_depth;
+                atomicMax(cw(ctrl, kMaxDepth), (unsigned long long)emit_depth);
+            }
         }
         if (roots && emask) {
             // one update per warp while its emitted ranges share a root, as
@@ -440,10 +485,10 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
             it[33 * S] = __uint_as_float(path);
         }
         n += __popc(smask);
-        splits += (unsigned)__popc(smask);
+        if (lane == 0) kept[0] += (unsigned)__popc(smask);
         obase = __shfl_sync(0xffffffffu, obase, 0);
         if (dec == kDraw) {
-            const unsigned long long o = obase + __popc(emask & lanemask_lt());
+            const unsigned o = obase + __popc(emask & lanemask_lt());
             if ((long long)o < out.capacity) {
                 out.range[o] = r;
                 out.meta[o] = make_int2(pid, draw);
@@ -456,9 +501,9 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
         }
         __syncwarp();
         // hand the oldest pairs over: to waiting warps, and what crowds the ring
-        long long wanting = 0;
+        int wanting = 0;
         if (may_give && n > kGiveAbove) {
-            if ((long long)filled < q.capacity) wanting = (long long)taken + (n_warps - busy) - (long long)filled;
+            if ((long long)filled < q.capacity) wanting = (int)taken - (int)filled;
             wanting = __shfl_sync(0xffffffffu, wanting, 0);
         }
         while (n > kFull || (wanting > 0 && n > kGiveAbove)) {

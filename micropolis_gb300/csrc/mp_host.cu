@@ -768,6 +768,7 @@ mp_status mp_create(const mp_options* opts, mp_ctx** out) {
     if (o.reyes_patches_per_pass < 1 || o.batch_views < 1 || o.batch_views > 65536) return MP_ERR_INVALID_ARG;
     if (o.path != MP_PATH_PLAIN && o.path != MP_PATH_BATCHED) return MP_ERR_INVALID_ARG;
     if (o.spin_limit <= 0) o.spin_limit = 1 << 20;
+    o.spin_limit = std::min<int64_t>(o.spin_limit, 0xfffffffeu);   // (an hour of polls; the kernels count in 32 bits)
     if (o.bound_criterion != MP_BOUND_CPU && o.bound_criterion != MP_BOUND_GPU) return MP_ERR_INVALID_ARG;
     if (o.raster_tile == 0) o.raster_tile = 8;
     if (o.raster_tile != 8 && o.raster_tile != 16 && o.raster_tile != 32) return MP_ERR_INVALID_ARG;
@@ -1145,6 +1146,14 @@ mp_status mp_set_stage_timing(mp_ctx* c, int32_t on) {
     if (!c) return MP_ERR_INVALID_ARG;
     if (c->in_frame) return fail(c, MP_ERR_STATE, "stage timing change inside a frame");
     c->stage_timing = on != 0;
+    return MP_OK;
+}
+
+mp_status mp_set_bns_blocks(mp_ctx* c, int32_t blocks) {
+    if (!c || blocks < 0 || blocks > 65535) return MP_ERR_INVALID_ARG;
+    if (c->in_frame) return fail(c, MP_ERR_STATE, "launch change inside a frame");
+    c->bns_grid = blocks ? blocks : bns_persistent_grid(c->fr.criterion);
+    c->graph_stale = true;
     return MP_OK;
 }
 

@@ -14,8 +14,9 @@ namespace mp {
 // atomics of different roles land in different L2 slices.
 enum CtrlWord {
     kQTail = 0,        // units of work not finished | bundle slots reserved << 32 (mp_handover.h)
-    kQHead,            // bundle tickets taken by waiting warps (beyond the first, dealt by warp number)
-    kRootHead,         // roots taken (beyond the first, dealt by warp number)
+    kQHead,            // bundle tickets taken by waiting warps
+    kClaims,           // claims of dealt roots: by blocks that started, and by warps in the place of others
+    kRootHead,         // roots taken beyond the dealt ones
     kSplits,           // ranges split
     kGiven,            // bundles given so far, for the warps that decide whether to give
     kOutCount,         // sub-patches emitted

@@ -747,8 +747,10 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     constexpr size_t kPtsOffset = kFramePtsOffset;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ long long s_group;
+    __shared__ unsigned s_claim;
     stamp_start(ctrl, 3);
     if ((int)blockIdx.x < n_bns_ctas) {
+        if (threadIdx.x == 0) s_claim = bns_claim(ctrl);
         // draw constants staged in the (not yet used) raster buffer
         DrawDev* sd = reinterpret_cast<DrawDev*>(smem_raw);
         const bool staged = n_draws <= kStaged;
@@ -756,13 +758,12 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
             const int words = n_draws * (int)(sizeof(DrawDev) / 4);
             for (int i = threadIdx.x; i < words; i += blockDim.x)
                 reinterpret_cast<int*>(sd)[i] = __ldg(reinterpret_cast<const int*>(gdraws) + i);
-            __syncthreads();
         }
+        __syncthreads();
         // the CPU criterion only: the host runs the GPU criterion as two launches
         bns_warp_loop<0, kStackPairsFrame>(
             staged ? sd : gdraws, root_prefix, n_draws, fr, q, sub, sub.seq, nullptr, ctrl, spin_limit,
-            reinterpret_cast<float*>(smem_raw + kPtsOffset), (int)(blockIdx.x + n_bns_ctas * (threadIdx.x >> 5)),
-            n_bns_ctas * (fused_threads<NS>() / 32));
+            reinterpret_cast<float*>(smem_raw + kPtsOffset), s_claim, (unsigned)n_bns_ctas);
         // the rings were written by ordinary stores, and bulk copies (another
         // proxy) write the same bytes next: each thread orders its own before them
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -237,6 +237,10 @@ class Renderer:
     def set_stage_timing(self, on: bool) -> None:
         self._ck(lib().mp_set_stage_timing(self._ctx, int(bool(on))))
 
+    def set_bns_blocks(self, blocks: int) -> None:
+        """Blocks of the separate bound-and-split launch (0: as many as the device holds at once)."""
+        self._ck(lib().mp_set_bns_blocks(self._ctx, blocks))
+
     def dice_subpatches(self, draw: int, pid, rng):
         pid = np.ascontiguousarray(pid, np.int32)
         rng = np.ascontiguousarray(rng, np.float32).reshape(-1, 4)
