@@ -58,8 +58,6 @@ struct mp_ctx {
     unsigned long long* h_ctrl = nullptr;      // pinned readback
     DrawDev* d_draws = nullptr;
     DrawDev* h_draws = nullptr;                // pinned staging
-    int* d_root_prefix = nullptr;
-    int* h_root_prefix = nullptr;
     int draws_cap = 0;
     Queue q{};
     SubPatches sub{};                 // bound-and-split output, in emission order
@@ -294,6 +292,9 @@ mp_status ensure_mshade(mp_ctx* c) {
     return MP_OK;
 }
 
+// A frame's n draws are followed by their n + 1 root prefixes: one copy, of the
+// frame's own size, uploads both.
+int* root_prefix(DrawDev* draws, int n) { return reinterpret_cast<int*>(draws + n); }
 size_t draw_bytes(int cap) { return sizeof(DrawDev) * (size_t)cap + sizeof(int) * (size_t)(cap + 1); }
 
 mp_status ensure_draws(mp_ctx* c, int n) {
@@ -302,7 +303,6 @@ mp_status ensure_draws(mp_ctx* c, int n) {
     int cap = std::max(n, std::max(4, c->draws_cap * 2));
     // earlier draws of a plain frame may still be read by queued kernels: keep them
     CK(cudaStreamSynchronize(c->stream));
-    // the root prefixes follow the draws: one copy uploads both
     DrawDev* nd = nullptr;
     CK(cudaMalloc((void**)&nd, draw_bytes(cap)));
     if (c->d_draws && c->draws_cap > 0)
@@ -310,13 +310,10 @@ mp_status ensure_draws(mp_ctx* c, int n) {
     cudaFree(c->d_draws);
     cudaFreeHost(c->h_draws);
     c->d_draws = nd;
-    c->d_root_prefix = reinterpret_cast<int*>(nd + cap);
     c->h_draws = nullptr;
-    c->h_root_prefix = nullptr;
     c->draws_cap = 0;
     CK(cudaMallocHost((void**)&c->h_draws, draw_bytes(cap)));
     std::memset((void*)c->h_draws, 0, draw_bytes(cap));
-    c->h_root_prefix = reinterpret_cast<int*>(c->h_draws + cap);
     c->draws_cap = cap;
     return MP_OK;
 }
@@ -500,8 +497,8 @@ long long batched_kernels(const mp_ctx* c) {
     return 6;
 }
 
-void launch_sort(mp_ctx* c) {
-    launch_canonical_sort(c->d_root_prefix, c->sub, c->sorted, c->sb, c->ctrl, c->opt.spin_limit, c->sort_passes,
+void launch_sort(mp_ctx* c, int n) {
+    launch_canonical_sort(root_prefix(c->d_draws, n), c->sub, c->sorted, c->sb, c->ctrl, c->opt.spin_limit, c->sort_passes,
                           c->sort_grid, c->stream);
 }
 
@@ -531,7 +528,7 @@ void mark(mp_ctx* c, int k, bool capturing) {
 // launches, or (option `overlap`) bound-and-split and rasterization as one
 // overlapped launch over the list in emission order.
 void enqueue_frame(mp_ctx* c, int n, long long roots, bool capturing) {
-    cudaMemcpyAsync(c->d_draws, c->h_draws, draw_bytes(c->draws_cap), cudaMemcpyHostToDevice, c->stream);
+    cudaMemcpyAsync(c->d_draws, c->h_draws, draw_bytes(n), cudaMemcpyHostToDevice, c->stream);
     mark(c, 0, capturing);
     launch_clear(c->fb, c->fr, 0, c->stream, c->ctrl, roots, overlapped(c) ? nullptr : c->root_info);
     mark(c, 1, capturing);
@@ -539,13 +536,13 @@ void enqueue_frame(mp_ctx* c, int n, long long roots, bool capturing) {
         // one launch, reported as dice+raster; bound-and-split and sort show 0
         mark(c, 2, capturing);
         mark(c, 3, capturing);
-        launch_frame_kernel(c->d_draws, c->d_root_prefix, n, c->fr, c->q, c->sub, c->fb, c->mshade, c->big, c->big_cap,
+        launch_frame_kernel(c->d_draws, root_prefix(c->d_draws, n), n, c->fr, c->q, c->sub, c->fb, c->mshade, c->big, c->big_cap,
                             c->ctrl, c->opt.spin_limit, c->frame_grid, bns_blocks(c), c->opt.dice_group, c->stream);
     } else {
-        launch_bns_persistent(c->d_draws, c->d_root_prefix, n, c->fr, c->q, c->sub, c->sb, c->ctrl, c->bns_grid,
+        launch_bns_persistent(c->d_draws, root_prefix(c->d_draws, n), n, c->fr, c->q, c->sub, c->sb, c->ctrl, c->bns_grid,
                               c->opt.spin_limit, c->stream);
         mark(c, 2, capturing);
-        launch_sort(c);
+        launch_sort(c, n);
         mark(c, 3, capturing);
         launch_raster_fused(c->d_draws, c->fr, c->sorted, c->fb, c->mshade, c->big, c->big_cap, c->ctrl,
                             c->raster_grid, c->opt.dice_group, c->stream);
@@ -609,12 +606,13 @@ mp_status batched_frame(mp_ctx* c) {
     mp_status st = ensure_draws(c, n);
     if (st) return st;
     long long roots = 0;
-    c->h_root_prefix[0] = 0;
+    int* prefix = root_prefix(c->h_draws, n);
+    prefix[0] = 0;
     for (int i = 0; i < n; ++i) {
         c->h_draws[i] = c->draws[(size_t)i];
         c->h_draws[i].grad_cp = (size_t)i < c->grad_ptr.size() ? c->grad_ptr[(size_t)i] : nullptr;
         roots += c->draws[(size_t)i].n_patches;
-        c->h_root_prefix[i + 1] = (int)roots;
+        prefix[i + 1] = (int)roots;
     }
     if (roots >= (1LL << 31)) return fail(c, MP_ERR_INVALID_ARG, "more than 2^31 patches in one frame");
     // queue_capacity counts ranges, the queue bundles of them
