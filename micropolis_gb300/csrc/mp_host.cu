@@ -837,8 +837,8 @@ mp_status mp_create(const mp_options* opts, mp_ctx** out) {
     if (st == MP_OK) st = grow_big(c, 1 << 16);
     if (st == MP_OK) {
         c->bns_grid = bns_persistent_grid(fr.criterion);
-        c->raster_grid = raster_fused_grid(fr.PS, o.dice_group, fr.displacement);
-        c->frame_grid = frame_kernel_grid(fr.PS, o.dice_group);
+        c->raster_grid = raster_fused_grid(fr, o.dice_group);
+        c->frame_grid = frame_kernel_grid(fr, o.dice_group);
         c->sort_grid = canonical_sort_grid();
         launch_clear(c->fb, c->fr, 1, c->stream);
         ck(cudaStreamSynchronize(c->stream), "init");

@@ -155,7 +155,7 @@ void launch_clear(const Framebuffer& fb, const FrameDev& fr, int with_color, cud
 void launch_raster_fused(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,
                          float* mshade, BigQuad* big, long long big_cap, unsigned long long* ctrl, int grid, int group,
                          cudaStream_t s);
-int raster_fused_grid(int PS, int group, int displacement);
+int raster_fused_grid(const FrameDev& fr, int group);
 // bound-and-split and rasterization overlapped in one launch: the first
 // n_bns_ctas blocks run bound-and-split, then every block consumes emitted
 // sub-patches as they become ready
@@ -163,7 +163,7 @@ void launch_frame_kernel(const DrawDev* draws, const int* root_prefix, int n_dra
                          const SubPatches& sub, const Framebuffer& fb, float* mshade, BigQuad* big, long long big_cap,
                          unsigned long long* ctrl, long long spin_limit, int grid, int n_bns_ctas, int group,
                          cudaStream_t s);
-int frame_kernel_grid(int PS, int group);
+int frame_kernel_grid(const FrameDev& fr, int group);
 void launch_raster_big(const DrawDev* draws, const FrameDev& fr, const Framebuffer& fb, const BigQuad* big,
                        long long big_cap, unsigned long long* ctrl, cudaStream_t s);
 void launch_resolve(const DrawDev* draws, const FrameDev& fr, const SubPatches& sub, const Framebuffer& fb,

@@ -30,6 +30,7 @@ namespace {
 
 constexpr int kFastCoord = 1 << 19;
 constexpr int kFastExtent = 1024;
+constexpr int kWidePixels = 4;   // a warp with a box of more pixels sets edges up once (raster_quad_fast)
 
 // Block bound of kernels/reyes.cl:97-166 for one quad: pmin/pmax start at
 // the viewport max/min, is_front_facing on the wrapped integer coordinates.
@@ -107,19 +108,85 @@ __device__ __forceinline__ bool edge_inside(int v, int ax, int ay, int bx, int b
     // V > C with C = -1 where Dx > 0 or (Dx == 0 and Dy > 0), else 0; Dx = ra.y - rb.y, Dy = rb.x - ra.x
     return v > ((ay > by || (ay == by && bx > ax)) ? -1 : 0);
 }
-__device__ __forceinline__ float tri_depth(int va, int vb, int vc, float da, float db, float dc) {
+__device__ __forceinline__ float tri_rcp(int va, int vb, int vc) { return frcp((float)wadd(wadd(va, vb), vc)); }
+__device__ __forceinline__ float tri_depth(int va, int vb, int vc, float rdn, float da, float db, float dc) {
     // weights: edge b -> c's function for a, c -> a's for b, a -> b's for c (va, vb, vc: edges from a, b, c)
-    const float rdn = frcp((float)wadd(wadd(va, vb), vc));
     return ffma(dc, fmul((float)va, rdn), ffma(db, fmul((float)vc, rdn), fmul(da, fmul((float)vb, rdn))));
+}
+// Writes a covered sample.  The reference writes only depths below the cleared
+// 0x7fffffff (kernels/reyes.cl:389).
+__device__ __forceinline__ void put_fragment(unsigned long long* key, float depth, unsigned mp_id) {
+    const unsigned idp = idepth_of(depth);
+    if (idp < 0x7fffffffu) atomicMin(key, ((unsigned long long)idp << 32) | mp_id);
+}
+
+// raster_quad_fast for boxes of many pixels: the five edges (0 -> 3 is 3 -> 0
+// turned around) set up once and stepped along a row, and one reciprocal a
+// triangle.  The same integers and floats at every sample.
+__device__ __forceinline__ int raster_quad_wide(const FrameDev& fr, unsigned long long* keys, const int* px,
+                                                const int* py, const float* qd, int4 box, unsigned mp_id) {
+    const int x0 = box.x, y0 = box.y, x1 = box.z, y1 = box.w, shift = fr.shift;
+    const int from[5] = {0, 1, 3, 3, 2}, to[5] = {1, 3, 0, 2, 0};
+    int row[5], step[5], down[5];   // each edge's function at the row's first sample, per pixel and per row
+    bool low[5];                    // accepts 0
+#pragma unroll
+    for (int e = 0; e < 5; ++e) {
+        const int a = from[e], b = to[e], dx = wsub(py[b], py[a]), dy = wsub(px[a], px[b]);
+        row[e] = wadd(wmul(dx, (x0 << shift) - px[a]), wmul(dy, (y0 << shift) - py[a]));
+        step[e] = wmul(dx, 1 << shift);
+        down[e] = wmul(dy, 1 << shift);
+        low[e] = dx > 0 || (dx == 0 && dy > 0);
+    }
+    const bool low03 = !low[2] && (px[0] != px[3] || py[0] != py[3]);
+    const float r1 = tri_rcp(row[0], row[1], row[2]), r2 = tri_rcp(wsub(0, row[2]), row[3], row[4]);
+    int frags = 0;
+    for (int y = y0; y <= y1; ++y) {
+        int v[5];
+#pragma unroll
+        for (int e = 0; e < 5; ++e) v[e] = row[e];
+        for (int x = x0; x <= x1; ++x) {
+            const int v03 = wsub(0, v[2]);
+            auto in = [](int value, bool zero) { return value > (zero ? -1 : 0); };
+            const bool in1 = in(v[0], low[0]) && in(v[1], low[1]) && in(v[2], low[2]);
+            const bool in2 = in(v03, low03) && in(v[3], low[3]) && in(v[4], low[4]);
+            if (in1 || in2) {
+                float depth = 1.0f;
+                if (in1) {
+                    const float d = tri_depth(v[0], v[1], v[2], r1, qd[0], qd[1], qd[3]);
+                    if (d < depth) depth = d;
+                }
+                if (in2) {
+                    const float d = tri_depth(v03, v[3], v[4], r2, qd[0], qd[3], qd[2]);
+                    if (d < depth) depth = d;
+                }
+                put_fragment(keys + key_index(fr, x, y), depth, mp_id);
+                ++frags;
+            }
+#pragma unroll
+            for (int e = 0; e < 5; ++e) v[e] = wadd(v[e], step[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 5; ++e) row[e] = wadd(row[e], down[e]);
+    }
+    return frags;
 }
 
 // Fast path: rasterize one quad over its own pixel bbox (see file header).
-// The quad's triangles are (0, 1, 3) and (0, 3, 2).
+// The quad's triangles are (0, 1, 3) and (0, 3, 2).  A warp with a box of more
+// than kWidePixels takes `wide` for all of its quads: its time is that of its
+// largest box, and both ways one after the other would add up.  Dice+raster of
+// the mixed 4,096-patch scene at 1920x1080, split limits 24, 32, 64 and 200
+// (quads of some 9, 16, 64 and 625 pixels): 0.215, 0.190, 0.313 and 0.502 ms
+// without it, 0.200, 0.154, 0.136 and 0.176 with it (boxes above 3 or 8:
+// 0.201 and 0.205 at limit 24, 0.338 and 0.334 at 16; each lane by its own
+// box: 0.232 at 24).
+template <bool WIDE, typename F>
 __device__ __forceinline__ int raster_quad_fast(const FrameDev& fr, unsigned long long* keys, const int* qx,
                                                 const int* qy, const float* qd, int minx, int miny, int maxx,
-                                                int maxy, unsigned mp_id) {
+                                                int maxy, unsigned mp_id, F&& wide) {
     int x0, y0, x1, y1;
     if (!quad_pixels(fr, minx, miny, maxx, maxy, x0, y0, x1, y1)) return 0;
+    if (WIDE && __any_sync(__activemask(), (x1 - x0 + 1) * (y1 - y0 + 1) > kWidePixels)) return wide(make_int4(x0, y0, x1, y1));
     int frags = 0;
     for (int y = y0; y <= y1; ++y)
         for (int x = x0; x <= x1; ++x) {
@@ -138,16 +205,14 @@ __device__ __forceinline__ int raster_quad_fast(const FrameDev& fr, unsigned lon
             if (in1 || in2) {
                 float depth = 1.0f;
                 if (in1) {
-                    const float d = tri_depth(v01, v13, v30, qd[0], qd[1], qd[3]);
+                    const float d = tri_depth(v01, v13, v30, tri_rcp(v01, v13, v30), qd[0], qd[1], qd[3]);
                     if (d < depth) depth = d;
                 }
                 if (in2) {
-                    const float d = tri_depth(v03, v32, v20, qd[0], qd[3], qd[2]);
+                    const float d = tri_depth(v03, v32, v20, tri_rcp(v03, v32, v20), qd[0], qd[3], qd[2]);
                     if (d < depth) depth = d;
                 }
-                // the reference writes only depths below the cleared 0x7fffffff (kernels/reyes.cl:389)
-                const unsigned idp = idepth_of(depth);
-                if (idp < 0x7fffffffu) atomicMin(keys + key_index(fr, x, y), ((unsigned long long)idp << 32) | mp_id);
+                put_fragment(keys + key_index(fr, x, y), depth, mp_id);
                 ++frags;
             }
         }
@@ -399,6 +464,29 @@ __device__ __forceinline__ int4 group_block_tiles(const int2* pxy, int W, int H,
     return make_int4(t[0], t[1], t[2], t[3]);
 }
 
+// raster_quad_wide for a quad of the group whose first vertex is at pxy[0],
+// edep[0] (rows G apart).  Out of line, and the quad read again from shared
+// memory: its state, or its operands as arguments, cost the usual case
+// registers.
+template <int G>
+static __device__ __noinline__ int raster_wide_shared(unsigned long long* keys, const int2* pxy, const float4* edep,
+                                                      int shift, int kshift, int kgx, int4 box, unsigned mp_id) {
+    FrameDev fr{};
+    fr.shift = shift;
+    fr.kshift = kshift;
+    fr.kgx = kgx;
+    const int at[4] = {0, 1, G, G + 1};
+    int qx[4], qy[4];
+    float qd[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        qx[c] = pxy[at[c]].x;
+        qy[c] = pxy[at[c]].y;
+        qd[c] = edep[at[c]].w;
+    }
+    return raster_quad_wide(fr, keys, qx, qy, qd, box, mp_id);
+}
+
 // Modelview and the perspective matrix's entries 0, 5, 10, 14 from 32 floats
 // (modelview, projection; 16-byte aligned).
 __device__ __forceinline__ void load_matrices(const float* m, float (&mv)[16], float (&pr)[4]) {
@@ -478,8 +566,8 @@ __device__ __noinline__ void dice_run_general(FusedSmem<PS, NS>& sm, int b, int 
 // x = 0, so only large quads and those with maxx <= 0 look at the bound, each
 // on its own (group_block_tiles); an eye-plane vertex still skips the block.
 // DISP is the frame's displacement option, compiled in: frames without it
-// carry neither its code nor its registers.
-template <int PS, int NS, bool DISP>
+// carry neither its code nor its registers; WIDE (wide_quads) likewise.
+template <int PS, int NS, bool DISP, bool WIDE>
 __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int base, int n, int next_base, int n_next,
                                              unsigned next_parity, const DrawDev* __restrict__ draws, const FrameDev& fr,
                                              const SubPatches& sub, const Framebuffer& fb,
@@ -658,7 +746,10 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
             const int tiles[4] = {t.x, t.y, t.z, t.w};
             if (!fast) push_big(big, big_cap, ctrl, qx, qy, qd, mp_id, view, tiles);
         }
-        if (fast) f = raster_quad_fast(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id);
+        if (fast)
+            f = raster_quad_fast<WIDE>(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id, [&](int4 box) {
+                return raster_wide_shared<G>(keys, sm.pxy + i0, sm.edep + i0, fr.shift, fr.kshift, fr.kgx, box, mp_id);
+            });
         if (f > 0 || !fast) {
             // the diffuse factor of a quad that may own pixels; resolve
             // turns it into the colour of kernels/reyes.cl:191
@@ -670,7 +761,7 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
     return __syncthreads_and(n_next == 0 || bulk_wait(&sm.full[b ^ 1], next_parity));
 }
 
-template <int PS, int NS, bool DISP>
+template <int PS, int NS, bool DISP, bool WIDE>
 __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     raster_fused_kernel(const DrawDev* __restrict__ draws, FrameDev frp, SubPatches sub, Framebuffer fb,
                         float* __restrict__ mshade, BigQuad* big, long long big_cap, unsigned long long* ctrl) {
@@ -702,7 +793,7 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
         init_stages(sm);
         bool ok = stage_group(sm, 0, 0, base, count(base), sub, draws, fr);
         for (unsigned it = 0; ok && base < S; ++it) {
-            ok = raster_group<PS, NS, DISP>(sm, it & 1, base, count(base), next, count(next), ((it + 1) >> 1) & 1, draws,
+            ok = raster_group<PS, NS, DISP, WIDE>(sm, it & 1, base, count(base), next, count(next), ((it + 1) >> 1) & 1, draws,
                                             fr, sub, fb, mshade, big, big_cap, ctrl, cw(ctrl, kGroupTicket), frags);
             base = next;
             next = (2 * (int)gridDim.x + (int)sm.claimed) * NS;
@@ -733,7 +824,7 @@ constexpr size_t frame_smem() {
                : kFramePtsOffset + bns_smem<fused_threads<NS>(), kStackPairsFrame>();
 }
 
-template <int PS, int NS>
+template <int PS, int NS, bool WIDE>
 __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
     frame_kernel(const DrawDev* __restrict__ gdraws, const int* __restrict__ root_prefix, int n_draws, FrameDev frp,
                  Queue q, SubPatches sub, Framebuffer fb, float* __restrict__ mshade, BigQuad* big, long long big_cap,
@@ -807,10 +898,10 @@ __global__ void __launch_bounds__(fused_threads<NS>(), fused_blocks<NS>())
         bool ok = stage_group(sm, 0, parity, (int)base, n, sub, gdraws, fr);
         parity ^= 1;
         if (ok && fr.displacement)
-            ok = raster_group<PS, NS, true>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
+            ok = raster_group<PS, NS, true, WIDE>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
                                             nullptr, frags);
         else if (ok)
-            ok = raster_group<PS, NS, false>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
+            ok = raster_group<PS, NS, false, WIDE>(sm, 0, (int)base, n, 0, 0, 0, gdraws, fr, sub, fb, mshade, big, big_cap, ctrl,
                                              nullptr, frags);
         if (!ok) {
             if (threadIdx.x == 0) set_status(ctrl, kErrTimeout);
@@ -1088,7 +1179,9 @@ __global__ void sample_grid_kernel(const DrawDev* __restrict__ draws, FrameDev f
             unsigned mp_id = (unsigned)((base + s) * PS * PS + nu + nv * PS);
             int minx, miny, maxx, maxy;
             if (quad_is_fast(qx, qy, minx, miny, maxx, maxy))
-                frags = raster_quad_fast(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id);
+                frags = raster_quad_fast<true>(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id, [&](int4 box) {
+                    return raster_quad_wide(fr, keys, qx, qy, qd, box, mp_id);
+                });
             else
                 push_big(big, big_cap, ctrl, qx, qy, qd, mp_id, view, tiles);
         }
@@ -1185,6 +1278,29 @@ void dispatch_group(int PS, int group, F&& f) {
     }
 }
 
+// Whether a frame's quads are expected to cover many pixels: a sub-patch of PS
+// quads a side is split while it is wider than the limit.  The wide raster pays
+// from some three pixels a side, and its mere presence costs frames of smaller
+// quads 0.4-1.3 % of dice+raster (64 views 4.056 -> 4.073 ms, displaced Gregory
+// patches 0.215 -> 0.218); at two pixels a side (limit 16) both take 0.333 ms.
+bool wide_quads(const FrameDev& fr) { return fr.limit > 2.0f * (float)fr.PS; }
+
+// Calls f(the fused kernel of the shape T and the frame's options).
+template <typename T, typename F>
+void with_fused(const FrameDev& fr, F&& f) {
+    if (wide_quads(fr)) {
+        if (fr.displacement)
+            f(raster_fused_kernel<T::ps, T::ns, true, true>);
+        else
+            f(raster_fused_kernel<T::ps, T::ns, false, true>);
+    } else {
+        if (fr.displacement)
+            f(raster_fused_kernel<T::ps, T::ns, true, false>);
+        else
+            f(raster_fused_kernel<T::ps, T::ns, false, false>);
+    }
+}
+
 int grid_for(long long n, int block) {
     long long g = (n + block - 1) / block;
     if (g < 1) g = 1;
@@ -1207,17 +1323,14 @@ void launch_clear(const Framebuffer& fb, const FrameDev& fr, int with_color, cud
         fb, fr, with_color, reset_ctrl, roots, root_info);
 }
 
-int raster_fused_grid(int PS, int group, int displacement) {
+int raster_fused_grid(const FrameDev& fr, int group) {
     int g = 0;
-    dispatch_group(PS, group, [&](auto t) {
+    dispatch_group(fr.PS, group, [&](auto t) {
         using T = decltype(t);
         auto fit = [&](auto kernel) {
             g = resident_grid(kernel, sizeof(FusedSmem<T::ps, T::ns>), fused_threads<T::ns>());
         };
-        if (displacement)
-            fit(raster_fused_kernel<T::ps, T::ns, true>);
-        else
-            fit(raster_fused_kernel<T::ps, T::ns, false>);
+        with_fused<T>(fr, fit);
     });
     return g;
 }
@@ -1231,18 +1344,21 @@ void launch_raster_fused(const DrawDev* draws, const FrameDev& fr, const SubPatc
             kernel<<<grid, fused_threads<T::ns>(), sizeof(FusedSmem<T::ps, T::ns>), s>>>(draws, fr, sub, fb, mshade, big,
                                                                                         big_cap, ctrl);
         };
-        if (fr.displacement)
-            launch(raster_fused_kernel<T::ps, T::ns, true>);
-        else
-            launch(raster_fused_kernel<T::ps, T::ns, false>);
+        with_fused<T>(fr, launch);
     });
 }
 
-int frame_kernel_grid(int PS, int group) {
+int frame_kernel_grid(const FrameDev& fr, int group) {
     int g = 0;
-    dispatch_group(PS, group, [&](auto t) {
+    dispatch_group(fr.PS, group, [&](auto t) {
         using T = decltype(t);
-        g = resident_grid(frame_kernel<T::ps, T::ns>, frame_smem<T::ps, T::ns>(), fused_threads<T::ns>());
+        auto fit = [&](auto kernel) {
+            g = resident_grid(kernel, frame_smem<T::ps, T::ns>(), fused_threads<T::ns>());
+        };
+        if (wide_quads(fr))
+            fit(frame_kernel<T::ps, T::ns, true>);
+        else
+            fit(frame_kernel<T::ps, T::ns, false>);
     });
     return g;
 }
@@ -1253,8 +1369,14 @@ void launch_frame_kernel(const DrawDev* draws, const int* root_prefix, int n_dra
                          cudaStream_t s) {
     dispatch_group(fr.PS, group, [&](auto t) {
         using T = decltype(t);
-        frame_kernel<T::ps, T::ns><<<grid, fused_threads<T::ns>(), frame_smem<T::ps, T::ns>(), s>>>(
-            draws, root_prefix, n_draws, fr, q, sub, fb, mshade, big, big_cap, ctrl, spin_limit, n_bns_ctas);
+        auto launch = [&](auto kernel) {
+            kernel<<<grid, fused_threads<T::ns>(), frame_smem<T::ps, T::ns>(), s>>>(
+                draws, root_prefix, n_draws, fr, q, sub, fb, mshade, big, big_cap, ctrl, spin_limit, n_bns_ctas);
+        };
+        if (wide_quads(fr))
+            launch(frame_kernel<T::ps, T::ns, true>);
+        else
+            launch(frame_kernel<T::ps, T::ns, false>);
     });
 }
 
