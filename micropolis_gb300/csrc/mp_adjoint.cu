@@ -49,17 +49,32 @@ __device__ __forceinline__ float face_rcp(float den) { return den == 0.0f ? 0.0f
 __device__ __forceinline__ V3 displace_adjoint(float4 pos, const FrameDev& fr, V3 g, float& gamp) {
     const float K[3] = {10.0f, 14.0f, 22.0f}, B[3] = {0.04f, 0.02f, 0.01f};
     const bool small = displace_is_small(pos, fr.fdisp);
-    auto sc = [&](float x) { return small ? sincos_small(x) : make_float2(mp_sinf(x), mp_cosf(x)); };
-    float2 sy0[3], sx1[3], s6[3], sy1[3];
+    // two arguments at a time, as in displace_vertices: those of one x, and of one y
+    auto sines = [&](float a, float b) { return small ? sin2_small(a, b) : make_float2(mp_sinf(a), mp_sinf(b)); };
+    auto cosines = [&](float a, float b) { return small ? cos2_small(a, b) : make_float2(mp_cosf(a), mp_cosf(b)); };
+    auto both = [&](float a) {
+        return small ? make_float2(sin_small(a), cos_small(a)) : make_float2(mp_sinf(a), mp_cosf(a));
+    };
+    float2 sy0[3], sx1[3], s6[3], sy1[3];   // sine, cosine
     float x = pos.x, y = pos.y;
+    sy0[0] = both(fmul(K[0], y));
 #pragma unroll
     for (int st = 0; st < 3; ++st) {
-        sy0[st] = sc(fmul(K[st], y));
         x = ffma(sy0[st].x, fr.fdisp[st], x);
-        sx1[st] = sc(fmul(K[st], x));
-        s6[st] = sc(fmul(6.0f, x));
+        const float a = fmul(K[st], x), b = fmul(6.0f, x);
+        const float2 s = sines(a, b), c = cosines(a, b);
+        sx1[st] = make_float2(s.x, c.x);
+        s6[st] = make_float2(s.y, c.y);
         y = ffma(sx1[st].x, fr.fdisp[st], y);
-        sy1[st] = sc(fmul(K[st], y));
+        const float d = fmul(K[st], y);
+        if (st < 2) {
+            const float e = fmul(K[st < 2 ? st + 1 : 2], y);
+            const float2 t = sines(d, e), u = cosines(d, e);
+            sy1[st] = make_float2(t.x, u.x);
+            sy0[st + 1] = make_float2(t.y, u.y);
+        } else {
+            sy1[st] = both(d);
+        }
     }
 #pragma unroll
     for (int st = 2; st >= 0; --st) {

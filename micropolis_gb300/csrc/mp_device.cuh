@@ -309,55 +309,11 @@ __device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ float frcp(float y) { return __frcp_rn(y); }
 __device__ __forceinline__ float kdiv(float x, float y) { return fmul(x, frcp(y)); }
 
+}  // namespace mp
 
-// Cosine for the adjoint's derivatives: Cody-Waite reduction with pi/2 =
-// P1 + P2 + P3 (three floats from the exact value of pi) and Taylor
-// polynomials (degree 9 / 10) on |r| <= pi/4, with fused multiply-adds.
-__device__ __forceinline__ void sincos_reduced(float x, float& sr, float& cr, int& q) {
-    float k = rintf(fmul(x, 0x1.45f306p-1f));
-    float r = ffma(-k, 0x1.921fb6p+0f, x);
-    r = ffma(-k, -0x1.777a5cp-25f, r);
-    r = ffma(-k, -0x1.ee59dap-50f, r);
-    float kq = fsub(k, fmul(4.0f, floorf(fmul(k, 0.25f))));
-    q = (int)kq;
-    float r2 = fmul(r, r);
-    float ps = ffma(r2, 0x1.71de3ap-19f, -0x1.a01a02p-13f);
-    ps = ffma(r2, ps, 0x1.111112p-7f);
-    ps = ffma(r2, ps, -0x1.555556p-3f);
-    sr = ffma(fmul(r, r2), ps, r);
-    float pc = ffma(r2, -0x1.27e4fcp-22f, 0x1.a01a02p-16f);
-    pc = ffma(r2, pc, -0x1.6c16c2p-10f);
-    pc = ffma(r2, pc, 0x1.555556p-5f);
-    pc = ffma(r2, pc, -0x1.0p-1f);
-    cr = ffma(r2, pc, 1.0f);
-}
-// R6 native_sin: reduction by pi = PI1 + PI2 + PI3 (the pi/2 split doubled,
-// exactly) to |r| <= pi/2, the odd Taylor polynomial of degree 13, the sign
-// of (-1)^k; one polynomial instead of the two of sincos_reduced.
-__device__ __forceinline__ float mp_sinf(float x) {
-    if (!isfinite(x)) return fsub(x, x);
-    const float k = rintf(fmul(x, 0x1.45f306p-2f));
-    float r = ffma(-k, 0x1.921fb6p+1f, x);
-    r = ffma(-k, -0x1.777a5cp-24f, r);
-    r = ffma(-k, -0x1.ee59dap-49f, r);
-    const float r2 = fmul(r, r);
-    float p = ffma(r2, 0x1.612462p-33f, -0x1.ae6456p-26f);
-    p = ffma(r2, p, 0x1.71de3ap-19f);
-    p = ffma(r2, p, -0x1.a01a02p-13f);
-    p = ffma(r2, p, 0x1.111112p-7f);
-    p = ffma(r2, p, -0x1.555556p-3f);
-    const float sn = ffma(fmul(r, r2), p, r);
-    const float odd = fsub(k, fmul(2.0f, floorf(fmul(k, 0.5f))));
-    return odd != 0.0f ? -sn : sn;
-}
-__device__ __forceinline__ float mp_cosf(float x) {
-    if (!isfinite(x)) return fsub(x, x);
-    float s, c;
-    int q;
-    sincos_reduced(x, s, c, q);
-    q &= 3;
-    return q == 0 ? c : q == 1 ? -s : q == 2 ? -c : s;
-}
+#include "mp_trig.cuh"
+
+namespace mp {
 
 __device__ __forceinline__ float sel_nan(float x) { return isnan(x) ? 0.0f : x; }
 
@@ -449,64 +405,6 @@ __device__ __forceinline__ void load_amplitude(FrameDev& fr) {
     }
 }
 
-// mp_sinf for |x| < 2^22 pi, one value and a packed pair, bit for bit: k is
-// rounded by adding and taking away 1.5 * 2^23 (round to nearest even, as
-// rintf, with no conversion instruction), its parity is the sum's lowest bit,
-// and k * -P equals -k * P.  x * (1 / pi) stays a scalar product: a packed
-// one feeding the packed sum could be fused with it.
-constexpr float kRintMagic = 12582912.0f;
-__device__ __forceinline__ float sin_small(float x) {
-    const float km = fadd(fmul(x, 0x1.45f306p-2f), kRintMagic);
-    const float k = fsub(km, kRintMagic);
-    float r = ffma(k, -0x1.921fb6p+1f, x);
-    r = ffma(k, 0x1.777a5cp-24f, r);
-    r = ffma(k, 0x1.ee59dap-49f, r);
-    const float r2 = fmul(r, r);
-    float p = ffma(r2, 0x1.612462p-33f, -0x1.ae6456p-26f);
-    p = ffma(r2, p, 0x1.71de3ap-19f);
-    p = ffma(r2, p, -0x1.a01a02p-13f);
-    p = ffma(r2, p, 0x1.111112p-7f);
-    p = ffma(r2, p, -0x1.555556p-3f);
-    const float sn = ffma(fmul(r, r2), p, r);
-    return __uint_as_float(__float_as_uint(sn) ^ (__float_as_uint(km) << 31));
-}
-__device__ __forceinline__ float2 sin2_small(float x, float y) {
-    const float2 km = fadd2(make_float2(fmul(x, 0x1.45f306p-2f), fmul(y, 0x1.45f306p-2f)), dup2(kRintMagic));
-    const float2 k = fadd2(km, dup2(-kRintMagic));
-    float2 r = ffma2(k, dup2(-0x1.921fb6p+1f), make_float2(x, y));
-    r = ffma2(k, dup2(0x1.777a5cp-24f), r);
-    r = ffma2(k, dup2(0x1.ee59dap-49f), r);
-    const float2 r2 = fmul2(r, r);
-    float2 p = ffma2(r2, dup2(0x1.612462p-33f), dup2(-0x1.ae6456p-26f));
-    p = ffma2(r2, p, dup2(0x1.71de3ap-19f));
-    p = ffma2(r2, p, dup2(-0x1.a01a02p-13f));
-    p = ffma2(r2, p, dup2(0x1.111112p-7f));
-    p = ffma2(r2, p, dup2(-0x1.555556p-3f));
-    const float2 sn = ffma2(fmul2(r, r2), p, r);
-    return make_float2(__uint_as_float(__float_as_uint(sn.x) ^ (__float_as_uint(km.x) << 31)),
-                       __uint_as_float(__float_as_uint(sn.y) ^ (__float_as_uint(km.y) << 31)));
-}
-
-// Sine and cosine together, for the adjoint: sin_small's reduction and sine,
-// and beside it, as the other half of the same packed chain, the even Taylor
-// polynomial of degree 12 (the next term is below 7e-9 on |r| <= pi/2).
-__device__ __forceinline__ float2 sincos_small(float x) {
-    const float km = fadd(fmul(x, 0x1.45f306p-2f), kRintMagic);
-    const float k = fsub(km, kRintMagic);
-    float r = ffma(k, -0x1.921fb6p+1f, x);
-    r = ffma(k, 0x1.777a5cp-24f, r);
-    r = ffma(k, 0x1.ee59dap-49f, r);
-    const float r2 = fmul(r, r);
-    float2 p = ffma2(dup2(r2), make_float2(0x1.612462p-33f, 0x1.1eed8ep-29f),
-                     make_float2(-0x1.ae6456p-26f, -0x1.27e4fcp-22f));
-    p = ffma2(dup2(r2), p, make_float2(0x1.71de3ap-19f, 0x1.a01a02p-16f));
-    p = ffma2(dup2(r2), p, make_float2(-0x1.a01a02p-13f, -0x1.6c16c2p-10f));
-    p = ffma2(dup2(r2), p, make_float2(0x1.111112p-7f, 0x1.555556p-5f));
-    p = ffma2(dup2(r2), p, make_float2(-0x1.555556p-3f, -0x1.0p-1f));
-    const float2 sc = ffma2(make_float2(fmul(r, r2), r2), p, make_float2(r, 1.0f));
-    const unsigned flip = __float_as_uint(km) << 31;
-    return make_float2(__uint_as_float(__float_as_uint(sc.x) ^ flip), __uint_as_float(__float_as_uint(sc.y) ^ flip));
-}
 // Whether every argument of the displacement of an eye position stays in the
 // range of the _small functions.
 __device__ __forceinline__ bool displace_is_small(float4 pos, const float* fd) {
