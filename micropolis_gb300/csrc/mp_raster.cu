@@ -437,7 +437,8 @@ __device__ __forceinline__ bool stage_group(FusedSmem<PS, NS>& sm, int b, unsign
 
 // The 8x8 block bound over front-facing quads (kernels/reyes.cl:120-166) of a
 // block whose first vertex is pxy[0] (rows G apart), clamped, as its tile
-// range; x > z when is_empty (kernels/reyes.cl:287) skips the block.
+// range (which may hold no tile); x < 0 when is_empty (kernels/reyes.cl:287)
+// skips the block.
 template <int G>
 __device__ __forceinline__ int4 group_block_tiles(const int2* pxy, int W, int H, int shift, int backface) {
     FrameDev fr{};
@@ -460,7 +461,7 @@ __device__ __forceinline__ int4 group_block_tiles(const int2* pxy, int W, int H,
         }
     }
     int t[4];
-    if (!block_tiles(fr, x0, y0, x1, y1, true, t)) return make_int4(1, 0, 0, 0);
+    if (!block_tiles(fr, x0, y0, x1, y1, true, t)) return make_int4(-1, 0, 0, 0);
     return make_int4(t[0], t[1], t[2], t[3]);
 }
 
@@ -742,9 +743,13 @@ __device__ __forceinline__ bool raster_group(FusedSmem<PS, NS>& sm, int b, int b
         if (!fast || maxx <= 0) {
             const int4 t = group_block_tiles<G>(sm.pxy + k * NV + (nu & ~7) + (nv & ~7) * G, fr.W, fr.H, fr.shift,
                                                 fr.backface);
-            if (t.x > t.z) continue;
+            if (t.x < 0) continue;
             const int tiles[4] = {t.x, t.y, t.z, t.w};
-            if (!fast) push_big(big, big_cap, ctrl, qx, qy, qd, mp_id, view, tiles);
+            if (!fast) {
+                // (with no tile to replay, a large quad is only counted)
+                if (t.x > t.z) atomicAdd(cw(ctrl, kBigTotal), 1ull);
+                else push_big(big, big_cap, ctrl, qx, qy, qd, mp_id, view, tiles);
+            }
         }
         if (fast)
             f = raster_quad_fast<WIDE>(fr, keys, qx, qy, qd, minx, miny, maxx, maxy, mp_id, [&](int4 box) {

@@ -1,5 +1,6 @@
 """Quads too large for the fast raster: more of them than the first list holds
-(the status is set while the fused kernel runs, then the frame regrows)."""
+(the status is set while the fused kernel runs, then the frame regrows), and
+their number, the same on both paths."""
 import numpy as np
 import pytest
 
@@ -33,3 +34,21 @@ def test_list_overflows_while_rasterizing(built, cuda, n):
         render_scene(r, sc)
         assert_identical_to_oracle(r, sc)
     r.close()
+
+
+@pytest.mark.parametrize("dice, limit, culling", [(8, 100.0, 1), (8, 200.0, 1), (8, 200.0, 0), (16, 300.0, 1)])
+def test_number_of_large_quads(built, cuda, dice, limit, culling):
+    """(blocks without a front-facing quad hold some that have no tile to visit)"""
+    from micropolis_gb300 import scenes
+    from micropolis_gb300.renderer import render_scene, renderer_for
+    rng = np.random.default_rng(3)
+    mv = scenes.look_at((8, -11, 5), (0, 0, 0), (0, 0, 1))
+    sc = scenes.Scene("mixed", 1920, 1080, [scenes.Draw(scenes.scattered_patches(rng, 700, g), mv) for g in (False, True)],
+                      options=dict(reyes_patch_size=dice, bound_n_split_limit=limit, backface_culling=culling))
+    count = []
+    for path in ("plain", "batched"):
+        r = renderer_for(sc, path)
+        render_scene(r, sc)
+        count.append(r.stats()["big_quads"])
+        r.close()
+    assert count[0] == count[1] > 0
