@@ -176,8 +176,7 @@ def backward_work(scene, r, view: int = 0) -> dict:
     B_bwd = W*H*(8 + 16 + 16) B (the depth|id key, dL/dcolour and the
     colour of every pixel) + 12 B per control point of the gradient;
     A_bwd = control-point gradient updates the adjoint kernel issues (one
-    per control-point coordinate per warp of 32 pixels when every pixel of
-    the warp has the same winning patch, else one per covered pixel;
+    per control-point coordinate and distinct patch of each warp of 32 pixels;
     updates of zero are skipped on the device, so this is an upper bound)."""
     import numpy as np
     W, H = scene.width, scene.height
@@ -185,15 +184,11 @@ def backward_work(scene, r, view: int = 0) -> dict:
     vis = r.visibility(view)
     draw, pid, _ = r.subpatches()
     PS2 = r.options.reyes_patch_size ** 2
-    covered = vis >= 0
-    owner = np.full(len(vis), -1, np.int64)
-    s = vis[covered] // PS2
-    owner[covered] = (draw[s].astype(np.int64) << 32) | pid[s].astype(np.int64)
-    per = np.zeros(len(vis), np.int64)
+    covered = np.flatnonzero(vis >= 0)
+    sub = vis[covered] // PS2
+    first = np.concatenate([[0], np.cumsum([d.mesh.n_patches for d in scene.draws])])
+    root = first[draw[sub]] + pid[sub]
+    seen = np.unique((covered // 32).astype(np.int64) * int(first[-1]) + root) % max(int(first[-1]), 1)
     cps = np.array([d.mesh.cp.shape[1] for d in scene.draws])
-    per[covered] = cps[draw[s]] * 3
-    n = len(vis) // 32 * 32
-    wo = owner[:n].reshape(-1, 32)
-    uniform = np.all(wo == wo[:, :1], axis=1) & (wo[:, 0] >= 0)
-    a = int(per[:n].reshape(-1, 32)[~uniform].sum() + per[:n].reshape(-1, 32)[uniform, 0].sum() + per[n:].sum())
-    return {"B_bwd": W * H * 40 + 12 * ncp, "A_bwd": a, "covered_pixels": int(covered.sum())}
+    a = int(3 * cps[np.searchsorted(first, seen, side="right") - 1].sum())
+    return {"B_bwd": W * H * 40 + 12 * ncp, "A_bwd": a, "covered_pixels": len(covered)}
