@@ -45,9 +45,9 @@ L2_FLUSH_BYTES = 256 << 20
 # caches, so the traffic is an upper bound for a launch inside a frame.
 CSRC = os.path.join(ROOT, "micropolis_gb300", "csrc")
 KERNEL_SOURCES = {
-    "dice_raster": ["mp_raster.cu", "mp_device.cuh", "mp_bns_loop.cuh", "mp_internal.h"],
-    "bound_split": ["mp_bns.cu", "mp_device.cuh", "mp_bns_loop.cuh", "mp_internal.h"],
-    "resolve_or_shade": ["mp_raster.cu", "mp_device.cuh", "mp_bns_loop.cuh", "mp_internal.h"],
+    "dice_raster": ["mp_raster.cu", "mp_device.cuh", "mp_trig.cuh", "mp_bns_loop.cuh", "mp_internal.h"],
+    "bound_split": ["mp_bns.cu", "mp_device.cuh", "mp_trig.cuh", "mp_bns_loop.cuh", "mp_handover.h", "mp_internal.h"],
+    "resolve_or_shade": ["mp_raster.cu", "mp_device.cuh", "mp_trig.cuh", "mp_bns_loop.cuh", "mp_internal.h"],
     "canonical_sort_or_sample": ["mp_sort.cu", "mp_bns_loop.cuh", "mp_internal.h"],
 }
 NCU_FIGURES = {

@@ -153,7 +153,7 @@ __device__ __forceinline__ void bns_warp_loop(const DrawDev* draws, const int* _
                                               const FrameDev& fr, const Queue& q, const SubPatches& out,
                                               unsigned* out_seq, RootInfo* roots, unsigned long long* ctrl,
                                               long long spin_limit, float* smem, unsigned claim, unsigned blocks) {
-    static_assert(stack_stride<C>() > C + 32 && kPairWords > 27 && C >= 32, "scratch columns");
+    static_assert(stack_stride<C>() > C + 32 && kPairWords > 27, "scratch columns and the words beside them");
     static_assert(C >= 32, "a step adds up to 16 pairs, or 32 to an empty ring");
     // Pairs are given to waiting warps when more than kGiveAbove are left, and
     // kKeep stay (a step of 16 ranges: on 1,024 Gregory patches bound-and-split

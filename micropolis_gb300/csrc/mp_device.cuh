@@ -147,7 +147,10 @@ __device__ __forceinline__ F3 blend3(float a, const F3& A, float b, const F3& B,
     return F3{fdiv(fadd(fmul(a, A.x), fmul(b, B.x)), den), fdiv(fadd(fmul(a, A.y), fmul(b, B.y)), den),
               fdiv(fadd(fmul(a, A.z), fmul(b, B.z)), den)};
 }
-__device__ __forceinline__ F3 eval_gregory_sample(const float4* pd, float u_in, float v_in) {
+// Not inlined: the nine calls of bound_range share one copy of the code, which
+// keeps the per-pass bound kernel inside the instruction cache, and the
+// persistent kernel's samples (bound_sample) the Bezier scenes' loop small.
+static __device__ __noinline__ F3 eval_gregory_cpu(const float4* pd, float u_in, float v_in) {
     float u = v_in, v = u_in;  // std::swap(u, v)
     F3 F0 = blend3(u, ld3(pd + 12), v, ld3(pd + 16), fadd(u, v));
     F3 F1 = blend3(fsub(1.0f, u), ld3(pd + 17), v, ld3(pd + 13), fadd(fsub(1.0f, u), v));
@@ -161,12 +164,6 @@ __device__ __forceinline__ F3 eval_gregory_sample(const float4* pd, float u_in, 
     F3 P2 = spline3(wu, ld3(pd + 9), F1, F2, ld3(pd + 6));
     F3 P3 = spline3(wu, ld3(pd + 1), ld3(pd + 5), ld3(pd + 10), ld3(pd + 2));
     return spline3(spline_weights(v), P0, P1, P2, P3);
-}
-
-// Not inlined: the nine calls of bound_range share one copy of the code,
-// which keeps the per-pass bound kernel inside the instruction cache.
-static __device__ __noinline__ F3 eval_gregory_cpu(const float4* pd, float u_in, float v_in) {
-    return eval_gregory_sample(pd, u_in, v_in);
 }
 
 // The range bound of src/Reyes/BoundNSplitCLCPU.cpp:249-336: 3x3 samples at
@@ -513,7 +510,7 @@ struct DiceColumn {
     // per factor and two cycles of the FMA pipe (with the packed test below:
     // dice+raster, mixed 4096 patches 1.17 -> 1.12 ms, at
     // 16x16 dicing 3.78 -> 3.65, 64 views 4.30 -> 4.08, displaced 512x512
-    // heightfield at 3840x2160 3.03 -> 2.95).
+    // heightfield at 3840x2160 3.03 -> 2.93).
     __device__ __forceinline__ void add(float vw, const float (&cw)[N], float4 c) {
 #pragma unroll
         for (int n = 0; n < N; ++n) {

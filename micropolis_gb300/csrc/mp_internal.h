@@ -35,7 +35,7 @@ enum CtrlWord {
     kSortTicket,       // tile tickets of the canonical sort, one word per radix pass (kSortPasses)
     kSortDone = kSortTicket + 8,   // grid-barrier arrivals of the sort kernel this frame
     kSortMost,         // keys of the fullest bucket of the canonical sort, when it is too full
-    kStamp,            // start of each stage of a batched frame and the end of the last, ns (kStamps words)
+    kStamp,            // start of each stage of a batched frame and the end of the last, ns (kStamp to kStampEnd)
     kStampEnd = kStamp + 6,
     kNumCtrl
 };

@@ -1227,13 +1227,14 @@ __global__ void image_kernel(const float4* __restrict__ color, FrameDev fr, unsi
     }
 }
 
-// 64-bit atomicMin throughput probe: pattern 0 = uniform random slots,
-// pattern 1 = each warp updates one 8x8-pixel tile (micropolygon-like locality).
+// Control points from xyz triples to (x, y, z, 1).
 __global__ void widen_points_kernel(const float* __restrict__ xyz, float4* __restrict__ out, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], 1.0f);
 }
 
+// 64-bit atomicMin throughput probe: pattern 0 = uniform random slots,
+// pattern 1 = each warp updates one 8x8-pixel tile (micropolygon-like locality).
 __global__ void atomic_bench_kernel(unsigned long long* buf, long long n_slots, long long n_ops, int pattern) {
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
