@@ -53,11 +53,11 @@ KERNEL_SOURCES = {
 NCU_FIGURES = {
     # ncu of one frame (profiles/raster_fused_mixed4096_1920x1080.md and the
     # summaries beside it), sources as of the capture
-    "dice_raster": {"source": "62aea51f17c8749a", "traffic": 101_773_312 + 65_697_792, "inst": 686_423_965},
-    "bound_split": {"source": "d623e6a3bf979e5b", "traffic": 4_508_928 + 15_795_456, "inst": 136_367_102},
-    "resolve_or_shade": {"source": "62aea51f17c8749a", "traffic": 61_491_968 + 5_449_728, "inst": 7_686_845},
-    "canonical_sort_or_sample": {"source": "c963fb5b008b97ec", "traffic": 34_220_544 + 2_097_664,
-                                 "inst": 15_268_433},
+    "dice_raster": {"source": "885e235bfffe0950", "traffic": 101_935_872 + 65_866_752, "inst": 686_421_775},
+    "bound_split": {"source": "a26d95dc5594d17e", "traffic": 4_569_856 + 16_483_328, "inst": 136_955_167},
+    "resolve_or_shade": {"source": "885e235bfffe0950", "traffic": 61_481_472 + 5_368_832, "inst": 7_686_845},
+    "canonical_sort_or_sample": {"source": "8a9e8c5c830fc1d5", "traffic": 34_237_952 + 2_170_368,
+                                 "inst": 15_271_424},
 }
 
 
